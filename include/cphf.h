@@ -44,7 +44,7 @@ typedef enum cphf_status {
 
 /* Arithmetic of the solve. */
 typedef enum cphf_precision {
-  CPHF_PRECISION_FP64 = 0,   /* every contraction in FP64 (the reference's arithmetic) */
+  CPHF_PRECISION_FP64 = 0,   /* every contraction to FP64 (the reference's arithmetic; tensor_cores) */
   CPHF_PRECISION_MIXED = 1   /* split-FP16 tensor-core operator inside FP64 defect correction */
 } cphf_precision;
 
@@ -70,7 +70,11 @@ typedef struct cphf_config {
                                 x0 only (the Krylov iteration and stopping test stay the reference's). */
   int32_t verbose;           /* print per-cycle diagnostics like krylov_block.rs:148-151 (default 0) */
   int64_t aux_chunk;         /* aux functions per K-term chunk (default 0 = automatic) */
-  int32_t tensor_cores;      /* mixed: 1 = tcgen05 split-FP16 K term (default), 0 = FP32 CUDA cores */
+  int32_t tensor_cores;      /* mixed: 1 = tcgen05 split-FP16 K term (default), 0 = FP32 CUDA cores.
+                                FP64 GEMMs (either precision): 1 = large ones on the tensor cores as exact
+                                sums of 62-bit fixed-point digit products, rounded to FP64 once (error
+                                2^-62 |a||b| plus one rounding, below that of a chain of FP64 FMAs);
+                                0 = every one on the FP64 CUDA cores */
   int32_t verify_residual;   /* mixed: how the residual of every correction after the first is obtained and
                                 convergence decided.  0 = updated with the split-precision operator,
                                 r -= (I + A_lowp) d (no FP64-accurate application);  1 = recomputed with

@@ -20,22 +20,41 @@ struct CounterScope {
   ~CounterScope() { g_launch_counter = prev; }
 };
 
+// Reads (and clears) the error flag of the fixed-point GEMMs launched during this call.
+void check_fx(cphf_ctx* c) {
+  if (!c->fx_used) return;
+  c->fx_used = false;
+  int flag = 0;
+  CPHF_CUDA(cudaMemcpyAsync(&flag, c->fx_err.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  CPHF_CUDA(cudaStreamSynchronize(c->stream));
+  if (!flag) return;
+  CPHF_CUDA(cudaMemsetAsync(c->fx_err.p, 0, sizeof(int), c->stream));
+  throw Error(CPHF_ERR_TIMEOUT, "fixed-point FP64 GEMM: a bounded pipeline wait expired");
+}
+
 template <typename F>
 cphf_status guarded(cphf_ctx* c, F&& f) {
   if (!c) return CPHF_ERR_ARG;
+  cphf_status status;
   try {
     CPHF_CUDA(cudaSetDevice(c->device));
     CounterScope scope(c);
     f();
+    check_fx(c);
     c->last_error.clear();
     return CPHF_OK;
   } catch (const Error& e) {
     c->last_error = e.what();
-    return e.status;
+    status = e.status;
   } catch (const std::exception& e) {
     c->last_error = e.what();
-    return CPHF_ERR_CUDA;
+    status = CPHF_ERR_CUDA;
   }
+  if (c->fx_used) {  // a failed call leaves no flag behind for the next one
+    c->fx_used = false;
+    if (cudaMemsetAsync(c->fx_err.p, 0, sizeof(int), c->stream) != cudaSuccess) cudaGetLastError();
+  }
+  return status;
 }
 
 // Copy `bytes` from a host or device pointer into device memory (cudaMemcpyDefault / UVA).

@@ -191,7 +191,8 @@ enum ProfClass {
   PROF_OZC3_WGEN = 24,
   PROF_OZC3_TERM2 = 25,
   PROF_XC_TC64C = 26,
-  PROF_NCLASS = 27
+  PROF_GEMM_FX = 27,
+  PROF_NCLASS = 28
 };
 extern const char* const kProfNames[PROF_NCLASS];
 
@@ -233,6 +234,8 @@ struct cphf_ctx {
   cphf::SpinState spin[2];
 
   // scratch (grown on demand)
+  cphf::DevBuf ws_fx, fx_err;  // fixed-point GEMM: workspace, error flag of its bounded waits
+  bool fx_used = false;        // ... launched since the flag was last read
   cphf::DevBuf ws_gemm, s_c1, s_resp, s_T, s_W, s_d, s_ket, s_rho, s_y, s_x, s_misc, s_host_io;
   cphf::DevBuf k_xs, k_ax, k_h, k_g, k_b, k_xacc, k_x1, k_axt, k_coef, k_ip, k_keep, k_part, k_idx,
       k_hw, k_info, k_r, k_norm, k_finite, k_pre;

@@ -375,6 +375,7 @@ void solve_by_j2c_right(cphf_ctx* c, double* J, int64_t n, int64_t naux, DecompW
       g.B = L + k0; g.b_k = naux; g.b_n = 1;
       g.C = S; g.c_m = 1; g.c_n = n;
       g.alpha = -1.0; g.beta = 1.0;
+      g.k_balance = true;  // the columns of X grow as those of L shrink
       gemm64(c, g);
     }
     GemmDesc x;  // X_k = S inv(L_kk)^T
@@ -382,6 +383,7 @@ void solve_by_j2c_right(cphf_ctx* c, double* J, int64_t n, int64_t naux, DecompW
     x.A = S; x.a_m = 1; x.a_k = n;
     x.B = w.inv.as<double>() + k * TB * TB; x.b_k = wd; x.b_n = 1;
     x.C = J + n * k0; x.c_m = 1; x.c_n = n;
+    x.k_balance = true;
     gemm64(c, x);
   }
 }

@@ -31,7 +31,9 @@ __device__ __forceinline__ int64_t off2(int64_t m, int64_t div, int64_t s1, int6
 }
 
 template <typename T, typename Cfg, typename TA, typename TB, typename TC>
-__global__ void __launch_bounds__(256) gemm_kernel(GemmDesc d, int ksplit, int64_t kchunk, T* ws) {
+__global__ void __launch_bounds__(256) gemm_kernel(GemmDesc d, int ksplit, int64_t kchunk, T* ws,
+                                                   const int* only_if) {
+  if (only_if != nullptr && *only_if == 0) return;
   constexpr int BM = Cfg::BM, BN = Cfg::BN, BK = Cfg::BK, TM = Cfg::TM, TN = Cfg::TN;
   constexpr int NTX = BN / TN, NTY = BM / TM, NT = NTX * NTY;
   constexpr int LA = BM * BK / NT, LB = BK * BN / NT;
@@ -168,7 +170,8 @@ __global__ void __launch_bounds__(256) gemm_kernel(GemmDesc d, int ksplit, int64
 
 // Fixed-order reduction of the split-K partials: C = alpha * sum_s W[s] + beta * C.
 template <typename T, typename TC>
-__global__ void splitk_reduce_kernel(GemmDesc d, int ksplit, const T* __restrict__ ws) {
+__global__ void splitk_reduce_kernel(GemmDesc d, int ksplit, const T* __restrict__ ws, const int* only_if) {
+  if (only_if != nullptr && *only_if == 0) return;
   const int64_t nb = d.batch1 * d.batch2;
   const int64_t total = nb * d.M * d.N;
   const T alpha = (T)d.alpha, beta = (T)d.beta;
@@ -201,7 +204,8 @@ int choose_split(const GemmDesc& d, int num_sms) {
 }
 
 template <typename T, typename Cfg, typename TA, typename TB, typename TC>
-cudaError_t run(const GemmDesc& d, cudaStream_t stream, void* workspace, size_t ws_bytes, int num_sms) {
+cudaError_t run(const GemmDesc& d, cudaStream_t stream, void* workspace, size_t ws_bytes, int num_sms,
+                const int* only_if = nullptr) {
   const int64_t nb = d.batch1 * d.batch2;
   int ksplit = choose_split<Cfg>(d, num_sms);
   if (ksplit > 1) {
@@ -227,14 +231,15 @@ cudaError_t run(const GemmDesc& d, cudaStream_t stream, void* workspace, size_t 
       s.batch1 = bn;
     }
     dim3 grid((unsigned)gx, (unsigned)gy, (unsigned)(bn * ksplit));
-    gemm_kernel<T, Cfg, TA, TB, TC><<<grid, 256, 0, stream>>>(s, ksplit, kchunk, static_cast<T*>(workspace));
+    gemm_kernel<T, Cfg, TA, TB, TC><<<grid, 256, 0, stream>>>(s, ksplit, kchunk, static_cast<T*>(workspace), only_if);
     count_launch();
     cudaError_t err = cudaGetLastError();
     if (err != cudaSuccess) return err;
     if (ksplit > 1) {
       const int64_t total = bn * d.M * d.N;
       const int64_t blocks = std::min<int64_t>((total + 255) / 256, 8 * (int64_t)num_sms);
-      splitk_reduce_kernel<T, TC><<<(unsigned)blocks, 256, 0, stream>>>(s, ksplit, static_cast<const T*>(workspace));
+      splitk_reduce_kernel<T, TC><<<(unsigned)blocks, 256, 0, stream>>>(s, ksplit, static_cast<const T*>(workspace),
+                                                                                only_if);
       count_launch();
       err = cudaGetLastError();
       if (err != cudaSuccess) return err;
@@ -264,7 +269,7 @@ cudaError_t gemm(const GemmDesc& d, cudaStream_t stream, void* workspace, size_t
     // C = beta * C (alpha term is empty)
     GemmDesc z = d;
     z.K = 0;
-    splitk_reduce_kernel<T, TC><<<std::max<int64_t>(1, std::min<int64_t>(4096, (nb * d.M * d.N + 255) / 256)), 256, 0, stream>>>(z, 0, (const T*)nullptr);
+    splitk_reduce_kernel<T, TC><<<std::max<int64_t>(1, std::min<int64_t>(4096, (nb * d.M * d.N + 255) / 256)), 256, 0, stream>>>(z, 0, (const T*)nullptr, nullptr);
     count_launch();
     return cudaGetLastError();
   }
@@ -292,6 +297,12 @@ CPHF_INST(float, double, double, double)
 cudaError_t gemm_f64_emulated(const GemmDesc& d, cudaStream_t stream, void* workspace, size_t ws_bytes,
                               int num_sms) {
   return gemm<dfloat, double, double, double>(d, stream, workspace, ws_bytes, num_sms);
+}
+
+cudaError_t gemm_f64_if(const GemmDesc& d, cudaStream_t stream, void* workspace, size_t ws_bytes, int num_sms,
+                        const int* flag) {
+  if (d.M <= 0 || d.N <= 0 || d.K <= 0) return cudaSuccess;
+  return run<double, CfgF64, double, double, double>(d, stream, workspace, ws_bytes, num_sms, flag);
 }
 
 }  // namespace cphf

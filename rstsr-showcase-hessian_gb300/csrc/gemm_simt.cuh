@@ -33,6 +33,9 @@ struct GemmDesc {
   // columns).  Lets a batch of narrow GEMMs run as one tall GEMM.
   int64_t m_div = 0, a_m2 = 0, c_m2 = 0;
   int64_t n_div = 0, b_n2 = 0, c_n2 = 0;
+  // The scales of A(:, k) and B(k, :) oppose each other along k (a large column of A meets a small
+  // row of B): fixed-point slices are taken after balancing them (gemm_fx.cu); no other effect.
+  bool k_balance = false;
 };
 
 enum class Prec { F64, F32 };
@@ -52,5 +55,9 @@ size_t gemm_workspace_bytes(const GemmDesc& d, size_t elem_bytes, int num_sms = 
 // (about 2^-46 relative per term; GB300 runs FP32 ~60x faster than FP64).
 cudaError_t gemm_f64_emulated(const GemmDesc& d, cudaStream_t stream, void* workspace = nullptr,
                               size_t ws_bytes = 0, int num_sms = 152);
+
+// The native FP64 kernel, launched so that it returns at once unless the device flag is set.
+cudaError_t gemm_f64_if(const GemmDesc& d, cudaStream_t stream, void* workspace, size_t ws_bytes, int num_sms,
+                        const int* flag);
 
 }  // namespace cphf

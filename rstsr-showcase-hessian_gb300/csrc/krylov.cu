@@ -85,6 +85,7 @@ void projected_solve(cphf_ctx* c, const KrylovWork& w, int64_t n, int64_t nd, in
   x.B = w.gw; x.b_k = 1; x.b_n = nd;
   x.C = x_out; x.c_m = 1; x.c_n = n;
   x.beta = accumulate ? 1.0 : 0.0;
+  x.k_balance = true;  // later basis vectors are smaller, their coefficients larger
   gemm64(c, x);
   CPHF_CUDA(cudaStreamSynchronize(c->stream));
   if (info != 0) throw Error(CPHF_ERR_NONFINITE, "singular projected Krylov system (zero pivot " + std::to_string(info) + ")");
@@ -206,6 +207,7 @@ bool krylov_device(cphf_ctx* c, const DeviceOp& aop, const double* b, const doub
       pr.B = w.coef; pr.b_k = 1; pr.b_n = nd;
       pr.C = w.x1; pr.c_m = 1; pr.c_n = n;
       pr.alpha = -1.0; pr.beta = 1.0;
+      pr.k_balance = true;
       gemm64(c, pr);
       // MGS of the new directions; convergence on the unfiltered max (krylov_block.rs:127-131)
       orth_block(c, w, w.x1, n, nblock, p.lindep, keep, ip);

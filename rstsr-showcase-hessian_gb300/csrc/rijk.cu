@@ -18,6 +18,7 @@
 #include <algorithm>
 
 #include "ctx.cuh"
+#include "gemm_fx.cuh"
 #include "kernels.cuh"
 #include "tc_ozaki.cuh"
 
@@ -35,7 +36,7 @@ const char* const kProfNames[PROF_NCLASS] = {"gemm_fp64_simt", "gemm_fp32_simt",
                                              "term2_tcgen05_bf16x4c_exact", "slice_exact",
                                              "kterm_tcgen05_bf16x3c_exact", "tgen_tcgen05_bf16x3c_exact",
                                              "wgen_tcgen05_bf16x3c_exact", "term2_tcgen05_bf16x3c_exact",
-                                             "xc_tcgen05_bf16c_exact"};
+                                             "xc_tcgen05_bf16c_exact", "gemm_fp64_tcgen05"};
 
 static double gemm_flops(const GemmDesc& d) { return 2.0 * d.M * d.N * d.K * d.batch1 * d.batch2; }
 
@@ -44,6 +45,20 @@ void gemm64(cphf_ctx* c, const GemmDesc& d) {
     // FP64 operands and result, FP32 arithmetic: the GEMMs of an operator applied to a small
     // correction, whose result is needed only to ~1e-7 of the correction itself
     gemm32x<double, double, double>(c, d);
+    return;
+  }
+  // large products on the tensor cores as exact sums of fixed-point digit products (gemm_fx.cu);
+  // tensor_cores = 0 keeps every FP64 GEMM on the CUDA cores
+  FxPlan fx;
+  if (c->cfg.tensor_cores != 0 && fx_available(c->device) && fx_plan(d, c->num_sms, fx)) {
+    if (c->fx_err.p == nullptr) {
+      c->fx_err.ensure(sizeof(int), c->counter());
+      CPHF_CUDA(cudaMemsetAsync(c->fx_err.p, 0, sizeof(int), c->stream));
+    }
+    c->ws_fx.ensure(fx.total, c->counter());
+    c->fx_used = true;  // the error flag is read at the end of the API call
+    ProfScope ps(c, PROF_GEMM_FX, gemm_flops(d), 8.0 * (d.M * d.K + d.K * d.N + d.M * d.N) * d.batch1 * d.batch2);
+    CPHF_CUDA(fx_gemm(fx, c->stream, c->ws_fx.p, c->fx_err.as<int>(), c->num_sms));
     return;
   }
   const size_t need = gemm_workspace_bytes(d, 8, c->num_sms);
@@ -83,19 +98,19 @@ void rijk_prepare(cphf_ctx* c) {
     sp.Z.ensure((size_t)nao * no * naux * 8, c->counter());
     sp.O.ensure((size_t)no * no * naux * 8, c->counter());
     if (no == 0) continue;
-    // Z_P = B_P Cocc  (batched over P)
+    // Z_P[mu, i] = sum_nu B_P[nu, mu] Cocc[nu, i] (B_P symmetric): rows (mu, P), one tall GEMM
     GemmDesc z;
-    z.M = nao; z.N = no; z.K = nao; z.batch1 = naux;
-    z.A = c->Bd.p; z.a_m = 1; z.a_k = nao; z.a_b1 = nao * nao;
-    z.B = sp.C.p; z.b_k = 1; z.b_n = nao; z.b_b1 = 0;
-    z.C = sp.Z.p; z.c_m = 1; z.c_n = nao; z.c_b1 = nao * no;
+    z.M = nao * naux; z.N = no; z.K = nao; z.m_div = nao;
+    z.A = c->Bd.p; z.a_m = nao; z.a_m2 = nao * nao; z.a_k = 1;
+    z.B = sp.C.p; z.b_k = 1; z.b_n = nao;
+    z.C = sp.Z.p; z.c_m = 1; z.c_m2 = nao * no; z.c_n = nao;
     gemm64(c, z);
-    // O_P = Cocc^T Z_P
+    // O_P = Cocc^T Z_P: columns (i, P)
     GemmDesc o;
-    o.M = no; o.N = no; o.K = nao; o.batch1 = naux;
-    o.A = sp.C.p; o.a_m = nao; o.a_k = 1; o.a_b1 = 0;
-    o.B = sp.Z.p; o.b_k = 1; o.b_n = nao; o.b_b1 = nao * no;
-    o.C = sp.O.p; o.c_m = 1; o.c_n = no; o.c_b1 = no * no;
+    o.M = no; o.N = no * naux; o.K = nao;
+    o.A = sp.C.p; o.a_m = nao; o.a_k = 1;
+    o.B = sp.Z.p; o.b_k = 1; o.b_n = nao;
+    o.C = sp.O.p; o.c_m = 1; o.c_n = no;
     gemm64(c, o);
   }
 }
@@ -160,11 +175,12 @@ void rijk_response_fp64(cphf_ctx* c, const double* const* bra, int64_t nb, doubl
       c->s_W.ensure((size_t)no * np_max * no * nb * 8, c->counter());
       for (int64_t P0 = 0; P0 < naux; P0 += np_max) {
         const int64_t np = std::min<int64_t>(np_max, naux - P0);
-        GemmDesc t;  // T[(nu,Pl),(i,a)] = sum_j bra[nu,j,a] O_P[j,i]
-        t.M = nao; t.N = no; t.K = no; t.batch1 = np; t.batch2 = nb;
-        t.A = bra[s]; t.a_m = 1; t.a_k = nao; t.a_b1 = 0; t.a_b2 = nao * no;
-        t.B = sp.O.as<double>() + P0 * no * no; t.b_k = 1; t.b_n = no; t.b_b1 = no * no; t.b_b2 = 0;
-        t.C = c->s_T.p; t.c_m = 1; t.c_n = nao * np; t.c_b1 = nao; t.c_b2 = nao * np * no;
+        // T[(nu,Pl),(i,a)] = sum_j bra[nu,j,a] O_P[j,i]: rows (nu, a), columns (i, Pl), one GEMM
+        GemmDesc t;
+        t.M = nao * nb; t.N = no * np; t.K = no; t.m_div = nao; t.n_div = no;
+        t.A = bra[s]; t.a_m = 1; t.a_m2 = nao * no; t.a_k = nao;
+        t.B = sp.O.as<double>() + P0 * no * no; t.b_k = 1; t.b_n = no; t.b_n2 = no * no;
+        t.C = c->s_T.p; t.c_m = 1; t.c_m2 = nao * np * no; t.c_n = nao * np; t.c_n2 = nao;
         gemm64(c, t);
         GemmDesc k1;  // out += -scale_k Bdense[mu,(nu,P)] T[(nu,P),(i,a)]
         k1.M = nao; k1.N = no * nb; k1.K = nao * np;
@@ -174,11 +190,12 @@ void rijk_response_fp64(cphf_ctx* c, const double* const* bra, int64_t nb, doubl
         k1.alpha = -c->scale_k; k1.beta = written[s] ? 1.0 : 0.0;
         gemm64(c, k1);
         written[s] = true;
-        GemmDesc w;  // Wt[(j,Pl),(i,a)] = sum_nu Z_P[nu,i] bra[nu,j,a]
-        w.M = no; w.N = no; w.K = nao; w.batch1 = np; w.batch2 = nb;
-        w.A = sp.Z.as<double>() + P0 * nao * no; w.a_m = nao; w.a_k = 1; w.a_b1 = nao * no; w.a_b2 = 0;
-        w.B = bra[s]; w.b_k = 1; w.b_n = nao; w.b_b1 = 0; w.b_b2 = nao * no;
-        w.C = c->s_W.p; w.c_m = no * np; w.c_n = 1; w.c_b1 = no; w.c_b2 = no * np * no;
+        // Wt[(j,Pl),(i,a)] = sum_nu bra[nu,j,a] Z_P[nu,i]: rows (j, a), columns (i, Pl), one GEMM
+        GemmDesc w;
+        w.M = no * nb; w.N = no * np; w.K = nao; w.m_div = no; w.n_div = no;
+        w.A = bra[s]; w.a_m = nao; w.a_m2 = nao * no; w.a_k = 1;
+        w.B = sp.Z.as<double>() + P0 * nao * no; w.b_k = 1; w.b_n = nao; w.b_n2 = nao * no;
+        w.C = c->s_W.p; w.c_m = 1; w.c_m2 = no * np * no; w.c_n = no * np; w.c_n2 = no;
         gemm64(c, w);
         GemmDesc k2;  // out += -scale_k Z[mu,(j,P)] Wt[(j,P),(i,a)]
         k2.M = nao; k2.N = no * nb; k2.K = no * np;

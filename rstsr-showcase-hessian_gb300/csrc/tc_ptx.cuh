@@ -67,6 +67,13 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
   return d;
 }
 
+// Offset of a tile `bytes` (a multiple of 16) further on, to be added to a descriptor (the 14-bit
+// address field holds all of shared memory, so no carry leaves it): an issuing thread that adds
+// such constants to one descriptor per pipeline stage keeps up with 128 x 64 x 16 MMAs (48
+// clocks each, the shared-memory read rate), where composing both descriptors from addresses for
+// every MMA took ~110 clocks.
+__host__ __device__ constexpr uint64_t desc_off(int bytes) { return (uint64_t)(bytes >> 4); }
+
 // Instruction descriptor of kind::f16 with FP32 accumulation, K-major A and B.
 // bf16 = false: A/B FP16; true: A/B BF16 (both operands always share one type).
 __host__ __device__ constexpr uint32_t instr_desc_f16(int m, int n, bool bf16) {
@@ -81,21 +88,32 @@ __device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t a, uint64_t b,
       : "memory");
 }
 
+// One lane of a converged warp (the same one at every call): the MMA loop runs warp-uniformly, so
+// that its descriptors live in uniform registers, and only the issue itself is predicated.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n selp.u32 %0, 1, 0, q;\n}\n" : "=r"(p));
+  return p != 0;
+}
+
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
+// 32 columns; the wait is part of the statement, so that no arithmetic on the results can be
+// scheduled before it
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
   uint32_t r[32];
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n"
+      "tcgen05.wait::ld.sync.aligned;"
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
         "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
         "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
         "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      : "r"(taddr)
+      : "memory");
 #pragma unroll
   for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
