@@ -136,112 +136,284 @@ __global__ void sum_partials_kernel(const double* __restrict__ partials, int64_t
 }
 
 // ---- modified Gram-Schmidt --------------------------------------------------------------
-constexpr int kMgsMaxRows = 2048;  // rows per block slice (smem 2 x 16 KB)
+// All columns in one cooperative launch.  Right-looking MGS needs two grid-wide steps per
+// projector (its dot products with the columns after it, then their update); as launches of their
+// own these cost more than the arithmetic, and even inside one launch the two barriers and the
+// reduction between them take ~10 us.  Here each block keeps its rows for the whole sweep, a
+// step's update also forms the partial dot products of the next, and up to kMgsPanel = 4 columns
+// project at once:
+//   the dots of the panel's columns v_0 .. v_3 with every later column are taken before the panel
+//   is orthogonalised, and the coefficients follow by substitution, c_qj = <v_q', v_j> / d_q with
+//   <v_q', v_j> = <v_q, v_j> - sum_{r<q} c_rq <v_r', v_j> and d_q = <v_q', v_q>:
+// the same projections as column by column.  The substitution loses digits where a panel column
+// nearly lies in the span of those before it; when a d_q falls below kMgsMinRatio <v_q, v_q> (or
+// near lindep) the step projects with the panel's first column alone, which is plain MGS.
+// Bound by the FP64 pipe where the rows are many (n m^2 FMA pairs, one pair a clock and SM: 2.0 of
+// the 3.8 ms at 36000 x 180; with two launches per column it took 12 ms), else by the ~20 us a
+// step's barriers, reduction and latencies take: 6561 x 72 0.42 ms (3.0 ms), 741 x 18 68 us (~150).
+constexpr int kMgsThreads = 512, kMgsWarps = kMgsThreads / 32, kMgsPanel = 4;
+constexpr double kMgsMinRatio = 1e-2;
+constexpr int64_t kMgsStage = 2048;        // rows of a block whose projectors sit in shared memory
+constexpr int64_t kMgsCoefs = 1024;        // columns whose coefficients sit in shared memory
+constexpr unsigned kMgsSpins = 1u << 24;   // bound of the barrier's wait
+constexpr int64_t kMgsMaxBlocks = 256;
 
-struct MgsGeom {
-  int64_t nblk, rows;
-};
-
-MgsGeom mgs_geom(int64_t n) {
-  MgsGeom g;
-  int64_t nblk = std::min<int64_t>(304, std::max<int64_t>(1, div_up(n, 64)));
-  int64_t rows = div_up(n, nblk);
-  if (rows > kMgsMaxRows) {
-    rows = kMgsMaxRows;
-    nblk = div_up(n, rows);
+// Waits until every block has arrived `target` / gridDim.x times; false when the bound is reached.
+__device__ __forceinline__ bool mgs_barrier(unsigned* bar, unsigned target) {
+  __shared__ int ok;
+  __syncthreads();
+  if (gridDim.x > 1) {
+    if (threadIdx.x == 0) {
+      __threadfence();
+      atomicAdd(bar, 1u);
+      unsigned seen = 0, spin = 0;
+      do {
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
+      } while (seen < target && ++spin < kMgsSpins);
+      ok = seen >= target;
+    }
+    __syncthreads();
+    return ok != 0;
   }
-  g.nblk = nblk;
-  g.rows = rows;
-  return g;
+  return true;
 }
 
-// partials[b + nblk * j] = sum over block-b rows of v_j . v_c, for j in [c, m)
-__global__ void mgs_init_kernel(const double* __restrict__ V, int64_t n, int64_t m, int64_t c,
-                                int64_t rows, double* __restrict__ partials) {
-  const int64_t nblk = gridDim.x;
-  const int64_t r0 = (int64_t)blockIdx.x * rows, r1 = min(n, r0 + rows);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int64_t j = c + wid; j < m; j += nw) {
-    double acc = 0.0;
-    for (int64_t r = r0 + lane; r < r1; r += 32) acc = fma(V[r + n * j], V[r + n * c], acc);
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-    if (lane == 0) partials[blockIdx.x + nblk * j] = acc;
+// Sum of each of the N (a power of two, at most 32) values over the lanes: every exchange halves
+// the values a lane keeps, N + log2(32 / N) shuffles instead of 5 N.  The total of value i ends in
+// the lanes i (32 / N) .. (i + 1) (32 / N) - 1.
+template <int N>
+__device__ __forceinline__ double warp_totals(double (&v)[N], int lane) {
+  int o = 16;
+#pragma unroll
+  for (int h = N / 2; h >= 1; h /= 2, o /= 2) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int i = 0; i < h; ++i) {
+      const double send = up ? v[i] : v[i + h];
+      v[i] = (up ? v[i + h] : v[i]) + __shfl_xor_sync(0xffffffffu, send, o);
+    }
   }
-}
-
-// sum of the nblk partials of column j: one warp, lanes over blocks, then a shuffle tree
-__device__ __forceinline__ double mgs_sum(const double* __restrict__ partials, int64_t nblk, int64_t j, int lane) {
-  double s = 0.0;
-  for (int64_t k = lane; k < nblk; k += 32) s += partials[k + nblk * j];
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  double s = v[0];
+  for (; o > 0; o /= 2) s += __shfl_xor_sync(0xffffffffu, s, o);
   return s;
 }
 
-// Reduce partials of step i: ip[i], keep[i], coef[j] for j > i.  One warp per column (every
-// warp first forms the squared norm of column i itself, so that no block waits on another).
-__global__ void mgs_reduce_kernel(const double* __restrict__ partials, int64_t nblk, int64_t m,
-                                  int64_t i, double lindep, double* __restrict__ ip,
-                                  int* __restrict__ keep, double* __restrict__ coef) {
-  const int lane = threadIdx.x & 31;
-  const int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  const double nsq = mgs_sum(partials, nblk, i, lane);
-  const bool kept = nsq > lindep;
-  if (w == 0 && lane == 0) {
-    ip[i] = nsq;
-    keep[i] = kept ? 1 : 0;
+struct MgsArgs {
+  double* V;
+  int64_t n, m, rows, stage;  // rows per block, of which in shared memory
+  double lindep;
+  double* ip;
+  int* keep;
+  double* coef;      // [m][kMgsPanel]; coef[4 m]: columns projected by the step
+  double* partials;  // [m][kMgsPanel][block]: <v_(p0 + q), v_j> of the block's rows
+  unsigned* bar;
+};
+
+__global__ void __launch_bounds__(kMgsThreads) mgs_kernel(MgsArgs a) {
+  constexpr int B = kMgsPanel;
+  extern __shared__ double mgs_smem[];
+  const int64_t n = a.n, m = a.m, nblk = gridDim.x, stage = a.stage;
+  const int64_t r0 = (int64_t)blockIdx.x * a.rows, len = max((int64_t)0, min(n, r0 + a.rows) - r0);
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  double* const Vb = a.V + r0;
+  double* cur = mgs_smem;                       // [B][stage]: the panel (orthogonalised once projecting)
+  double* nxt = mgs_smem + B * stage;           // the next panel
+  double* const cfs = mgs_smem + 2 * B * stage; // [columns][B]: coefficients of the step
+  unsigned target = 0;
+  int64_t p0 = 0;
+  int w = (int)min((int64_t)B, m);
+  // row r of panel column q (panel starting at column p)
+  auto panel = [&](const double* st, int64_t p, int q, int64_t r) { return r < stage ? st[q * stage + r] : Vb[r + n * (p + q)]; };
+  auto publish = [&](double (&acc)[B], int64_t j, int used) {
+    const double t = warp_totals<B>(acc, lane);
+    const int q = lane >> 3;
+    if ((lane & 7) == 0 && q < used) a.partials[blockIdx.x + nblk * (j * B + q)] = t;
+  };
+  for (int64_t e = threadIdx.x; e < w * len; e += blockDim.x) {
+    const int64_t q = e / len, r = e - q * len;
+    if (r < stage) cur[q * stage + r] = Vb[r + n * q];
   }
-  for (int64_t j = i + 1 + w; j < m; j += nw) {
-    double s = 0.0;
-    if (kept) s = mgs_sum(partials, nblk, j, lane) / nsq;
-    if (lane == 0) coef[j] = s;
+  __syncthreads();
+  for (int64_t j = wid; j < m; j += kMgsWarps) {
+    double acc[B] = {0.0, 0.0, 0.0, 0.0};
+    for (int64_t r = lane; r < len; r += 32) {
+      const double v = Vb[r + n * j];
+#pragma unroll
+      for (int q = 0; q < B; ++q)
+        if (q < w) acc[q] = fma(v, panel(cur, 0, q, r), acc[q]);
+    }
+    publish(acc, j, w);
+  }
+  while (true) {
+    target += gridDim.x;
+    if (!mgs_barrier(a.bar, target)) {
+      if (threadIdx.x == 0) a.keep[0] = -1;  // reported by the host
+      return;
+    }
+    // coefficients of column j: one warp per column over the grid, each from the panel's own dot
+    // products (10) and the column's (4)
+    for (int64_t j = p0 + (int64_t)wid * nblk + blockIdx.x; j < m; j += nblk * kMgsWarps) {
+      double v[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] = 0.0;
+      for (int64_t k = lane; k < nblk; k += 32) {
+        int i = 0;
+#pragma unroll
+        for (int q = 0; q < B; ++q)
+#pragma unroll
+          for (int r = 0; r <= q; ++r, ++i)
+            if (q < w) v[i] += __ldcg(a.partials + k + nblk * ((p0 + q) * B + r));
+#pragma unroll
+        for (int q = 0; q < B; ++q)
+          if (q < w) v[10 + q] += __ldcg(a.partials + k + nblk * (j * B + q));
+      }
+      const double tot = warp_totals<16>(v, lane);  // total i in lanes 2 i, 2 i + 1
+      // g[r][q] = <v_r, v_(p0 + q)> (r <= q), then <v_r', .>
+      double g[B][B], d[B], rd[B], c[B][B], x[B];
+      int width = w;
+      {
+        int i = 0;
+#pragma unroll
+        for (int q = 0; q < B; ++q)
+#pragma unroll
+          for (int r = 0; r <= q; ++r, ++i) g[r][q] = __shfl_sync(0xffffffffu, tot, 2 * i);
+      }
+#pragma unroll
+      for (int q = 0; q < B; ++q) x[q] = __shfl_sync(0xffffffffu, tot, 2 * (10 + q));
+#pragma unroll
+      for (int q = 0; q < B; ++q) {
+        const double full = g[q][q];
+#pragma unroll
+        for (int r = 0; r < q; ++r) {
+#pragma unroll
+          for (int t = 0; t < r; ++t) g[r][q] = fma(-c[t][r], g[t][q], g[r][q]);
+          c[r][q] = g[r][q] * rd[r];
+          g[q][q] = fma(-c[r][q], g[r][q], g[q][q]);
+        }
+        d[q] = g[q][q];
+        rd[q] = 1.0 / d[q];
+        // (a NaN fails the comparison: the first column alone then decides)
+        if (q > 0 && q < width && !(d[q] > kMgsMinRatio * full && d[q] > 4.0 * a.lindep)) width = 1;
+      }
+      const bool kept0 = d[0] > a.lindep;
+      if (!kept0) width = 1;
+      const int64_t e = j - p0;
+      if (e < width) {  // a column of the panel itself
+        double de = d[0];
+#pragma unroll
+        for (int q = 0; q < B; ++q) x[q] = 0.0;
+#pragma unroll
+        for (int q = 1; q < B; ++q)
+          if (e == q) {
+            de = d[q];
+#pragma unroll
+            for (int r = 0; r < q; ++r) x[r] = c[r][q];
+          }
+        if (lane == 0) {
+          a.ip[j] = de;
+          a.keep[j] = de > a.lindep ? 1 : 0;
+          if (e == 0) a.coef[B * m] = (double)width;
+        }
+      } else {
+#pragma unroll
+        for (int q = 0; q < B; ++q) {
+#pragma unroll
+          for (int r = 0; r < q; ++r) x[q] = fma(-c[r][q], x[r], x[q]);
+        }
+#pragma unroll
+        for (int q = 0; q < B; ++q) x[q] = q < width && kept0 ? x[q] * rd[q] : 0.0;
+      }
+      if (lane == 0) {
+#pragma unroll
+        for (int q = 0; q < B; ++q) a.coef[j * B + q] = x[q];
+      }
+    }
+    target += gridDim.x;
+    if (!mgs_barrier(a.bar, target)) {
+      if (threadIdx.x == 0) a.keep[0] = -1;
+      return;
+    }
+    const int64_t nc = min(m - p0, kMgsCoefs);
+    for (int64_t e = threadIdx.x; e < nc * B; e += blockDim.x) cfs[e] = __ldcg(a.coef + p0 * B + e);
+    const int width = (int)__ldcg(a.coef + B * m);
+    const int64_t p1 = p0 + width;
+    const int w1 = (int)max((int64_t)0, min((int64_t)B, m - p1));
+    __syncthreads();
+    auto coef = [&](int64_t j, int t) { return j - p0 < kMgsCoefs ? cfs[(j - p0) * B + t] : __ldcg(a.coef + j * B + t); };
+    // the panel's own columns, a row to a thread
+    if (width > 1)
+      for (int64_t r = threadIdx.x; r < len; r += blockDim.x) {
+        double v[B];
+#pragma unroll
+        for (int q = 0; q < B; ++q) {
+          v[q] = q < width ? panel(cur, p0, q, r) : 0.0;
+#pragma unroll
+          for (int t = 0; t < q; ++t) v[q] = fma(-coef(p0 + min(q, width - 1), t), v[t], v[q]);
+          if (q > 0 && q < width) {
+            if (r < stage) cur[q * stage + r] = v[q];
+            Vb[r + n * (p0 + q)] = v[q];
+          }
+        }
+      }
+    if (p1 >= m) return;
+    __syncthreads();
+    // the next panel's columns first: they are the projectors of the next step
+    for (int64_t e = threadIdx.x; e < w1 * len; e += blockDim.x) {
+      const int64_t q = e / len, r = e - q * len;
+      double v = Vb[r + n * (p1 + q)];
+#pragma unroll
+      for (int t = 0; t < B; ++t)
+        if (t < width) v = fma(-coef(p1 + q, t), panel(cur, p0, t, r), v);
+      if (r < stage) nxt[q * stage + r] = v;
+      Vb[r + n * (p1 + q)] = v;
+    }
+    __syncthreads();
+    for (int64_t j = p1 + wid; j < m; j += kMgsWarps) {
+      double acc[B] = {0.0, 0.0, 0.0, 0.0}, cj[B];
+      const bool mine = j >= p1 + w1;  // not yet updated
+#pragma unroll
+      for (int t = 0; t < B; ++t) cj[t] = mine && t < width ? coef(j, t) : 0.0;
+      if (width == B && w1 == B && mine && len <= stage) {
+#pragma unroll 4
+        for (int64_t r = lane; r < len; r += 32) {
+          double v = Vb[r + n * j];
+#pragma unroll
+          for (int t = 0; t < B; ++t) v = fma(-cj[t], cur[t * stage + r], v);
+          Vb[r + n * j] = v;
+#pragma unroll
+          for (int q = 0; q < B; ++q) acc[q] = fma(v, nxt[q * stage + r], acc[q]);
+        }
+      } else {
+        for (int64_t r = lane; r < len; r += 32) {
+          double v = Vb[r + n * j];
+          if (mine) {
+#pragma unroll
+            for (int t = 0; t < B; ++t)
+              if (t < width) v = fma(-cj[t], panel(cur, p0, t, r), v);
+            Vb[r + n * j] = v;
+          }
+#pragma unroll
+          for (int q = 0; q < B; ++q)
+            if (q < w1) acc[q] = fma(v, panel(nxt, p1, q, r), acc[q]);
+        }
+      }
+      publish(acc, j, w1);
+    }
+    double* const tmp = cur;
+    cur = nxt;
+    nxt = tmp;
+    p0 = p1;
+    w = w1;
   }
 }
 
-// v_j -= coef[j] v_i (j > i), then partials of step i+1.
-__global__ void mgs_update_kernel(double* __restrict__ V, int64_t n, int64_t m, int64_t i,
-                                  int64_t rows, const double* __restrict__ coef,
-                                  const int* __restrict__ keep, double* __restrict__ partials) {
-  __shared__ double vi[kMgsMaxRows];
-  __shared__ double vn[kMgsMaxRows];
-  const int64_t nblk = gridDim.x;
-  const int64_t r0 = (int64_t)blockIdx.x * rows, r1 = min(n, r0 + rows);
-  const int64_t len = r1 - r0;
-  const bool kept = keep[i] != 0;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int64_t r = threadIdx.x; r < len; r += blockDim.x) vi[r] = V[r0 + r + n * i];
-  __syncthreads();
-  // column i+1 first: it is the projector of the next step
-  const int64_t c = i + 1;
-  {
-    const double cf = kept ? coef[c] : 0.0;
-    for (int64_t r = threadIdx.x; r < len; r += blockDim.x) {
-      double v = V[r0 + r + n * c];
-      if (kept) v = fma(-cf, vi[r], v);
-      V[r0 + r + n * c] = v;
-      vn[r] = v;
-    }
-  }
-  __syncthreads();
-  for (int64_t j = c + wid; j < m; j += nw) {
-    const double cf = kept ? coef[j] : 0.0;
-    double acc = 0.0;
-    for (int64_t r = lane; r < len; r += 32) {
-      double v;
-      if (j == c) {
-        v = vn[r];
-      } else {
-        v = V[r0 + r + n * j];
-        if (kept) {
-          v = fma(-cf, vi[r], v);
-          V[r0 + r + n * j] = v;
-        }
-      }
-      acc = fma(v, vn[r], acc);
-    }
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-    if (lane == 0) partials[blockIdx.x + nblk * j] = acc;
-  }
+// Blocks of the sweep: a step takes 2 n m clocks of FP64 work over the blocks and ~15000 clocks for
+// the two barriers and the reduction between them (a third of that with a single block).
+int64_t mgs_blocks(int64_t n, int64_t m, int num_sms) {
+  const double work = 2.0 * (double)n * (double)m;
+  if (work < 16000.0) return 1;
+  return std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(num_sms, kMgsMaxBlocks),
+                                                std::min<int64_t>((int64_t)(work / 4000.0), div_up(n, 32))));
 }
 
 __global__ void gather_cols_kernel(const double* __restrict__ src, int64_t n,
@@ -270,79 +442,212 @@ __global__ void add_diag_kernel(double* h, int64_t ldh, const double* ip, int64_
 }
 
 // ---- LU with partial pivoting -----------------------------------------------------------
-__global__ void lu_pivot_kernel(double* h, int64_t ldh, double* g, int64_t ldg, int64_t m,
-                                int64_t nrhs, int64_t k, int* info) {
-  __shared__ double best_v[kThreads];
-  __shared__ int64_t best_i[kThreads];
-  __shared__ int64_t piv_sh;
-  double bv = -1.0;
-  int64_t bi = k;
-  for (int64_t r = k + threadIdx.x; r < m; r += blockDim.x) {
-    const double v = fabs(h[r + ldh * k]);
-    if (v > bv) { bv = v; bi = r; }
-  }
-  best_v[threadIdx.x] = bv;
-  best_i[threadIdx.x] = bi;
+// Blocked right-looking LU of h with the right-hand sides carried along: per panel of kLuPanel
+// columns one CTA factors the panel (pivot search, scaling, update inside the panel), one launch
+// swaps and solves the panel's rows of every column to its right, one updates the trailing tiles;
+// the back substitution runs over blocks of the same width.  Launches and the panel's serial chain
+// bound it (5 launches per 16 columns instead of 3 per column): m = 216, 72 right-hand sides
+// 1.1 ms, m = 540, 180 right-hand sides 3.1 ms.
+constexpr int kLuPanel = 16;
+constexpr int kLuThreads = 512;
+
+// The row swaps of a panel as moves: row dst[i] receives row src[i], i < count (at most two rows
+// per column), so that a column loads all of them at once.
+struct LuMoves {
+  int count, dst[2 * kLuPanel], src[2 * kLuPanel];
+};
+
+// Panel columns [k0, k0 + w), rows [k0, m): partial pivoting, multipliers in place, the row swaps
+// to *moves.  The panel sits in shared memory when it fits (`smem`).  One division per column
+// (LAPACK's reciprocal scaling): a division per row would occupy the FP64 pipe longer than the
+// update.
+__global__ void __launch_bounds__(kLuThreads) lu_panel_kernel(double* __restrict__ h, int64_t ldh, int64_t m, int64_t k0,
+                                                              int w, int smem, LuMoves* __restrict__ moves, int* info) {
+  extern __shared__ double sp[];
+  __shared__ unsigned long long best_v[kLuThreads / 32];
+  __shared__ int best_i[kLuThreads / 32];
+  __shared__ int piv_sh, piv[kLuPanel];
+  __shared__ double rd_sh;
+  const int rows = (int)(m - k0);
+  const int64_t ld = smem ? rows : ldh;
+  double* const a = smem ? sp : h + k0 + ldh * k0;
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+  if (smem)
+    for (int64_t e = t; e < (int64_t)rows * w; e += blockDim.x) sp[e] = h[(k0 + e % rows) + ldh * (k0 + e / rows)];
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double v = -1.0;
-    int64_t p = k;
-    for (int t = 0; t < (int)blockDim.x; ++t) {
-      if (best_v[t] > v || (best_v[t] == v && best_i[t] < p)) { v = best_v[t]; p = best_i[t]; }
+  for (int j = 0; j < w; ++j) {
+    // the largest |entry| (its bit pattern orders like the value and costs no FP64 comparison; a
+    // NaN never wins), the lowest row among equals; 0 when every entry is zero or NaN
+    unsigned long long bv = 0;
+    int bi = j;
+    for (int r = j + t; r < rows; r += blockDim.x) {
+      const unsigned long long v = (unsigned long long)__double_as_longlong(a[r + ld * j]) & 0x7FFFFFFFFFFFFFFFull;
+      if (v > bv && v <= 0x7FF0000000000000ull) { bv = v; bi = r; }
     }
-    piv_sh = p;
-    if (!(v > 0.0) && *info == 0) *info = (int)(k + 1);
+    for (int o = 16; o > 0; o >>= 1) {
+      const unsigned long long ov = __shfl_xor_sync(0xffffffffu, bv, o);
+      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+      if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
+    }
+    if (lane == 0) { best_v[wid] = bv; best_i[wid] = bi; }
+    __syncthreads();
+    if (wid == 0) {
+      constexpr int NW = kLuThreads / 32;
+      bv = lane < NW ? best_v[lane] : 0;
+      bi = lane < NW ? best_i[lane] : rows;
+      for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long ov = __shfl_xor_sync(0xffffffffu, bv, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+        if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
+      }
+      if (lane == 0) {
+        if (bv == 0) bi = j;
+        piv_sh = bi;
+        piv[j] = bi;
+        rd_sh = 1.0 / a[bi + ld * j];
+        if (bv == 0 && *info == 0) *info = (int)(k0 + j + 1);
+      }
+    }
+    __syncthreads();
+    const int p = piv_sh;
+    if (p != j && t < w) {
+      const double x = a[j + ld * t];
+      a[j + ld * t] = a[p + ld * t];
+      a[p + ld * t] = x;
+    }
+    __syncthreads();
+    const double d = a[j + ld * j], rd = rd_sh;
+    for (int r = j + 1 + t; r < rows; r += blockDim.x) {
+      double l = a[r + ld * j];
+      // (a pivot whose reciprocal overflows is divided by)
+      if (d != 0.0) a[r + ld * j] = l = isfinite(rd) ? l * rd : l / d;
+      for (int c = j + 1; c < w; ++c) a[r + ld * c] = fma(-l, a[j + ld * c], a[r + ld * c]);
+    }
+    __syncthreads();
   }
-  __syncthreads();
-  const int64_t p = piv_sh;
-  if (p != k) {
-    for (int64_t c = threadIdx.x; c < m; c += blockDim.x) {
-      const double t = h[k + ldh * c];
-      h[k + ldh * c] = h[p + ldh * c];
-      h[p + ldh * c] = t;
+  if (smem)
+    for (int64_t e = t; e < (int64_t)rows * w; e += blockDim.x) h[(k0 + e % rows) + ldh * (k0 + e / rows)] = sp[e];
+  if (t == 0) {
+    // the swaps applied in order to the identity, on the rows they touch
+    int n = 0, row[2 * kLuPanel], from[2 * kLuPanel];
+    for (int j = 0; j < w; ++j) {
+      if (piv[j] == j) continue;
+      int x = -1, y = -1;
+      for (int i = 0; i < n; ++i) {
+        if (row[i] == j) x = i;
+        if (row[i] == piv[j]) y = i;
+      }
+      if (x < 0) { x = n++; row[x] = from[x] = j; }
+      if (y < 0) { y = n++; row[y] = from[y] = piv[j]; }
+      const int f = from[x];
+      from[x] = from[y];
+      from[y] = f;
     }
-    for (int64_t c = threadIdx.x; c < nrhs; c += blockDim.x) {
-      const double t = g[k + ldg * c];
-      g[k + ldg * c] = g[p + ldg * c];
-      g[p + ldg * c] = t;
+    for (int i = 0; i < n; ++i) {
+      moves->dst[i] = (int)k0 + row[i];
+      moves->src[i] = (int)k0 + from[i];
     }
-  }
-  __syncthreads();
-  const double d = h[k + ldh * k];
-  if (d != 0.0) {
-    for (int64_t r = k + 1 + threadIdx.x; r < m; r += blockDim.x) h[r + ldh * k] /= d;
+    moves->count = n;
   }
 }
 
-__global__ void lu_update_kernel(double* __restrict__ h, int64_t ldh, double* __restrict__ g,
-                                 int64_t ldg, int64_t m, int64_t nrhs, int64_t k) {
-  const int64_t rows = m - k - 1;
-  const int64_t cols = (m - k - 1) + nrhs;
-  const int64_t total = rows * cols;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t r = k + 1 + t % rows;
-    const int64_t cc = t / rows;
-    const double l = h[r + ldh * k];
-    if (cc < m - k - 1) {
-      const int64_t c = k + 1 + cc;
-      h[r + ldh * c] = fma(-l, h[k + ldh * c], h[r + ldh * c]);
-    } else {
-      const int64_t c = cc - (m - k - 1);
-      g[r + ldg * c] = fma(-l, g[k + ldg * c], g[r + ldg * c]);
-    }
+// column c of the trailing matrix (c < m - k0 - w) or right-hand side
+__device__ __forceinline__ double* lu_column(double* h, int64_t ldh, double* g, int64_t ldg, int64_t m, int64_t k1,
+                                             int64_t c) {
+  return c < m - k1 ? h + ldh * (k1 + c) : g + ldg * (c - (m - k1));
+}
+
+// Row swaps of the panel and the unit lower triangular solve of its w rows, one thread per column.
+__global__ void lu_rows_kernel(double* __restrict__ h, int64_t ldh, double* __restrict__ g, int64_t ldg, int64_t m,
+                               int64_t nrhs, int64_t k0, int w, const LuMoves* __restrict__ moves) {
+  __shared__ double l[kLuPanel][kLuPanel];
+  __shared__ LuMoves mv;
+  for (int e = threadIdx.x; e < w * w; e += blockDim.x) l[e % w][e / w] = h[(k0 + e % w) + ldh * (k0 + e / w)];
+  for (int e = threadIdx.x; e < (int)(sizeof(LuMoves) / sizeof(int)); e += blockDim.x)
+    reinterpret_cast<int*>(&mv)[e] = reinterpret_cast<const int*>(moves)[e];
+  __syncthreads();
+  const int64_t k1 = k0 + w, cols = (m - k1) + nrhs;
+  const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (c >= cols) return;
+  double* x = lu_column(h, ldh, g, ldg, m, k1, c);
+  double s[2 * kLuPanel];
+#pragma unroll
+  for (int i = 0; i < 2 * kLuPanel; ++i) s[i] = i < mv.count ? x[mv.src[i]] : 0.0;
+#pragma unroll
+  for (int i = 0; i < 2 * kLuPanel; ++i)
+    if (i < mv.count) x[mv.dst[i]] = s[i];
+  double v[kLuPanel];
+#pragma unroll
+  for (int j = 0; j < kLuPanel; ++j) v[j] = j < w ? x[k0 + j] : 0.0;
+#pragma unroll
+  for (int j = 0; j < kLuPanel; ++j)
+#pragma unroll
+    for (int q = 0; q < j; ++q)
+      if (j < w) v[j] = fma(-l[j][q], v[q], v[j]);
+#pragma unroll
+  for (int j = 0; j < kLuPanel; ++j)
+    if (j < w) x[k0 + j] = v[j];
+}
+
+// 32 x 32 tile of rows [lo, hi) and columns: X -= A(:, k0 .. k0 + w) X(k0 .. k0 + w, :), the
+// columns of the trailing matrix and the right-hand sides (forward) or the right-hand sides alone
+// (back substitution, k1 = m)
+__global__ void __launch_bounds__(256) lu_update_kernel(double* __restrict__ h, int64_t ldh, double* __restrict__ g,
+                                                        int64_t ldg, int64_t m, int64_t nrhs, int64_t k0, int w,
+                                                        int64_t k1, int64_t lo, int64_t hi) {
+  __shared__ double a[kLuPanel][33];
+  __shared__ double b[kLuPanel][33];
+  const int64_t cols = (m - k1) + nrhs;
+  const int64_t r0 = lo + (int64_t)blockIdx.x * 32, c0 = (int64_t)blockIdx.y * 32;
+  const int t = threadIdx.x;
+  for (int e = t; e < kLuPanel * 32; e += blockDim.x) {
+    const int i = e & 31, q = e >> 5;
+    a[q][i] = q < w && r0 + i < hi ? h[(r0 + i) + ldh * (k0 + q)] : 0.0;
+  }
+  for (int e = t; e < kLuPanel * 32; e += blockDim.x) {
+    const int q = e % kLuPanel, i = e / kLuPanel;
+    b[q][i] = q < w && c0 + i < cols ? lu_column(h, ldh, g, ldg, m, k1, c0 + i)[k0 + q] : 0.0;
+  }
+  __syncthreads();
+  const int i = t & 31;
+  if (r0 + i >= hi) return;
+#pragma unroll
+  for (int cc = 0; cc < 4; ++cc) {
+    const int j = (t >> 5) + 8 * cc;
+    if (c0 + j >= cols) continue;
+    double* x = lu_column(h, ldh, g, ldg, m, k1, c0 + j) + r0 + i;
+    double v = *x;
+#pragma unroll
+    for (int q = 0; q < kLuPanel; ++q) v = fma(-a[q][i], b[q][j], v);
+    *x = v;
   }
 }
 
-__global__ void lu_backsub_kernel(const double* __restrict__ h, int64_t ldh, double* __restrict__ g,
-                                  int64_t ldg, int64_t k) {
-  __shared__ double x_sh;
-  const int64_t c = blockIdx.x;
-  if (threadIdx.x == 0) x_sh = g[k + ldg * c] / h[k + ldh * k];
+// rows [k0, k0 + w) of every right-hand side: U_kk x = g, one thread per column
+__global__ void lu_back_kernel(const double* __restrict__ h, int64_t ldh, double* __restrict__ g, int64_t ldg,
+                               int64_t nrhs, int64_t k0, int w) {
+  __shared__ double u[kLuPanel][kLuPanel];
+  __shared__ double rd[kLuPanel];
+  for (int e = threadIdx.x; e < w * w; e += blockDim.x) u[e % w][e / w] = h[(k0 + e % w) + ldh * (k0 + e / w)];
   __syncthreads();
-  const double x = x_sh;
-  for (int64_t r = threadIdx.x; r < k; r += blockDim.x) g[r + ldg * c] = fma(-h[r + ldh * k], x, g[r + ldg * c]);
-  if (threadIdx.x == 0) g[k + ldg * c] = x;
+  if (threadIdx.x < w) rd[threadIdx.x] = 1.0 / u[threadIdx.x][threadIdx.x];
+  __syncthreads();
+  const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (c >= nrhs) return;
+  double* x = g + ldg * c + k0;
+  double v[kLuPanel];
+#pragma unroll
+  for (int j = 0; j < kLuPanel; ++j) v[j] = j < w ? x[j] : 0.0;
+#pragma unroll
+  for (int j = kLuPanel - 1; j >= 0; --j)
+    if (j < w) {
+      v[j] = isfinite(rd[j]) ? v[j] * rd[j] : v[j] / u[j][j];
+#pragma unroll
+      for (int q = 0; q < j; ++q) v[q] = fma(-u[q][j], v[j], v[q]);
+    }
+#pragma unroll
+  for (int j = 0; j < kLuPanel; ++j)
+    if (j < w) x[j] = v[j];
 }
 
 __global__ void axpby_kernel(double alpha, const double* __restrict__ x, double beta,
@@ -427,26 +732,41 @@ void launch_residual_norms(const double* b, const double* x, const double* ax, d
   count_launch(2);
 }
 
-int64_t mgs_partials_size(int64_t n, int64_t m) { return mgs_geom(n).nblk * std::max<int64_t>(m, 1); }
+// partial dot products, the coefficients and the barrier's counter
+int64_t mgs_partials_size(int64_t n, int64_t m) {
+  const int64_t mm = std::max<int64_t>(m, 1);
+  return kMgsPanel * mm * (std::min<int64_t>(kMgsMaxBlocks, div_up(n, 32)) + 1) + 4;
+}
 
-void launch_mgs(double* V, int64_t n, int64_t m, double lindep, double* ip, int* keep,
-                double* partials, cudaStream_t s) {
+void launch_mgs(double* V, int64_t n, int64_t m, double lindep, double* ip, int* keep, double* partials, int num_sms,
+                cudaStream_t s) {
   if (m <= 0) return;
-  const MgsGeom g = mgs_geom(n);
-  // partials [nblk, m] + coef [m] live in the same scratch
-  double* coef = partials + g.nblk * m;
-  mgs_init_kernel<<<(unsigned)g.nblk, kThreads, 0, s>>>(V, n, m, 0, g.rows, partials);
-  count_launch();
-  for (int64_t i = 0; i < m; ++i) {
-    // one warp per remaining column (8 per block)
-    const unsigned rblocks = (unsigned)std::max<int64_t>(1, div_up(m - i, 8));
-    mgs_reduce_kernel<<<rblocks, 256, 0, s>>>(partials, g.nblk, m, i, lindep, ip, keep, coef);
-    count_launch();
-    if (i + 1 < m) {
-      mgs_update_kernel<<<(unsigned)g.nblk, kThreads, 0, s>>>(V, n, m, i, g.rows, coef, keep, partials);
-      count_launch();
-    }
+  int64_t nblk = mgs_blocks(n, m, num_sms);
+  MgsArgs a;
+  a.V = V;
+  a.n = n;
+  a.m = m;
+  a.rows = div_up(n, nblk);
+  nblk = div_up(n, a.rows);
+  a.stage = std::min(a.rows, kMgsStage);
+  a.lindep = lindep;
+  a.ip = ip;
+  a.keep = keep;
+  a.partials = partials;
+  a.coef = partials + kMgsPanel * m * nblk;
+  a.bar = reinterpret_cast<unsigned*>(a.coef + kMgsPanel * m + 1);
+  const size_t smem = (size_t)kMgsPanel * (2 * a.stage + std::min(m, kMgsCoefs)) * 8;
+  static bool attr = false;
+  if (!attr) {
+    CPHF_CUDA(cudaFuncSetAttribute(mgs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   kMgsPanel * (int)(2 * kMgsStage + kMgsCoefs) * 8));
+    attr = true;
   }
+  CPHF_CUDA(cudaMemsetAsync(a.bar, 0, sizeof(unsigned), s));
+  void* args[] = {&a};
+  CPHF_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(mgs_kernel), dim3((unsigned)nblk),
+                                        dim3(kMgsThreads), args, smem, s));
+  count_launch();
 }
 
 void launch_gather_cols(const double* src, int64_t n, const int* idx, int64_t cnt, double* dst,
@@ -468,18 +788,44 @@ void launch_add_diag(double* h, int64_t ldh, const double* ip, int64_t m, cudaSt
   count_launch();
 }
 
-void launch_lu_solve(double* h, int64_t ldh, double* g, int64_t ldg, int64_t m, int64_t nrhs,
-                     int* info, cudaStream_t s) {
+int64_t lu_scratch_ints() { return 1 + (int64_t)(sizeof(LuMoves) / sizeof(int)); }
+
+void launch_lu_solve(double* h, int64_t ldh, double* g, int64_t ldg, int64_t m, int64_t nrhs, int* info,
+                     cudaStream_t s) {
+  LuMoves* moves = reinterpret_cast<LuMoves*>(info + 1);
   CPHF_CUDA(cudaMemsetAsync(info, 0, sizeof(int), s));
-  for (int64_t k = 0; k < m; ++k) {
-    lu_pivot_kernel<<<1, kThreads, 0, s>>>(h, ldh, g, ldg, m, nrhs, k, info);
-    const int64_t total = (m - k - 1) * ((m - k - 1) + nrhs);
-    if (total > 0) lu_update_kernel<<<grid_for(total, 4096), kThreads, 0, s>>>(h, ldh, g, ldg, m, nrhs, k);
-    count_launch(total > 0 ? 2 : 1);
+  constexpr int kMaxSmem = 200 * 1024;
+  static bool attr = false;
+  if (!attr) {
+    CPHF_CUDA(cudaFuncSetAttribute(lu_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
+    attr = true;
   }
-  for (int64_t k = m - 1; k >= 0; --k) {
-    lu_backsub_kernel<<<(unsigned)nrhs, kThreads, 0, s>>>(h, ldh, g, ldg, k);
+  for (int64_t k0 = 0; k0 < m; k0 += kLuPanel) {
+    const int w = (int)std::min<int64_t>(kLuPanel, m - k0);
+    const int64_t bytes = (m - k0) * w * 8, k1 = k0 + w, cols = (m - k1) + nrhs;
+    const int smem = bytes <= kMaxSmem;
+    lu_panel_kernel<<<1, kLuThreads, smem ? (size_t)bytes : 0, s>>>(h, ldh, m, k0, w, smem, moves, info);
     count_launch();
+    if (cols > 0) {
+      lu_rows_kernel<<<(unsigned)div_up(cols, 64), 64, 0, s>>>(h, ldh, g, ldg, m, nrhs, k0, w, moves);
+      count_launch();
+    }
+    if (k1 < m) {
+      lu_update_kernel<<<dim3((unsigned)div_up(m - k1, 32), (unsigned)div_up(cols, 32)), 256, 0, s>>>(
+          h, ldh, g, ldg, m, nrhs, k0, w, k1, k1, m);
+      count_launch();
+    }
+  }
+  if (nrhs <= 0) return;
+  for (int64_t k0 = (m - 1) / kLuPanel * kLuPanel; k0 >= 0 && m > 0; k0 -= kLuPanel) {
+    const int w = (int)std::min<int64_t>(kLuPanel, m - k0);
+    lu_back_kernel<<<(unsigned)div_up(nrhs, 64), 64, 0, s>>>(h, ldh, g, ldg, nrhs, k0, w);
+    count_launch();
+    if (k0 > 0) {
+      lu_update_kernel<<<dim3((unsigned)div_up(k0, 32), (unsigned)div_up(nrhs, 32)), 256, 0, s>>>(h, ldh, g, ldg, m, nrhs,
+                                                                                                k0, w, m, 0, k0);
+      count_launch();
+    }
   }
 }
 

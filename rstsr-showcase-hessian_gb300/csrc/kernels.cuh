@@ -44,10 +44,11 @@ int64_t residual_partials_size(int64_t n, int64_t nb);
 
 // Right-looking modified Gram-Schmidt over the m columns of V (ld = n), in place,
 // following _orth_block / orth_block (src/util/krylov_block.rs:225-253):
-// keep[i] = ||v_i||^2 > lindep; ip[i] = ||v_i||^2 after projection.
+// keep[i] = ||v_i||^2 > lindep; ip[i] = ||v_i||^2 after projection.  keep[0] = -1: a bounded wait
+// between the blocks ran out.
 // `partials`: mgs_partials_size(n, m) doubles.
 void launch_mgs(double* V, int64_t n, int64_t m, double lindep, double* ip, int* keep,
-                double* partials, cudaStream_t s);
+                double* partials, int num_sms, cudaStream_t s);
 int64_t mgs_partials_size(int64_t n, int64_t m);
 
 // dst[:, j] = src[:, idx[j]] for j < cnt (ld = n both); idx on the device.
@@ -62,9 +63,10 @@ void launch_scale_rows(double* coeff, int64_t ldc, const double* ip, int64_t m, 
 void launch_add_diag(double* h, int64_t ldh, const double* ip, int64_t m, cudaStream_t s);
 
 // Solve h c = g in place (LU with partial pivoting); h [m, m] (ld ldh), g [m, nrhs] (ld ldg).
-// info (device int) is set to k+1 if a zero pivot is met at step k, else 0.
+// info: lu_scratch_ints() device ints; *info is set to k+1 if a zero pivot is met at step k, else 0.
 void launch_lu_solve(double* h, int64_t ldh, double* g, int64_t ldg, int64_t m, int64_t nrhs,
                      int* info, cudaStream_t s);
+int64_t lu_scratch_ints();
 
 
 // y = alpha x + beta y over n elements

@@ -38,16 +38,17 @@ void orth_block(cphf_ctx* c, const KrylovWork& w, double* V, int64_t n, int64_t 
   keep.assign(m, 0);
   ip.assign(m, 0.0);
   if (m == 0) return;
-  double* ipd = w.part + mgs_partials_size(n, m) + m;  // after partials + coef
+  double* ipd = w.part + mgs_partials_size(n, m);
   {
     // algorithmic work of the right-looking MGS: m(m-1)/2 dot + axpy pairs of length n
     // (~2 n m^2 FLOPs), each step re-reading and re-writing the trailing columns (~8 n m^2 bytes)
     ProfScope ps(c, PROF_KRYLOV, 2.0 * n * m * m, 8.0 * n * m * m);
-    launch_mgs(V, n, m, lindep, ipd, w.keep, w.part, c->stream);
+    launch_mgs(V, n, m, lindep, ipd, w.keep, w.part, c->num_sms, c->stream);
   }
   CPHF_CUDA(cudaMemcpyAsync(keep.data(), w.keep, m * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   CPHF_CUDA(cudaMemcpyAsync(ip.data(), ipd, m * 8, cudaMemcpyDeviceToHost, c->stream));
   CPHF_CUDA(cudaStreamSynchronize(c->stream));
+  if (keep[0] < 0) throw Error(CPHF_ERR_TIMEOUT, "orthogonalisation: a bounded wait between blocks expired");
   for (int64_t i = 0; i < m; ++i)
     if (!std::isfinite(ip[i])) throw Error(CPHF_ERR_NONFINITE, "non-finite vector in the Krylov subspace");
 }
@@ -108,7 +109,7 @@ bool krylov_device(cphf_ctx* c, const DeviceOp& aop, const double* b, const doub
   c->k_part.ensure((size_t)(mgs_partials_size(n, nset) + 2 * nset + 8) * 8, c->counter());
   c->k_keep.ensure((size_t)std::max<int64_t>(nset, 1) * sizeof(int), c->counter());
   c->k_idx.ensure((size_t)std::max<int64_t>(nset, 1) * sizeof(int), c->counter());
-  c->k_info.ensure(sizeof(int), c->counter());
+  c->k_info.ensure((size_t)lu_scratch_ints() * sizeof(int), c->counter());
   KrylovWork w;
   w.xs = c->k_xs.as<double>();
   w.ax = c->k_ax.as<double>();
