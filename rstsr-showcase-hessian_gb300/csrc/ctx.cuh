@@ -278,6 +278,7 @@ namespace cphf {
 
 // gemm helpers bound to the context (stream, split-K workspace, SM count)
 void gemm64(cphf_ctx* c, const GemmDesc& d);
+double gemm64_us(cphf_ctx* c, const GemmDesc& d);      // its expected time (us)
 void gemm32(cphf_ctx* c, const GemmDesc& d);  // float compute, float operands/output
 template <typename TA, typename TB, typename TC>
 void gemm32x(cphf_ctx* c, const GemmDesc& d);

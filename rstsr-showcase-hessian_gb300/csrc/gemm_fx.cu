@@ -728,7 +728,7 @@ cudaError_t fx_gemm(const FxPlan& p, cudaStream_t st, void* ws, int* err, int nu
 }
 
 // Plan and choice.  The line between the two kernels is drawn by their measured times (us, GB300):
-//   native: a 64 x 64 tile of K c takes 1.08 c on its SM (the FP64 pipe; padding costs in full);
+//   native: gemm_f64_us;
 //   fixed point: 9.2 per 128 k of a 128 x 64 tile and SM, at least ~10 for the rounding of its
 //   results, ~4 to fill the pipeline; slicing and reducing stream at ~4.5e6 B/us; ~20 for the
 //   launches around the GEMM.
@@ -782,10 +782,11 @@ bool fx_plan(const GemmDesc& d0, int num_sms, FxPlan& p) {
   p.kb_per_split = (int)div_up(rounds, best) * SPLIT_KB;
   const double passes = (double)div_up(d.M, p.m_chunk);
   const double bytes = (double)(d.M + d.N) * d.K * nb * (16.0 + 4.0 * S) + 8.0 * d.M * d.N * nb;
-  const double t_fx = passes * (best_t + 10.0) + 10.0 + bytes / 4.5e6;
-  const int64_t ntiles = div_up(d0.M, 64) * div_up(d0.N, 64) * d0.batch1;
-  const int64_t nsplit = std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(div_up(2 * num_sms, ntiles), d0.K / 64), 32));
-  const double t_native = 5.0 + (double)div_up(ntiles * nsplit, num_sms) * div_up(d0.K, nsplit) * 1.08;
+  // an operand that is strided along k, or long in few rows, takes two slicing launches
+  const double launches = (d.a_k != 1 || d.K > 1024 ? 6.0 : 0.0) + (d.b_k != 1 || d.K > 1024 ? 6.0 : 0.0);
+  const double t_fx = passes * (best_t + 10.0) + 12.0 + launches + bytes / 4.5e6;
+  const double t_native = gemm_f64_us(d0, num_sms);
+  p.us = t_fx;
   if (t_fx > 0.8 * t_native) return false;
   size_t off = 256 + 8 * ((size_t)(d.N + p.m_chunk) * d.batch1 + (d.k_balance ? (size_t)d.K : 0));
   p.key_bytes = off;

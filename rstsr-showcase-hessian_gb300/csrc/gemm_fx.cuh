@@ -16,6 +16,7 @@ struct FxPlan {
   int m_tiles = 0, n_tiles = 0;
   int splits = 1, kb_per_split = 0;
   int64_t m_chunk = 0;     // rows of A per pass (bounds the planes)
+  double us = 0.0;         // expected time
   size_t key_bytes = 0;    // flag + row keys, cleared before each pass
   size_t off_ea = 0, off_eb = 0, off_a = 0, off_b = 0, off_ws = 0, total = 0;
 };

@@ -4,6 +4,7 @@
 #include "dfloat.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace cphf {
 
@@ -12,6 +13,10 @@ namespace {
 // FP64: 64x64 tile, 4x4 per thread, 256 threads.  FP64-pipe bound on GB300.
 struct CfgF64 {
   static constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;
+};
+// FP64, few or short outputs: 32x32 tile, 2x2 per thread, so that small products spread over the SMs.
+struct CfgF64S {
+  static constexpr int BM = 32, BN = 32, BK = 16, TM = 2, TN = 2;
 };
 // FP32: 128x128 tile, 8x8 per thread, 256 threads.
 struct CfgF32 {
@@ -107,6 +112,13 @@ __global__ void __launch_bounds__(256) gemm_kernel(GemmDesc d, int ksplit, int64
 #pragma unroll
     for (int j = 0; j < TN; ++j) acc[i][j] = (T)0;
 
+  // FP64: padding is not multiplied (a padded row or column of 16 costs the FP64 pipe as much as a
+  // real one): the 16-row / 16-column groups of the tile with a row or column inside the matrix
+  constexpr bool SKIP = std::is_same<T, double>::value;
+  const int imax = SKIP ? (int)min((int64_t)TM, (d.M - m0 + NTY - 1) / NTY) : TM;
+  const int jmax = SKIP ? (int)min((int64_t)TN, (d.N - n0 + NTX - 1) / NTX) : TN;
+  const bool whole = imax == TM && jmax == TN;
+
   int buf = 0;
   if (kbeg < kend) {
     load_tiles(kbeg);
@@ -115,6 +127,23 @@ __global__ void __launch_bounds__(256) gemm_kernel(GemmDesc d, int ksplit, int64
     for (int64_t k0 = kbeg; k0 < kend; k0 += BK) {
       const bool has_next = (k0 + BK < kend);
       if (has_next) load_tiles(k0 + BK);
+      if (SKIP && (!whole || kend - k0 < BK)) {
+        const int kn = (int)min((int64_t)BK, kend - k0);
+        for (int kk = 0; kk < kn; ++kk) {
+          T a[TM], b[TN];
+#pragma unroll
+          for (int i = 0; i < TM; ++i) a[i] = As[buf][kk][ty + i * NTY];
+#pragma unroll
+          for (int j = 0; j < TN; ++j) b[j] = Bs[buf][kk][tx + j * NTX];
+#pragma unroll
+          for (int i = 0; i < TM; ++i)
+            if (i < imax) {
+#pragma unroll
+              for (int j = 0; j < TN; ++j)
+                if (j < jmax) acc[i][j] = madd(a[i], b[j], acc[i][j]);
+            }
+        }
+      } else
 #pragma unroll
       for (int kk = 0; kk < BK; ++kk) {
         T a[TM], b[TN];
@@ -203,11 +232,45 @@ int choose_split(const GemmDesc& d, int num_sms) {
   return (int)std::max<int64_t>(want, 1);
 }
 
+// Tile and K split of a native FP64 GEMM, by the time they take (us): blocks in waves over the SMs
+// at 16-padded rows x columns x k / 2 clocks (1.9 GHz), a K tile at least ~0.5 us (load latency),
+// the reduction of the partial sums ~3 us.  24 x 60 x 2016: 64 x 64 tiles in 31 splits 95 us,
+// 32 x 32 tiles in 63 splits 15 us.
+struct F64Choice {
+  bool small;
+  int split;
+  double us;
+};
+template <typename Cfg>
+void f64_candidates(const GemmDesc& d, int num_sms, bool small, F64Choice& best) {
+  const int64_t nb = d.batch1 * d.batch2;
+  const int64_t tiles = ((d.M + Cfg::BM - 1) / Cfg::BM) * ((d.N + Cfg::BN - 1) / Cfg::BN) * nb;
+  const double rows = (double)std::min<int64_t>(Cfg::BM, (d.M + 15) / 16 * 16);
+  const double cols = (double)std::min<int64_t>(Cfg::BN, (d.N + 15) / 16 * 16);
+  for (int s = 1; s <= 128; s *= 2) {
+    if (s > 1 && ((int64_t)s * 2 * Cfg::BK > d.K || tiles * s > 8 * (int64_t)num_sms ||
+                  (double)s * d.M * d.N * nb * 8 > 256e6))
+      break;
+    const double kc = (double)div_up(div_up(d.K, s), Cfg::BK) * Cfg::BK;
+    const double waves = (double)div_up(tiles * s, num_sms);
+    const double t = std::max(waves * rows * cols * std::min(kc, (double)d.K) / 2.0 / 1900.0, kc / Cfg::BK * 0.5) +
+                     (s > 1 ? 3.0 + (double)s * d.M * d.N * nb * 8 / 3e6 : 0.0);
+    if (best.us < 0.0 || t < best.us) best = F64Choice{small, s, t};
+  }
+}
+F64Choice f64_choice(const GemmDesc& d, int num_sms) {
+  F64Choice best{false, 1, -1.0};
+  f64_candidates<CfgF64>(d, num_sms, false, best);
+  f64_candidates<CfgF64S>(d, num_sms, true, best);
+  best.us += 3.0;
+  return best;
+}
+
 template <typename T, typename Cfg, typename TA, typename TB, typename TC>
 cudaError_t run(const GemmDesc& d, cudaStream_t stream, void* workspace, size_t ws_bytes, int num_sms,
-                const int* only_if = nullptr) {
+                const int* only_if = nullptr, int split = 0) {
   const int64_t nb = d.batch1 * d.batch2;
-  int ksplit = choose_split<Cfg>(d, num_sms);
+  int ksplit = split > 0 ? split : choose_split<Cfg>(d, num_sms);
   if (ksplit > 1) {
     const size_t need = (size_t)ksplit * nb * d.M * d.N * sizeof(T);
     if (workspace == nullptr || need > ws_bytes) ksplit = 1;
@@ -248,6 +311,13 @@ cudaError_t run(const GemmDesc& d, cudaStream_t stream, void* workspace, size_t 
   return cudaSuccess;
 }
 
+cudaError_t run_f64(const GemmDesc& d, cudaStream_t stream, void* workspace, size_t ws_bytes, int num_sms,
+                    const int* only_if) {
+  const F64Choice f = f64_choice(d, num_sms);
+  if (f.small) return run<double, CfgF64S, double, double, double>(d, stream, workspace, ws_bytes, num_sms, only_if, f.split);
+  return run<double, CfgF64, double, double, double>(d, stream, workspace, ws_bytes, num_sms, only_if, f.split);
+}
+
 // narrow-output FP32 shapes take the 256 x 64 tile
 bool use_tall(const GemmDesc& d) { return d.N <= 64 && d.M >= 512; }
 
@@ -255,7 +325,7 @@ bool use_tall(const GemmDesc& d) { return d.N <= 64 && d.M >= 512; }
 
 size_t gemm_workspace_bytes(const GemmDesc& d, size_t elem_bytes, int num_sms) {
   int s;
-  if (elem_bytes == 8) s = choose_split<CfgF64>(d, num_sms);
+  if (elem_bytes == 8) s = std::max(choose_split<CfgF64>(d, num_sms), f64_choice(d, num_sms).split);
   else s = use_tall(d) ? choose_split<CfgF32Tall>(d, num_sms) : choose_split<CfgF32>(d, num_sms);
   if (s <= 1) return 0;
   return (size_t)s * d.batch1 * d.batch2 * d.M * d.N * elem_bytes;
@@ -273,7 +343,9 @@ cudaError_t gemm(const GemmDesc& d, cudaStream_t stream, void* workspace, size_t
     count_launch();
     return cudaGetLastError();
   }
-  if constexpr (sizeof(T) == 8) {
+  if constexpr (std::is_same<T, double>::value) {
+    return run_f64(d, stream, workspace, ws_bytes, num_sms, nullptr);
+  } else if constexpr (sizeof(T) == 8) {
     return run<T, CfgF64, TA, TB, TC>(d, stream, workspace, ws_bytes, num_sms);
   } else {
     if (use_tall(d)) return run<T, CfgF32Tall, TA, TB, TC>(d, stream, workspace, ws_bytes, num_sms);
@@ -302,7 +374,9 @@ cudaError_t gemm_f64_emulated(const GemmDesc& d, cudaStream_t stream, void* work
 cudaError_t gemm_f64_if(const GemmDesc& d, cudaStream_t stream, void* workspace, size_t ws_bytes, int num_sms,
                         const int* flag) {
   if (d.M <= 0 || d.N <= 0 || d.K <= 0) return cudaSuccess;
-  return run<double, CfgF64, double, double, double>(d, stream, workspace, ws_bytes, num_sms, flag);
+  return run_f64(d, stream, workspace, ws_bytes, num_sms, flag);
 }
+
+double gemm_f64_us(const GemmDesc& d, int num_sms) { return f64_choice(d, num_sms).us; }
 
 }  // namespace cphf

@@ -51,6 +51,9 @@ cudaError_t gemm(const GemmDesc& d, cudaStream_t stream, void* workspace = nullp
 // Workspace bytes that gemm<> may use for split-K on descriptor d.
 size_t gemm_workspace_bytes(const GemmDesc& d, size_t elem_bytes, int num_sms = 152);
 
+// Expected time (us) of the native FP64 kernel on d.
+double gemm_f64_us(const GemmDesc& d, int num_sms);
+
 // FP64 operands and result, products and sums in double-float arithmetic on the FP32 pipes
 // (about 2^-46 relative per term; GB300 runs FP32 ~60x faster than FP64).
 cudaError_t gemm_f64_emulated(const GemmDesc& d, cudaStream_t stream, void* workspace = nullptr,

@@ -40,6 +40,12 @@ const char* const kProfNames[PROF_NCLASS] = {"gemm_fp64_simt", "gemm_fp32_simt",
 
 static double gemm_flops(const GemmDesc& d) { return 2.0 * d.M * d.N * d.K * d.batch1 * d.batch2; }
 
+double gemm64_us(cphf_ctx* c, const GemmDesc& d) {
+  FxPlan fx;
+  if (c->cfg.tensor_cores != 0 && fx_available(c->device) && fx_plan(d, c->num_sms, fx)) return fx.us;
+  return gemm_f64_us(d, c->num_sms);
+}
+
 void gemm64(cphf_ctx* c, const GemmDesc& d) {
   if (c->f32_correction) {
     // FP64 operands and result, FP32 arithmetic: the GEMMs of an operator applied to a small

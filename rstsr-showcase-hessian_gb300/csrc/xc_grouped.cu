@@ -299,6 +299,52 @@ XcPlan& xc_plan(cphf_ctx* c, size_t esize, int64_t nb) {
   return pl;
 }
 
+// The two contractions of one batch as FP64 GEMMs: ket rows of the batch, out rows of its window.
+static GemmDesc batch_ket(cphf_ctx* c, const XcBatch& x, int64_t g0, int64_t pts, int64_t N, const double* phi,
+                          const double* bra, double* ket) {
+  GemmDesc d;
+  d.M = x.npts; d.N = N; d.K = x.nwin;
+  d.A = phi + x.phi_off; d.a_m = 1; d.a_k = x.npts;
+  d.B = bra + x.lo; d.b_k = 1; d.b_n = c->nao;
+  d.C = ket + (x.g0 - g0); d.c_m = 1; d.c_n = pts;
+  return d;
+}
+static GemmDesc batch_out(cphf_ctx* c, const XcBatch& x, int64_t g0, int64_t pts, int64_t N, const double* phi,
+                          const double* q, double* out, double fac) {
+  GemmDesc d;
+  d.M = x.nwin; d.N = N; d.K = x.npts;
+  d.A = phi + x.phi_off; d.a_m = x.npts; d.a_k = 1;
+  d.B = q + (x.g0 - g0); d.b_k = 1; d.b_n = pts;
+  d.C = out + x.lo; d.c_m = 1; d.c_n = c->nao;
+  d.alpha = fac; d.beta = 1.0;
+  return d;
+}
+
+// FP64: one GEMM per batch and contraction (on the tensor cores where gemm64 finds that faster)
+// instead of the two grouped launches, when the sum of their expected times is the smaller: the
+// grouped kernels run at the FP64 pipe's rate, and the second one gives each 64 x 64 output tile
+// to one CTA for all points (nao 83, 6600 points: 16 ms an application, batches 1.1 ms); with
+// many tiny batches the launches of the batch route cost more.
+static bool batches_faster(cphf_ctx* c, const XcChunk& ch, int64_t N) {
+  if (c->cfg.tensor_cores == 0 || N <= 0) return false;
+  constexpr double kTile = 64.0 * 64.0 / 2.0 / 1900.0;  // us per k of a tile on one SM
+  const double tn = (double)xc_tiles_n(N, true);
+  double batch = 0.0, work1 = 0.0;
+  std::vector<double> pts((size_t)div_up(c->nao, 64), 0.0);  // points that meet each row tile
+  for (int64_t b = ch.b0; b < ch.b1; ++b) {
+    const XcBatch& x = c->xc_batches[b];
+    if (x.npts == 0 || x.nwin == 0) continue;
+    batch += gemm64_us(c, batch_ket(c, x, ch.g0, ch.npts, N, nullptr, nullptr, nullptr)) +
+             gemm64_us(c, batch_out(c, x, ch.g0, ch.npts, N, nullptr, nullptr, nullptr, 1.0));
+    work1 += (double)xc_tiles_m(x.npts, true) * tn * (double)x.nwin;
+    for (int64_t t = x.lo / 64; t <= (x.lo + x.nwin - 1) / 64; ++t) pts[(size_t)t] += (double)x.npts;
+  }
+  double longest = 0.0, all = 0.0;
+  for (double p : pts) longest = std::max(longest, p), all += p;
+  const double grouped = kTile * (work1 / c->num_sms + std::max(longest, all * tn / c->num_sms)) + 10.0;
+  return batch < grouped;
+}
+
 template <typename T>
 void xc_response_grouped(cphf_ctx* c, const T* const* bra, int64_t nb, T* const* out, bool accumulate, const T* phi,
                          const T* const* aobra, DevBuf& ket_buf, DevBuf& rho_buf) {
@@ -333,7 +379,15 @@ void xc_response_grouped(cphf_ctx* c, const T* const* bra, int64_t nb, T* const*
       }
       // rows of batches with an empty AO window are never written: clear them first
       CPHF_CUDA(cudaMemsetAsync(ket[s], 0, (size_t)ch.npts * no * nb * sizeof(T), c->stream));
-      xc_grouped_gemm1<T>(c, gdev + ch.group_off + s * ng, ng, ch.tiles[s], phi, bra[s], no * nb, ch.npts, ket[s]);
+      bool batches = false;
+      if constexpr (sizeof(T) == 8) {
+        batches = batches_faster(c, ch, no * nb);
+        for (int64_t b = ch.b0; batches && b < ch.b1; ++b)
+          if (c->xc_batches[b].npts > 0 && c->xc_batches[b].nwin > 0)
+            gemm64(c, batch_ket(c, c->xc_batches[b], ch.g0, ch.npts, no * nb, phi, bra[s], ket[s]));
+      }
+      if (!batches)
+        xc_grouped_gemm1<T>(c, gdev + ch.group_off + s * ng, ng, ch.tiles[s], phi, bra[s], no * nb, ch.npts, ket[s]);
       launch_xc_rho<T>(aobra[s] + ch.g0, c->ngrids, ket[s], ch.npts, no, nb, rho_s, ch.npts, c->stream);
     }
     for (int s = 0; s < ns; ++s) {
@@ -341,7 +395,15 @@ void xc_response_grouped(cphf_ctx* c, const T* const* bra, int64_t nb, T* const*
       if (no == 0) continue;
       launch_xc_q<T>(aobra[s] + ch.g0, c->ngrids, c->weights.as<double>() + ch.g0, c->fxc.as<double>() + ch.g0,
                      c->ngrids, ns, s, rho, ch.npts, ch.npts * nb, ch.npts, no, nb, ket[s], c->stream);
-      xc_grouped_gemm2<T>(c, gdev + ch.group_off + s * ng, ng, phi, ket[s], no * nb, ch.npts, out[s], fac, 1.0);
+      bool batches = false;
+      if constexpr (sizeof(T) == 8) {
+        batches = batches_faster(c, ch, no * nb);
+        for (int64_t b = ch.b0; batches && b < ch.b1; ++b)
+          if (c->xc_batches[b].npts > 0 && c->xc_batches[b].nwin > 0)
+            gemm64(c, batch_out(c, c->xc_batches[b], ch.g0, ch.npts, no * nb, phi, ket[s], out[s], fac));
+      }
+      if (!batches)
+        xc_grouped_gemm2<T>(c, gdev + ch.group_off + s * ng, ng, phi, ket[s], no * nb, ch.npts, out[s], fac, 1.0);
     }
   }
 }

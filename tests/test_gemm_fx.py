@@ -59,7 +59,8 @@ def _context(C, occ, e, **cfg):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("nao,nocc,natm", [(128, 64, 3), (129, 33, 4), (191, 65, 2), (257, 31, 2), (320, 130, 1)])
+@pytest.mark.parametrize("nao,nocc,natm", [(128, 64, 3), (129, 33, 4), (191, 65, 2), (257, 31, 2), (320, 130, 1),
+                                           (128, 64, 40), (129, 33, 60), (191, 65, 24), (257, 31, 24), (320, 130, 8)])
 def test_against_extended_precision(nao, nocc, natm):
     """s1mo = C^T (s1ao Cocc), two GEMMs at the edges of the 128 x 64 tiles and of the 32-wide K
     blocks: the slices add 2^-62 |a||b| and each product one rounding, so the error stays within
@@ -68,7 +69,8 @@ def test_against_extended_precision(nao, nocc, natm):
     ctx = _context(C, occ, e)
     ctx.profile(True)
     _, _, got = ctx.compute_dimless_cphf_rhs(None, None, s1)
-    assert ctx.profile_report()["gemm_fp64_tcgen05"]["launches"] > 0
+    if natm >= 8:  # (small products are left to the native kernel)
+        assert ctx.profile_report()["gemm_fp64_tcgen05"]["launches"] > 0
     sel = (s1.reshape(nao, nao, -1, order="F")[:, :, ::max(1, natm)]).astype(np.longdouble)
     got = got.reshape(nao, nocc, -1, order="F")[:, :, ::max(1, natm)]
     Cl = C.astype(np.longdouble)
