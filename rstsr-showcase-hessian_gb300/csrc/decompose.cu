@@ -11,7 +11,7 @@
 // GPU design (everything FP64, the arithmetic the reference keeps for this step):
 //   * blocked right-looking Cholesky of the lower factor L = U^T (j2c = L L^T): a one-CTA kernel
 //     factors each 64 x 64 diagonal block in shared memory (records the first non-positive
-//     pivot), a row-parallel kernel solves the panel below it, and the trailing update is one
+//     pivot), forward substitutions give the panel below it, and the trailing update is one
 //     FP64 GEMM per block;
 //   * the triangular solve X L^T = J (X = cderi, J = j3c, [nao_tp, naux] col-major) runs
 //     left-looking over 128-column blocks: S = J_k - X_<k L_k,<k^T (one tall GEMM, K grows with
@@ -39,63 +39,115 @@ unsigned grid1(int64_t n) { return (unsigned)std::max<int64_t>(1, std::min<int64
 
 // Factor the b x b diagonal block A[k0:k0+b, k0:k0+b] (lower triangle, col-major, ld lda) in
 // shared memory: A = L L^T.  info (device) receives k0 + j + 1 at the first pivot that is not
-// positive and finite (unchanged when an earlier failure was recorded).
+// positive and finite (unchanged when an earlier failure was recorded).  Bound by the serial chain
+// of its columns (square root, scaling, rank-one update); one reciprocal square root per column,
+// multiplied into the rows, instead of a division per row, and no index division in the update:
+// 100 -> 45 us for b = 64.
 __global__ void chol_diag_kernel(double* __restrict__ A, int64_t lda, int64_t k0, int b, int* info) {
-  __shared__ double a[CB][CB + 1];
+  __shared__ double a[CB][CB + 1];  // a[j][i]: column j, row i
   __shared__ int bad;
+  __shared__ double rs;
   const int t = threadIdx.x;
   for (int e = t; e < b * b; e += blockDim.x) {
     const int i = e % b, j = e / b;
-    a[i][j] = A[(k0 + i) + lda * (k0 + j)];
+    a[j][i] = A[(k0 + i) + lda * (k0 + j)];
   }
   if (t == 0) bad = 0;
   __syncthreads();
+  const int i = t % CB, l0 = t / CB;
   for (int j = 0; j < b; ++j) {
     if (t == 0) {
-      const double d = a[j][j];
+      double d = a[j][j];
       if (!(d > 0.0) || !isfinite(d)) {
         if (!bad) atomicCAS(info, 0, (int)(k0 + j + 1));
         bad = 1;
-        a[j][j] = 1.0;  // keep the arithmetic finite; the result is discarded by the host
-      } else {
-        a[j][j] = sqrt(d);
+        d = 1.0;  // keep the arithmetic finite; the result is discarded by the host
       }
+      // sqrt(d) from its reciprocal, corrected by one Newton step
+      const double r = rsqrt(d), s = d * r;
+      rs = r;
+      a[j][j] = fma(0.5 * r, fma(-s, s, d), s);
     }
     __syncthreads();
-    const double d = a[j][j];
-    for (int i = j + 1 + t; i < b; i += blockDim.x) a[i][j] /= d;
+    if (t < b && t > j) a[j][t] *= rs;
     __syncthreads();
     // trailing update of the lower triangle: a[i][l] -= a[i][j] a[l][j], j < l <= i
-    const int m = b - j - 1;
-    for (int e = t; e < m * m; e += blockDim.x) {
-      const int i = j + 1 + e % m, l = j + 1 + e / m;
-      if (l <= i) a[i][l] -= a[i][j] * a[l][j];
-    }
+    if (i < b)
+      for (int l = j + 1 + l0; l <= i; l += kThreads / CB) a[l][i] = fma(-a[j][i], a[j][l], a[l][i]);
     __syncthreads();
   }
   for (int e = t; e < b * b; e += blockDim.x) {
-    const int i = e % b, j = e / b;
-    if (i >= j) A[(k0 + i) + lda * (k0 + j)] = a[i][j];
+    const int r = e % b, j = e / b;
+    if (r >= j) A[(k0 + r) + lda * (k0 + j)] = a[j][r];
   }
 }
 
-// Panel below a factored diagonal block: rows r in [k0 + b, n), x L_kk^T = a, in place
-// (forward substitution over the b columns; one thread per row, coalesced over rows).
-__global__ void chol_panel_kernel(double* __restrict__ A, int64_t lda, int64_t n, int64_t k0, int b) {
-  __shared__ double l[CB][CB + 1];
-  for (int e = threadIdx.x; e < b * b; e += blockDim.x) {
-    const int i = e % b, j = e / b;
-    l[i][j] = i >= j ? A[(k0 + i) + lda * (k0 + j)] : 0.0;
+// Forward substitutions x_j = (v_j - sum_{q<j} L[j][q] x_q) / L[j][j] with a w x w lower factor
+// (w <= TB) for many vectors v: kTriRows vectors per CTA, vectors and factor in shared memory, the
+// update of the later elements spread over the block (a thread per vector leaves the chain of
+// w^2 / 2 FMAs and their loads to one lane: 221 us for 600 rows of 64, now ~20; the inverse of a
+// 128 block 493 us, now ~45).  Vector r's element j sits at v + r vr + j vj; with `identity` the
+// vectors start as the unit vectors e_r and are only written (the columns of inv(L)).  blockIdx.y:
+// diagonal blocks of width TB of the factor L [n, n] (ldl), one after the other.
+constexpr int kTriRows = 16;
+struct TriArgs {
+  const double* L;
+  int64_t ldl, n;       // factor of block y: L + y TB (ldl + 1), width min(TB, n - y TB)
+  double* v;
+  int64_t vr, vj, vb;   // vector, element and block strides
+  int64_t rows;
+  int identity;
+};
+__global__ void __launch_bounds__(kThreads) tri_rows_kernel(TriArgs a) {
+  extern __shared__ double sm[];  // [w][w] columns of L, [w][kTriRows] vectors, [w] reciprocals
+  const int64_t k0 = (int64_t)blockIdx.y * TB;
+  const int w = (int)min((int64_t)TB, a.n - k0);
+  double* const l = sm;
+  double* const x = sm + TB * TB;
+  double* const rd = x + TB * kTriRows;
+  const double* L = a.L + k0 * (a.ldl + 1);
+  const int t = threadIdx.x, r = t % kTriRows;
+  const int64_t r0 = (int64_t)blockIdx.x * kTriRows, rows = a.identity ? (int64_t)w : a.rows;
+  if (r0 >= rows) return;
+  for (int e = t; e < w * w; e += kThreads) {
+    const int i = e % w, j = e / w;
+    l[j * w + i] = i >= j ? L[i + a.ldl * j] : 0.0;
+  }
+  double* v = a.v + blockIdx.y * a.vb;
+  const int64_t vr = a.identity ? w : a.vr;  // (the last inverse is narrower)
+  for (int e = t; e < w * kTriRows; e += kThreads) {
+    const int j = e / kTriRows;
+    const int64_t rr = r0 + e % kTriRows;
+    x[e] = rr >= rows ? 0.0 : a.identity ? (rr == j ? 1.0 : 0.0) : v[rr * vr + j * a.vj];
   }
   __syncthreads();
-  const int64_t r = k0 + b + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (r >= n) return;
-  double* row = A + r + lda * k0;
-  for (int j = 0; j < b; ++j) {
-    double v = row[lda * j];
-    for (int q = 0; q < j; ++q) v -= row[lda * q] * l[j][q];
-    row[lda * j] = v / l[j][j];
+  if (t < w) rd[t] = 1.0 / l[t * w + t];
+  __syncthreads();
+  // (the inverse's columns are zero above their first row)
+  for (int j = a.identity ? (int)r0 : 0; j < w; ++j) {
+    const double xj = x[j * kTriRows + r] * rd[j];
+    for (int i = j + 1 + t / kTriRows; i < w; i += kThreads / kTriRows)
+      x[i * kTriRows + r] = fma(-l[j * w + i], xj, x[i * kTriRows + r]);
+    __syncthreads();
+    if (t < kTriRows) x[j * kTriRows + t] *= rd[j];  // (not read again by the updates)
   }
+  __syncthreads();
+  for (int e = t; e < w * kTriRows; e += kThreads) {
+    const int j = e / kTriRows;
+    const int64_t rr = r0 + e % kTriRows;
+    if (rr < rows) v[rr * vr + j * a.vj] = x[e];
+  }
+}
+constexpr int kTriSmem = (TB * TB + TB * kTriRows + TB) * 8;
+void launch_tri_rows(cphf_ctx* c, const TriArgs& a, int64_t rows, int64_t blocks) {
+  static bool attr = false;
+  if (!attr) {
+    CPHF_CUDA(cudaFuncSetAttribute(tri_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTriSmem));
+    attr = true;
+  }
+  tri_rows_kernel<<<dim3((unsigned)div_up(rows, kTriRows), (unsigned)blocks), kThreads, kTriSmem, c->stream>>>(a);
+  count_launch();
+  CPHF_CUDA(cudaGetLastError());
 }
 
 // U = L^T (upper, zeros below the diagonal) from the lower factor in A; min |diag| -> dmin bits.
@@ -106,32 +158,6 @@ __global__ void chol_upper_kernel(const double* __restrict__ A, int64_t n, doubl
     const int64_t i = e % n, j = e / n;  // U[i, j]
     U[e] = i <= j ? A[j + n * i] : 0.0;
     if (i == j) atomicMin(dmin, (unsigned long long)__double_as_longlong(fabs(A[i + n * i])));
-  }
-}
-
-// inv(L_kk) for every diagonal block of width <= TB of the lower factor L [n, n]: block k is
-// written to inv + k * TB * TB as a w x w col-major lower-triangular matrix; one CTA per block,
-// one thread per column of the inverse (forward substitution on L_kk e_j).
-__global__ void tri_inv_blocks_kernel(const double* __restrict__ L, int64_t n, double* __restrict__ inv) {
-  extern __shared__ double sl[];  // [TB][TB + 1]
-  const int64_t k0 = (int64_t)blockIdx.x * TB;
-  const int w = (int)(n - k0 < TB ? n - k0 : TB);
-  for (int e = threadIdx.x; e < w * w; e += blockDim.x) {
-    const int i = e % w, j = e / w;
-    sl[i * (TB + 1) + j] = i >= j ? L[(k0 + i) + n * (k0 + j)] : 0.0;
-  }
-  __syncthreads();
-  const int j = threadIdx.x;
-  if (j >= w) return;
-  double* x = inv + (int64_t)blockIdx.x * TB * TB + (int64_t)w * j;  // column j of the inverse
-  for (int i = 0; i < w; ++i) {
-    if (i < j) {
-      x[i] = 0.0;
-      continue;
-    }
-    double v = i == j ? 1.0 : 0.0;
-    for (int q = j; q < i; ++q) v -= sl[i * (TB + 1) + q] * x[q];
-    x[i] = v / sl[i * (TB + 1) + i];
   }
 }
 
@@ -247,8 +273,11 @@ int cholesky_lower(cphf_ctx* c, double* A, int64_t n, int* info_dev) {
     count_launch();
     const int64_t rest = n - k0 - b;
     if (rest <= 0) break;
-    chol_panel_kernel<<<(unsigned)div_up(rest, 128), 128, 0, s>>>(A, n, n, k0, b);
-    count_launch();
+    TriArgs p{};  // rows below the block: x L_kk^T = a
+    p.L = A + k0 * (n + 1); p.ldl = n; p.n = b;
+    p.v = A + (k0 + b) + n * k0; p.vr = 1; p.vj = n;
+    p.rows = rest;
+    launch_tri_rows(c, p, rest, 1);
     GemmDesc g;  // A[r, r'] -= L[r, k] L[r', k], r, r' >= k0 + b (full square of the trailing block)
     g.M = rest; g.N = rest; g.K = b;
     g.A = A + (k0 + b) + n * k0; g.a_m = 1; g.a_k = n;
@@ -353,15 +382,11 @@ void solve_by_j2c_right(cphf_ctx* c, double* J, int64_t n, int64_t naux, DecompW
   const double* L = w.A.as<double>();  // lower factor from j2c_cholesky
   const int64_t nblk = div_up(naux, TB);
   w.inv.ensure((size_t)nblk * TB * TB * 8, c->counter());
-  static bool attr = false;
-  const int smem = TB * (TB + 1) * 8;
-  if (!attr) {
-    CPHF_CUDA(cudaFuncSetAttribute(tri_inv_blocks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    attr = true;
-  }
-  tri_inv_blocks_kernel<<<(unsigned)nblk, TB, smem, s>>>(L, naux, w.inv.as<double>());
-  count_launch();
-  CPHF_CUDA(cudaGetLastError());
+  TriArgs inv{};  // inv(L_kk) of every diagonal block, w x w col-major at k TB TB
+  inv.L = L; inv.ldl = naux; inv.n = naux;
+  inv.v = w.inv.as<double>(); inv.vj = 1; inv.vb = (int64_t)TB * TB;
+  inv.identity = 1;
+  launch_tri_rows(c, inv, TB, nblk);
   if (n == 0) return;
   w.S.ensure((size_t)n * TB * 8, c->counter());
   double* S = w.S.as<double>();
