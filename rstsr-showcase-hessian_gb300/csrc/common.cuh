@@ -88,4 +88,12 @@ inline void count_launch(int64_t n = 1) {
 
 inline int64_t div_up(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
+// Row length of the 16-bit operand planes that TMA reads in 64- and 128-byte rows: a multiple of
+// 64 bytes (the fill of shared memory runs at 35 / 50 B/clk and SM then, at 30 / 44 with rows of
+// 1200 bytes), unless that would pad a short row by more than an eighth; then of 16 bytes.
+inline int64_t plane_ld(int64_t n) {
+  const int64_t l = div_up(n, 32) * 32;
+  return 8 * (l - n) <= n ? l : div_up(n, 8) * 8;
+}
+
 }  // namespace cphf

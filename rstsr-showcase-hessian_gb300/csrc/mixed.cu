@@ -148,7 +148,7 @@ static void rijk_response_lowp(cphf_ctx* c, float* const* bra, int64_t nb, float
                    });
         // W / term-2 chunk: W's two FP16 planes, nocc-wide rows, within the budget and with
         // 32-bit plane offsets
-        const int64_t ldj = (no + 7) / 8 * 8;
+        const int64_t ldj = plane_ld(no);
         int64_t np_w = std::max<int64_t>(1, std::min<int64_t>(naux, L.budget / std::max<int64_t>(4 * no * nb * ldj, 1)));
         np_w = std::max<int64_t>(1, std::min<int64_t>(np_w, ((int64_t)INT32_MAX - 1) / std::max<int64_t>(no * nb * ldj, 1)));
         for (int64_t P0 = 0; P0 < naux; P0 += np_w)

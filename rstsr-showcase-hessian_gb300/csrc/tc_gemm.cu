@@ -10,15 +10,8 @@
 // FP32 in tensor memory; the dropped lo*lo term and the FP32 accumulation leave ~1e-6
 // relative error, removed by the FP64 defect correction of the mixed solve.
 //
-// Kernel structure (one CTA per SM, 4 warps):
-//   warp 0 lane 0  -- TMA producer: 3-D tiled loads (K = nu, row = mu or n, P) of the four
-//                     planes into a 2-stage ring of 128B-swizzled shared-memory tiles (K = 64);
-//   warp 1 lane 0  -- MMA issuer: tcgen05.mma.cta_group::1.kind::f16 (M=128, N=256, K=16),
-//                     tcgen05.commit frees a stage when its MMAs retire;
-//   warp 2         -- TMEM allocation (256 FP32 columns) and release;
-//   warps 0-3      -- epilogue: tcgen05.ld of the 128 x 256 accumulator, scaled and
-//                     atomically added to out (split over P ranges across CTAs).
-// Every mbarrier wait is bounded; on expiry the kernel records an error flag and returns.
+// The contraction itself runs on CTA pairs (tc_pair.cu); this file holds the FP16 planes of the
+// cderi, the chunking over aux functions and the W generation.
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <cudaTypedefs.h>
@@ -30,6 +23,7 @@
 
 #include "kernels.cuh"
 #include "tc_gemm.cuh"
+#include "tc_pair.cuh"
 #include "tc_ptx.cuh"
 
 namespace cphf {
@@ -42,138 +36,6 @@ constexpr int A_TILE = BM * BK * 2;  // bytes, FP16
 constexpr int B_TILE = BN * BK * 2;
 constexpr int STAGE_BYTES = 2 * A_TILE + 2 * B_TILE;  // hi + lo planes of both operands
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*barriers*/ + 1024 /*alignment*/;
-constexpr int TMEM_COLS = 256;
-
-struct TcArgs {
-  float* out;
-  int64_t ld_out;   // out[mu + ld_out * n]
-  int M, N;         // mu rows (nao), n columns
-  int nkb;          // K blocks of 64 per aux function
-  int np;           // aux functions in this chunk
-  int p_per_cta;    // aux functions per CTA (P split)
-  int pA0;          // global aux index of the chunk's first function (A coordinate)
-  int m_tiles;
-  const float* scale;  // device: alpha / (sA * sT), or null (1)
-  const double* rowscale;  // per-row / per-column factors of the result (null: 1), the scales of
-  const double* colscale;  // row- / column-scaled operand planes
-  int* err;
-};
-
-__global__ void __launch_bounds__(128, 1)
-    tc_term1_kernel(const __grid_constant__ CUtensorMap mAh, const __grid_constant__ CUtensorMap mAl,
-                    const __grid_constant__ CUtensorMap mBh, const __grid_constant__ CUtensorMap mBl, TcArgs args) {
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 1);
-  const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + STAGES), accum = smem_u32(bars + 2 * STAGES);
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m_tile = blockIdx.x % args.m_tiles, n_tile = blockIdx.x / args.m_tiles;
-  const int m0 = m_tile * BM, n0 = n_tile * BN;
-  const int pbeg = blockIdx.y * args.p_per_cta;
-  const int pend = min(args.np, pbeg + args.p_per_cta);
-  const int total = (pend - pbeg) * args.nkb;
-
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
-      mbar_init(full0 + 8 * s, 1);
-      mbar_init(empty0 + 8 * s, 1);
-    }
-    mbar_init(accum, 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  if (warp == 2) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(TMEM_COLS)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = *tmem_slot;
-
-  if (total > 0) {
-    if (warp == 0 && lane == 0) {
-      // producer
-      int issued = 0;
-      for (int it = 0; it < total; ++it) {
-        const int s = it % STAGES;
-        const uint32_t ph = (it / STAGES) & 1;
-        if (!mbar_wait(empty0 + 8 * s, ph ^ 1, args.err)) break;
-        issued = it + 1;
-        const uint32_t full = full0 + 8 * s;
-        mbar_expect_tx(full, STAGE_BYTES);
-        const int P = pbeg + it / args.nkb;
-        const int k0 = (it % args.nkb) * BK;
-        uint8_t* st = smem + s * STAGE_BYTES;
-        tma_load_3d(smem_u32(st), &mAh, full, k0, m0, args.pA0 + P);
-        tma_load_3d(smem_u32(st + A_TILE), &mAl, full, k0, m0, args.pA0 + P);
-        tma_load_3d(smem_u32(st + 2 * A_TILE), &mBh, full, k0, n0, P);
-        tma_load_3d(smem_u32(st + 2 * A_TILE + B_TILE), &mBl, full, k0, n0, P);
-      }
-      // drain: the copies of the last round of every stage have landed before the CTA may exit
-      for (int it = max(0, issued - STAGES); it < issued; ++it) {
-        mbar_wait(full0 + 8 * (it % STAGES), (it / STAGES) & 1, nullptr);
-      }
-    } else if (warp == 1 && lane == 0) {
-      // MMA issuer
-      constexpr uint32_t idesc = instr_desc_f16(BM, BN, false);
-      for (int it = 0; it < total; ++it) {
-        const int s = it % STAGES;
-        const uint32_t ph = (it / STAGES) & 1;
-        if (!mbar_wait(full0 + 8 * s, ph, args.err)) break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t st = smem_u32(smem + s * STAGE_BYTES);
-        const uint64_t ah = smem_desc<128>(st), al = smem_desc<128>(st + A_TILE);
-        const uint64_t bh = smem_desc<128>(st + 2 * A_TILE), bl = smem_desc<128>(st + 2 * A_TILE + B_TILE);
-#pragma unroll
-        for (int k = 0; k < BK / 16; ++k) {
-          const uint64_t dk = (uint64_t)((k * 32) >> 4);  // 16 FP16 = 32 B along K inside the swizzle atom
-          mma_f16(tmem, ah + dk, bh + dk, idesc, (it > 0 || k > 0) ? 1u : 0u);
-          mma_f16(tmem, ah + dk, bl + dk, idesc, 1u);
-          mma_f16(tmem, al + dk, bh + dk, idesc, 1u);
-        }
-        mma_commit(empty0 + 8 * s);
-      }
-      mma_commit(accum);  // also covers an early exit: arrives when the issued MMAs retire
-    }
-    __syncwarp();
-    // epilogue: all four warps, warp w owns TMEM lanes [32 w, 32 w + 32)
-    // warp-uniform decision: tcgen05.ld is a whole-warp instruction
-    const bool have = __all_sync(0xffffffffu, mbar_wait(accum, 0, args.err) && *(volatile int*)args.err == 0);
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (have) {
-      const int row = m0 + warp * 32 + lane;
-      const float scale = (args.scale ? *args.scale : 1.f) *
-                          ((args.rowscale && row < args.M) ? (float)args.rowscale[row] : 1.f);
-      for (int c = 0; c < BN / 32; ++c) {
-        float v[32];
-        tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(c * 32), v);
-        // the chunk's 32 column factors: one load per lane, broadcast by shuffles
-        const int nl = n0 + c * 32 + lane;
-        const float csl = (args.colscale && nl < args.N) ? (float)args.colscale[nl] : 1.f;
-        float cs[32];
-#pragma unroll
-        for (int j = 0; j < 32; ++j) cs[j] = __shfl_sync(0xffffffffu, csl, j);
-        if (row < args.M) {
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const int n = n0 + c * 32 + j;
-            if (n < args.N) atomicAdd(args.out + row + args.ld_out * (int64_t)n, scale * cs[j] * v[j]);
-          }
-        }
-      }
-    }
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  if (warp == 2) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
-  }
-}
 
 // ---- W generation: one persistent split-FP16 GEMM per aux chunk ---------------------------
 //   W_P[(j,a), i] = sum_nu bra[nu, j, a] Z_P[nu, i]   (term 2's cderi_oxo_1, src/ri_jk/hess_r.rs:172-176,
@@ -183,7 +45,7 @@ __global__ void __launch_bounds__(128, 1)
 // planes of W * wscale (one power of two per chunk, from an upper bound of |W|) straight
 // into the layout term 2 reads, out[j + ldj i + s_a a + s_p Pl] (K = j).
 //   warp 0 lane 0 -- TMA producer over the CTA's tiles, 2-stage ring of the four planes;
-//   warp 1        -- TMEM owner (2 x 256 columns); lane 0 issues the MMAs of tile t into
+//   warp 1        -- TMEM owner (2 x 256 columns); an elected lane issues the MMAs of tile t into
 //                    accumulator t & 1 while the epilogue drains the other;
 //   warps 2-9     -- epilogue: TMEM lane quarter warp & 3, column half (warp - 2) / 4.
 // Tiles in a grouped raster: group_m row tiles walk every column tile with rows fastest, so a
@@ -266,35 +128,39 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
     }
     // the copies of the last round of every stage have landed before the CTA may exit
     for (int i = max(0, issued - STAGES); i < issued; ++i) mbar_wait(full0 + 8 * (i % STAGES), (i / STAGES) & 1, nullptr);
-  } else if (warp == 1 && lane == 0) {
+  } else if (warp == 1) {
     constexpr uint32_t idesc = instr_desc_f16(BM, BN, false);
+    const bool el = elect_one();
     int it = 0, lt = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++lt) {
       const int b = lt & 1;
-      if (!mbar_wait(acce0 + 8 * b, ((lt >> 1) & 1) ^ 1, args.err)) break;
+      if (!__all_sync(0xffffffffu, mbar_wait(acce0 + 8 * b, ((lt >> 1) & 1) ^ 1, args.err))) break;
       fence_after_sync();
       const uint32_t acc = tmem + (uint32_t)(b * WG_ACC);
       for (int kb = 0; kb < args.nkb; ++kb, ++it) {
         const int s = it % STAGES;
-        if (!mbar_wait(full0 + 8 * s, (it / STAGES) & 1, args.err)) { ok = false; break; }
+        if (!__all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, (it / STAGES) & 1, args.err))) { ok = false; break; }
         fence_after_sync();
-        const uint32_t st = smem_u32(smem + s * STAGE_BYTES);
-        const uint64_t ah = smem_desc<128>(st), al = smem_desc<128>(st + A_TILE);
-        const uint64_t bh = smem_desc<128>(st + 2 * A_TILE), bl = smem_desc<128>(st + 2 * A_TILE + B_TILE);
+        const uint64_t ah = smem_desc<128>(smem_u32(smem + s * STAGE_BYTES)), bh = ah + desc_off(2 * A_TILE);
+        if (el) {
 #pragma unroll
-        for (int k = 0; k < BK / 16; ++k) {
-          const uint64_t dk = (uint64_t)((k * 32) >> 4);
-          mma_f16(acc, ah + dk, bh + dk, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-          mma_f16(acc, ah + dk, bl + dk, idesc, 1u);
-          mma_f16(acc, al + dk, bh + dk, idesc, 1u);
+          for (int k = 0; k < BK / 16; ++k) {
+            const uint64_t dk = desc_off(k * 32);
+            mma_f16(acc, ah + dk, bh + dk, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+            mma_f16(acc, ah + dk, bh + (desc_off(B_TILE) + dk), idesc, 1u);
+            mma_f16(acc, ah + (desc_off(A_TILE) + dk), bh + dk, idesc, 1u);
+          }
+          mma_commit(empty0 + 8 * s);
         }
-        mma_commit(empty0 + 8 * s);
+        __syncwarp();
       }
-      if (ok) mma_commit(accf0 + 8 * b);
+      if (ok && el) mma_commit(accf0 + 8 * b);
+      __syncwarp();
     }
     // every issued MMA has retired before TMEM is released (also after an early exit)
-    mma_commit(done);
+    if (el) mma_commit(done);
+    __syncwarp();
     mbar_wait(done, 0, nullptr);
   } else if (warp >= 2) {
     const int q = warp & 3, h = (warp - 2) >> 2;
@@ -405,7 +271,7 @@ __global__ void split_cderi_kernel(const double* __restrict__ Bd, int64_t nao, i
     const int64_t r = t / ldk;  // P * nao + mu
     if (nu < nao) {
       const int64_t P = r / nao, mu = r % nao;
-      split_f16(Bd[mu + nao * nu + nao * nao * P], s, hi + t, lo + t);
+      split_f16(Bd[nu + nao * mu + nao * nao * P], s, hi + t, lo + t);  // (symmetric: read along nu)
     } else {
       hi[t] = __float2half(0.f);
       lo[t] = __float2half(0.f);
@@ -486,7 +352,7 @@ bool tc_available(cphf_ctx* c) {
   if (major != 10 || encode_fn() == nullptr) return false;
   static bool attr_set = false;
   if (!attr_set) {
-    if (cudaFuncSetAttribute(tc_term1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess ||
+    if (!pair_available(c->device) ||
         cudaFuncSetAttribute(tc_wgen_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess) {
       cudaGetLastError();
       return false;
@@ -498,7 +364,7 @@ bool tc_available(cphf_ctx* c) {
 
 void tc_prepare_cderi(cphf_ctx* c, DevBuf& hi, DevBuf& lo, int64_t& ldk) {
   const int64_t nao = c->nao, naux = c->naux;
-  ldk = (nao + 7) / 8 * 8;
+  ldk = plane_ld(nao);
   // power-of-two scale from max |B|
   DevBuf mx;
   mx.ensure(sizeof(unsigned), nullptr);
@@ -540,39 +406,24 @@ void tc_k_term1(cphf_ctx* c, const DevBuf& Bhi, const DevBuf& Blo, int64_t ldk, 
   unsigned* mx = L.s_acc.as<unsigned>();
   float* scale = reinterpret_cast<float*>(mx + 4);
   L.err.ensure(sizeof(int), c->counter());
-  const int m_tiles = (int)div_up(nao, BM), n_tiles = (int)div_up(N, BN);
-  const int nkb = (int)div_up(nao, BK);
-  const int ppc = 16;
   for (int64_t P0 = 0; P0 < naux; P0 += np) {
     const int64_t npc = std::min<int64_t>(np, naux - P0);
     // FP16 planes of T_P[nu, (i,a)] = sum_j bra[nu, j, a] O_P[j, i] and their scale from the
     // T generator (no FP32 T in HBM)
     tplanes(P0, npc, Thi.as<__half>(), Tlo.as<__half>(), mx, scale);
-    const CUtensorMap mAh = make_map(Bhi.p, nao, nao, naux, ldk, BM);
-    const CUtensorMap mAl = make_map(Blo.p, nao, nao, naux, ldk, BM);
-    const CUtensorMap mBh = make_map(Thi.p, nao, N, npc, ldk, BN);
-    const CUtensorMap mBl = make_map(Tlo.p, nao, N, npc, ldk, BN);
-    TcArgs a;
-    a.out = out;
-    a.ld_out = nao;
-    a.M = (int)nao;
-    a.N = (int)N;
-    a.nkb = nkb;
-    a.np = (int)npc;
-    a.p_per_cta = ppc;
-    a.pA0 = (int)P0;
-    a.m_tiles = m_tiles;
-    a.scale = scale + 1;
-    a.rowscale = nullptr;
-    a.colscale = nullptr;
-    a.err = L.err.as<int>();
-    dim3 grid((unsigned)(m_tiles * n_tiles), (unsigned)div_up(npc, ppc));
+    PairTerm t{};
+    t.x = PairPlanes{{Bhi.p, Blo.p}, nao, ldk, naux, 0};
+    t.y = PairPlanes{{Thi.p, Tlo.p}, N, ldk, npc, 0};
+    t.x_off = P0;
+    t.np = npc; t.M = nao; t.N = N; t.K = nao;
+    t.scale = scale + 1;
+    t.out = out;
+    t.ld_out = nao;
+    t.err = L.err.as<int>();
     // algorithmic FLOPs of the contraction (the tensor pipe executes three split products);
     // bytes: the FP16 planes of both operands read once
     ProfScope ps(c, PROF_TC_KTERM, 2.0 * nao * N * nao * npc, 4.0 * nao * npc * (nao + N));
-    tc_term1_kernel<<<grid, 128, SMEM_BYTES, c->stream>>>(mAh, mAl, mBh, mBl, a);
-    count_launch();
-    CPHF_CUDA(cudaGetLastError());
+    pair_split2(c, t);
   }
 }
 
@@ -580,33 +431,18 @@ void tc_planes_term(cphf_ctx* c, const __half* a_hi, const __half* a_lo, int64_t
                     const __half* b_hi, const __half* b_lo, int64_t npc, int64_t M, int64_t N, int64_t K, int64_t ld,
                     const double* rowscale, const double* colscale, float* out, int64_t ld_out, int* err,
                     const float* scale) {
-  if (M <= 0 || N <= 0 || K <= 0 || npc <= 0) return;
-  const int m_tiles = (int)div_up(M, BM), n_tiles = (int)div_up(N, BN);
-  const CUtensorMap mAh = make_map(a_hi, K, M, a_depth, ld, BM);
-  const CUtensorMap mAl = make_map(a_lo, K, M, a_depth, ld, BM);
-  const CUtensorMap mBh = make_map(b_hi, K, N, npc, ld, BN);
-  const CUtensorMap mBl = make_map(b_lo, K, N, npc, ld, BN);
-  TcArgs a;
-  a.out = out;
-  a.ld_out = ld_out;
-  a.M = (int)M;
-  a.N = (int)N;
-  a.nkb = (int)div_up(K, BK);
-  a.np = (int)npc;
-  // one K range per tile unless the tiles alone leave SMs idle
-  const int64_t tiles = (int64_t)m_tiles * n_tiles;
-  const int64_t ranges = std::max<int64_t>(1, std::min<int64_t>(npc, div_up(2 * (int64_t)c->num_sms, tiles)));
-  a.p_per_cta = (int)div_up(npc, ranges);
-  a.pA0 = (int)a_off;
-  a.m_tiles = m_tiles;
-  a.scale = scale;
-  a.rowscale = rowscale;
-  a.colscale = colscale;
-  a.err = err;
-  dim3 grid((unsigned)tiles, (unsigned)div_up(npc, a.p_per_cta));
-  tc_term1_kernel<<<grid, 128, SMEM_BYTES, c->stream>>>(mAh, mAl, mBh, mBl, a);
-  count_launch();
-  CPHF_CUDA(cudaGetLastError());
+  PairTerm t{};
+  t.x = PairPlanes{{a_hi, a_lo}, M, ld, a_depth, 0};
+  t.y = PairPlanes{{b_hi, b_lo}, N, ld, npc, 0};
+  t.x_off = a_off;
+  t.np = npc; t.M = M; t.N = N; t.K = K;
+  t.rowscale = rowscale;
+  t.colscale = colscale;
+  t.scale = scale;
+  t.out = out;
+  t.ld_out = ld_out;
+  t.err = err;
+  pair_split2(c, t);
 }
 
 void tc_wgen_planes(cphf_ctx* c, const __half* a_hi, const __half* a_lo, int64_t M, const __half* b_hi,

@@ -25,11 +25,12 @@
 // adds alpha 2^(eA + eB) (hi + lo) into the FP64 output (terms 1 and 2, split over K ranges
 // across CTAs) or stores the pair 2^(eA + eB) (hi, lo) into a staging array (T, W).
 //
-// Kernel structure (one CTA per SM, 4 warps):
+// Terms 1 and 2 run on CTA pairs (tc_pair.cu); the kernels below generate T and W and evaluate the
+// XC term.  Kernel structure (one CTA per SM, 4 warps):
 //   warp 0 lane 0  -- TMA producer: 3-D tiled loads of the 6 + 6 slice tiles (K = 32 wide,
 //                     64B swizzle) into a 2-stage ring;
-//   warp 1 lane 0  -- MMA issuer: 21 x tcgen05.mma.kind::f16 (BF16, M=128, N=BN, K=16)
-//                     per K step into 4 accumulators (4 x BN TMEM columns);
+//   warp 1         -- MMA issuer (warp-uniform, one elected lane): 21 x tcgen05.mma.kind::f16
+//                     (BF16, M=128, N=BN, K=16) per K step into 4 accumulators (4 x BN TMEM columns);
 //   warp 2         -- TMEM allocation and release;
 //   warps 0-3      -- epilogue.
 // Every mbarrier wait is bounded; on expiry the kernel raises the error flag and returns.
@@ -53,6 +54,7 @@
 #include "kernels.cuh"
 #include "tc_gemm.cuh"
 #include "tc_ozaki.cuh"
+#include "tc_pair.cuh"
 #include "slices.cuh"
 #include "tc_ptx.cuh"
 
@@ -195,41 +197,45 @@ __global__ void __launch_bounds__(128, 1)
       }
       for (int it = max(0, issued - STAGES); it < issued; ++it)
         mbar_wait(full0 + 8 * (it % STAGES), (it / STAGES) & 1, nullptr);
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1) {
       // MMA issuer
       constexpr uint32_t idesc = instr_desc_f16(BM, BN, PR::BF16);
+      const bool el = elect_one();
       for (int it = 0; it < total; ++it) {
         const int s = it % STAGES;
         const uint32_t ph = (it / STAGES) & 1;
-        if (!mbar_wait(full0 + 8 * s, ph, args.err)) break;
+        if (!__all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, ph, args.err))) break;
         fence_after_sync();
-        const uint32_t st = smem_u32(smem + s * C::STAGE_BYTES);
-        const uint32_t sb = st + PR::S * C::A_TILE;
+        const uint64_t da = smem_desc<64>(smem_u32(smem + s * C::STAGE_BYTES));
+        const uint64_t db = da + desc_off(PR::S * C::A_TILE);
+        if (el) {
 #pragma unroll
-        for (int k = 0; k < BK / 16; ++k) {
-          const uint64_t dk = (uint64_t)((k * 32) >> 4);  // 16 elements = 32 B along K inside the swizzle row
-          if constexpr (PR::NACC == 4) {
+          for (int k = 0; k < BK / 16; ++k) {
+            const uint64_t dk = desc_off(k * 32);  // 16 elements = 32 B along K inside the swizzle row
+            if constexpr (PR::NACC == 4) {
 #pragma unroll
-            for (int g = 0; g < PR::S; ++g) {
+              for (int g = 0; g < PR::S; ++g) {
 #pragma unroll
-              for (int t = 0; t <= g; ++t) {
-                const int u = g - t;
-                const int acc = g < 3 ? g : 3;
-                const bool first = it == 0 && k == 0 && t == 0 && g <= 3;
-                mma_f16(tmem + (uint32_t)(acc * BN), smem_desc<64>(st + t * C::A_TILE) + dk,
-                        smem_desc<64>(sb + u * C::B_TILE) + dk, idesc, first ? 0u : 1u);
+                for (int t = 0; t <= g; ++t) {
+                  const int acc = g < 3 ? g : 3;
+                  const bool first = it == 0 && k == 0 && t == 0 && g <= 3;
+                  mma_f16(tmem + (uint32_t)(acc * BN), da + (desc_off(t * C::A_TILE) + dk),
+                          db + (desc_off((g - t) * C::B_TILE) + dk), idesc, first ? 0u : 1u);
+                }
               }
+            } else {
+              // hi*hi + hi*lo + lo*hi
+              mma_f16(tmem, da + dk, db + dk, idesc, (it > 0 || k > 0) ? 1u : 0u);
+              mma_f16(tmem, da + dk, db + (desc_off(C::B_TILE) + dk), idesc, 1u);
+              mma_f16(tmem, da + (desc_off(C::A_TILE) + dk), db + dk, idesc, 1u);
             }
-          } else {
-            // hi*hi + hi*lo + lo*hi
-            mma_f16(tmem, smem_desc<64>(st) + dk, smem_desc<64>(sb) + dk, idesc, (it > 0 || k > 0) ? 1u : 0u);
-            mma_f16(tmem, smem_desc<64>(st) + dk, smem_desc<64>(sb + C::B_TILE) + dk, idesc, 1u);
-            mma_f16(tmem, smem_desc<64>(st + C::A_TILE) + dk, smem_desc<64>(sb) + dk, idesc, 1u);
           }
+          mma_commit(empty0 + 8 * s);
         }
-        mma_commit(empty0 + 8 * s);
+        __syncwarp();
       }
-      mma_commit(accum);  // arrives when every issued MMA has retired (also after an early exit)
+      if (el) mma_commit(accum);  // arrives when every issued MMA has retired (also after an early exit)
+      __syncwarp();
     }
     __syncwarp();
     // warp-uniform decision: tcgen05.ld is a whole-warp instruction
@@ -468,48 +474,54 @@ __global__ void __launch_bounds__(320, PR::NACC == 4 ? 1 : 2)
       }
       for (int it = max(0, issued - STAGES); it < issued; ++it)
         mbar_wait(full0 + 8 * (it % STAGES), (it / STAGES) & 1, nullptr);
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1) {
       // MMA issuer
       constexpr uint32_t idesc = instr_desc_f16(BM, BN, PR::BF16);
+      const bool el = elect_one();
       bool ok = true;
       for (int p = 0; p < nP && ok; ++p) {
         const int b = p & 1;
-        if (!mbar_wait(acce0 + 8 * b, ((p >> 1) & 1) ^ 1, args.err)) break;
+        if (!__all_sync(0xffffffffu, mbar_wait(acce0 + 8 * b, ((p >> 1) & 1) ^ 1, args.err))) break;
         fence_after_sync();
         const uint32_t acc_base = tmem + (uint32_t)b * ACC;
         for (int kb = 0; kb < nkb; ++kb) {
           const int it = p * nkb + kb;
           const int s = it % STAGES;
-          if (!mbar_wait(full0 + 8 * s, (it / STAGES) & 1, args.err)) { ok = false; break; }
+          if (!__all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, (it / STAGES) & 1, args.err))) { ok = false; break; }
           fence_after_sync();
-          const uint32_t st = smem_u32(smem + s * C::STAGE_BYTES);
-          const uint32_t sb = st + PR::S * C::A_TILE;
+          const uint64_t da = smem_desc<64>(smem_u32(smem + s * C::STAGE_BYTES));
+          const uint64_t db = da + desc_off(PR::S * C::A_TILE);
+          if (el) {
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {
-            const uint64_t dk = (uint64_t)((k * 32) >> 4);
-            if constexpr (PR::NACC == 4) {
+            for (int k = 0; k < BK / 16; ++k) {
+              const uint64_t dk = desc_off(k * 32);
+              if constexpr (PR::NACC == 4) {
 #pragma unroll
-              for (int g = 0; g < PR::S; ++g) {
+                for (int g = 0; g < PR::S; ++g) {
 #pragma unroll
-                for (int t = 0; t <= g; ++t) {
-                  const int acc = g < 3 ? g : 3;
-                  const bool first = kb == 0 && k == 0 && t == 0 && g <= 3;
-                  mma_f16(acc_base + (uint32_t)(acc * BN), smem_desc<64>(st + t * C::A_TILE) + dk,
-                          smem_desc<64>(sb + (g - t) * C::B_TILE) + dk, idesc, first ? 0u : 1u);
+                  for (int t = 0; t <= g; ++t) {
+                    const int acc = g < 3 ? g : 3;
+                    const bool first = kb == 0 && k == 0 && t == 0 && g <= 3;
+                    mma_f16(acc_base + (uint32_t)(acc * BN), da + (desc_off(t * C::A_TILE) + dk),
+                            db + (desc_off((g - t) * C::B_TILE) + dk), idesc, first ? 0u : 1u);
+                  }
                 }
+              } else {
+                mma_f16(acc_base, da + dk, db + dk, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                mma_f16(acc_base, da + dk, db + (desc_off(C::B_TILE) + dk), idesc, 1u);
+                mma_f16(acc_base, da + (desc_off(C::A_TILE) + dk), db + dk, idesc, 1u);
               }
-            } else {
-              mma_f16(acc_base, smem_desc<64>(st) + dk, smem_desc<64>(sb) + dk, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-              mma_f16(acc_base, smem_desc<64>(st) + dk, smem_desc<64>(sb + C::B_TILE) + dk, idesc, 1u);
-              mma_f16(acc_base, smem_desc<64>(st + C::A_TILE) + dk, smem_desc<64>(sb) + dk, idesc, 1u);
             }
+            mma_commit(empty0 + 8 * s);
           }
-          mma_commit(empty0 + 8 * s);
+          __syncwarp();
         }
-        if (ok) mma_commit(accf0 + 8 * b);  // accumulator set b complete when these MMAs retire
+        if (ok && el) mma_commit(accf0 + 8 * b);  // accumulator set b complete when these MMAs retire
+        __syncwarp();
       }
       // every issued MMA has retired before TMEM is released (also after an early exit)
-      mma_commit(done);
+      if (el) mma_commit(done);
+      __syncwarp();
       mbar_wait(done, 0, nullptr);
     } else if (warp >= 2) {
       // epilogue: TMEM lane quarter q, 32-column chunk c
@@ -1230,6 +1242,27 @@ void launch_split(cphf_ctx* c, OzState& z, const CUtensorMap& mA, const CUtensor
   launch_split_raw<PR, BN>(c, mA, mB, a);
 }
 
+// exact split-K contraction on CTA pairs: K blocks per pair tuned once per shape (candidates run
+// into a scratch output, the real one accumulates)
+void launch_pair_exact(cphf_ctx* c, OzState& z, const PairTerm& t, int slices) {
+  const TuneKey key{7000 + slices, t.M, t.N, t.K, t.np};
+  auto& tab = tune_table();
+  int best = KB_PER_CTA;
+  if (!tab.find(key, best) && !capturing(c->stream)) {
+    z.tune_out.ensure((size_t)t.ld_out * t.N * 8, c->counter());
+    PairTerm s = t;
+    s.out = z.tune_out.p;
+    float best_ms = 0.f;
+    for (int kb : {KB_PER_CTA, KB_PER_CTA / 2, KB_PER_CTA / 3}) {
+      if (div_up(t.np * div_up(t.K, BK), kb) > 65535) continue;
+      const float ms = time_launch(c->stream, [&] { pair_exact(c, s, slices, kb); });
+      if (best_ms == 0.f || ms < best_ms) best_ms = ms, best = kb;
+    }
+    tab.put(key, best);
+  }
+  pair_exact(c, t, slices, best);
+}
+
 // batched contraction over a.np aux functions: grid (aux ranges, tiles)
 template <class PR, int EPI>
 void launch_batched_raw(cphf_ctx* c, const CUtensorMap& mA, const CUtensorMap& mB, OzArgs a, int waves) {
@@ -1304,7 +1337,7 @@ void launch_tgen_resident(cphf_ctx* c, const CUtensorMap& mA, const CUtensorMap&
 
 // 3-D FP16 map of T's planes for the TMA stores of the resident T generation: dims {nu (nao),
 // n = i + nocc a (N), Pl (npc)}, row stride ldt, box {32 nu, ni, 1} (one epilogue warp's part,
-// ni of its 64 columns), no swizzle (the staged tile is [ni][32] dense)
+// ni of its columns), no swizzle (the staged tile is [ni][32] dense)
 CUtensorMap make_t_store_map(const __half* base, int64_t nao, int64_t N, int64_t npc, int64_t ldt, int64_t ni) {
   CUtensorMap m;
   std::memset(&m, 0, sizeof(m));
@@ -1357,7 +1390,7 @@ bool oz_supported(const cphf_ctx* c) {
 
 void oz_prepare_cderi(cphf_ctx* c, OzState& z) {
   const int64_t nao = c->nao, naux = c->naux;
-  z.ldk = (nao + 7) / 8 * 8;
+  z.ldk = plane_ld(nao);
   z.A.ensure((size_t)S * naux * nao * z.ldk * 2, c->counter());
   z.rowscale.ensure((size_t)nao * 8, c->counter());
   z.e_row.ensure((size_t)nao * 4, c->counter());
@@ -1383,7 +1416,7 @@ static void oz_prepare_spin(cphf_ctx* c, OzState& z, int s) {
   const SpinState& sp = c->spin[s];
   OzSpin& o = z.spin[s];
   const int64_t nao = c->nao, naux = c->naux, no = sp.nocc, ldk = z.ldk;
-  const int64_t ldj = o.ldj = (no + 7) / 8 * 8;
+  const int64_t ldj = o.ldj = plane_ld(no);
   // O_P[j, i]: rows (i, P) at O + no (i + no P), K = j
   o.O.ensure((size_t)S * naux * no * ldj * 2, c->counter());
   o.eO.ensure((size_t)naux * no * 4, c->counter());
@@ -1457,12 +1490,10 @@ static void oz_k_terms_t(cphf_ctx* c, OzState& z, int s, const double* bra, int6
   z.e_col.ensure((size_t)N * 4, c->counter());
   z.mxc.ensure((size_t)N * 8, c->counter());
 
-  const CUtensorMap mCd = make_map(z.A.p, nao, nao, S * naux, ldk, BM);            // term 1 A
   const CUtensorMap mBt = make_map(z.brat.p, no, nao * nb, S, ldj, BM);            // T-gen A
   const CUtensorMap mO = make_map(os.O.p, no, no, S * naux, ldj, 64);               // T-gen B
   const CUtensorMap mBw = make_map(z.braw.p, nao, N, S, ldk, BM);                  // W-gen A
   const CUtensorMap mZ = make_map(os.Z.p, nao, no, S * naux, ldk, 64);             // W-gen B
-  const CUtensorMap mZt = make_map(os.Zt.p, no, nao, S * naux, ldj, BM);           // term 2 A
   const int nkb_nao = (int)div_up(nao, BK), nkb_no = (int)div_up(no, BK);
 
   for (int64_t P0 = 0; P0 < naux; P0 += np) {
@@ -1495,20 +1526,18 @@ static void oz_k_terms_t(cphf_ctx* c, OzState& z, int s, const double* bra, int6
     }
     {
       // term 1: out[mu, n] += alpha sum_{P, nu} B_P[mu, nu] T_P[nu, n]
-      const CUtensorMap mT = make_map(z.B.p, nao, N, S * npc, ldk, BM);
-      OzArgs a = base_args(z, (int)nao, (int)N);
-      a.out = out;
-      a.nkb = nkb_nao;
-      a.total_kb = (int)(npc * nkb_nao);
-      a.a_depth = (int)naux;
-      a.a_off = (int)P0;
-      a.a_per_p = 1;
-      a.b_depth = (int)npc;
+      PairTerm a{};
+      a.x = PairPlanes{{z.A.p, nullptr}, nao, ldk, S * naux, naux};
+      a.y = PairPlanes{{z.B.p, nullptr}, N, ldk, PC::S * npc, npc};
+      a.x_off = P0;
+      a.np = npc; a.M = nao; a.N = N; a.K = nao;
       a.rowscale = z.rowscale.as<double>();
       a.colscale = z.colscale.as<double>();
+      a.out = out;
       a.ld_out = nao;
+      a.err = z.err.as<int>();
       ProfScope ps(c, kP, 2.0 * nao * N * nao * npc, 2.0 * S * nao * npc * (nao + N));
-      launch_split<PC, 128>(c, z, mCd, mT, a);
+      launch_pair_exact(c, z, a, PC::S);
     }
     {
       // W-gen: W[Pl][(i,a)][j] (FP32 pair), rows m = j + no a, columns i, K = nu
@@ -1538,20 +1567,18 @@ static void oz_k_terms_t(cphf_ctx* c, OzState& z, int s, const double* bra, int6
     }
     {
       // term 2: out[mu, n] += alpha sum_{P, j} Z_P[mu, j] W_P[j, n]
-      const CUtensorMap mW = make_map(z.Ws.p, no, N, S * npc, ldj, BM);
-      OzArgs a = base_args(z, (int)nao, (int)N);
-      a.out = out;
-      a.nkb = nkb_no;
-      a.total_kb = (int)(npc * nkb_no);
-      a.a_depth = (int)naux;
-      a.a_off = (int)P0;
-      a.a_per_p = 1;
-      a.b_depth = (int)npc;
+      PairTerm a{};
+      a.x = PairPlanes{{os.Zt.p, nullptr}, nao, ldj, S * naux, naux};
+      a.y = PairPlanes{{z.Ws.p, nullptr}, N, ldj, PC::S * npc, npc};
+      a.x_off = P0;
+      a.np = npc; a.M = nao; a.N = N; a.K = no;
       a.rowscale = os.sZt.as<double>();
       a.colscale = z.colscale.as<double>();
+      a.out = out;
       a.ld_out = nao;
+      a.err = z.err.as<int>();
       ProfScope ps(c, qP, 2.0 * nao * N * no * npc, 2.0 * S * no * npc * (nao + N));
-      launch_split<PC, 128>(c, z, mZt, mW, a);
+      launch_pair_exact(c, z, a, PC::S);
     }
   }
   int flag = 0;
@@ -1574,8 +1601,8 @@ static void lp_prepare_spin(cphf_ctx* c, OzState& z, int s) {
   OzSpin& o = z.spin[s];
   const int64_t nao = c->nao, naux = c->naux, no = sp.nocc;
   constexpr int S2 = Split2::S;
-  z.ldk = (nao + 7) / 8 * 8;
-  const int64_t ldk = z.ldk, ldj = o.ldj = (no + 7) / 8 * 8;
+  z.ldk = plane_ld(nao);
+  const int64_t ldk = z.ldk, ldj = o.ldj = plane_ld(no);
   z.mx.ensure((size_t)std::max<int64_t>(nao, 1) * 8, c->counter());
   o.O.ensure((size_t)S2 * naux * no * ldj * 2, c->counter());
   o.eO.ensure((size_t)naux * no * 4, c->counter());
@@ -1666,11 +1693,12 @@ void lp_tgen_planes(cphf_ctx* c, OzState& z, int s, int64_t P0, int64_t npc, int
   tbound_kernel<<<1, 256, 0, c->stream>>>(z.braS.as<unsigned>(), z.spin[s].Omax.as<unsigned>() + P0, npc, mx);
   count_launch();
   launch_t_scale(mx, sA, alpha, scale, c->stream);
-  if (a.nkb <= ResT::MAX_KB && no <= ResT::BN && res_attr_ok()) {
-    // bra tile resident, all i of a column in one 128-wide tile
-    const CUtensorMap mO128 = make_map(z.spin[s].O.p, no, no, S2 * naux, ldj, ResT::BN, false);
-    // store maps of the epilogue warps' parts: columns [0, 64) and [64, nocc)
-    const int64_t n0c = std::min<int64_t>(no, 64), n1c = std::max<int64_t>(no - 64, 1);
+  if (no <= 128 && res_attr_ok()) {
+    // bra tile resident, all i of a column in one tile of bn columns
+    const int bn = 128;
+    const CUtensorMap mO128 = make_map(z.spin[s].O.p, no, no, S2 * naux, ldj, bn, false);
+    // store maps of the epilogue warps' parts: columns [0, bn / 2) and [bn / 2, nocc)
+    const int64_t n0c = std::min<int64_t>(no, bn / 2), n1c = std::max<int64_t>(no - bn / 2, 1);
     const CUtensorMap mT[4] = {make_t_store_map(hi, nao, N, npc, ldt, n0c), make_t_store_map(hi, nao, N, npc, ldt, n1c),
                                make_t_store_map(lo, nao, N, npc, ldt, n0c), make_t_store_map(lo, nao, N, npc, ldt, n1c)};
     launch_tgen_resident(c, mBt, mO128, mT, a);
