@@ -657,27 +657,33 @@ __global__ void __launch_bounds__(320, PR::NACC == 4 ? 1 : 2)
   if (warp == 1) tmem_dealloc(tmem, 2 * ACC);
 }
 
-// Inner T generation with the bra tile resident (split FP16, K = nocc <= 128): one CTA per SM
-// and (row tile, range of aux functions).  A row tile is 128 consecutive nu of one perturbation
+// Inner T generation with the bra tile resident (split FP16, K = nocc <= 128): one CTA per (row
+// tile, range of aux functions).  A row tile is 128 consecutive nu of one perturbation
 // a (the last tile of each a is partial), so that T_P's tile is one box of the planes' layout.
 // The A tile -- every K block of the bra rows, both planes -- is loaded once and stays in
-// shared memory; O_P's 128-row tile (all i of a column, N = 128 >= nocc) streams through a
-// 4-stage ring.  Double-buffered TMEM accumulators (2 x 128 columns) let the epilogue of aux
-// function p overlap the MMAs of p + 1.  Each epilogue warp (32 nu x 64 i) writes the FP16
-// hi / lo planes of T * tscale of its part into its own shared-memory tile [64 i][32 nu] and
+// shared memory; O_P's tile (all i of a column, BN = 32, 64 or 128 >= nocc rows) streams through a
+// 4-stage ring.  Double-buffered TMEM accumulators (2 x BN columns) let the epilogue of aux
+// function p overlap the MMAs of p + 1.  Each epilogue warp (32 nu x BN / 2 i) writes the FP16
+// hi / lo planes of T * tscale of its part into its own shared-memory tile [BN / 2 i][32 nu] and
 // stores them with TMA (cp.async.bulk.tensor, clipped at nu = nao): the global writes are bulk
 // transfers off the warps' issue path, and a warp waits only for its own previous stores to
 // have left shared memory, so the stores of aux function p drain while p + 1 is computed.
 // Warp 0: TMA loads, warp 1: MMA issuer and TMEM owner, warps 2-9: epilogue.
+// The epilogue's serial chain per aux function (load, convert, stage, store) bounds it, so the
+// column tile follows nocc: with a fixed 128 half of the warps idled for nocc <= 64, and the smaller
+// tiles leave room for two CTAs per SM whose chains overlap (nao 243, nocc 27: 5.0 -> 3.1 ms of a
+// solve).  Staging 128 nu per half (256-byte rows) instead of 32 measured the same.
+template <int BN_>
 struct ResT {
-  static constexpr int BN = 128, STAGES = 4, MAX_KB = 4, THREADS = 320, EPI_WARPS = 8;
+  static constexpr int BN = BN_, HW = BN_ / 2, STAGES = 4, MAX_KB = BN_ / 32, THREADS = 320, EPI_WARPS = 8;
   static constexpr int A_TILE = BM * BK * 2;            // 8 KB: one K block of one plane
-  static constexpr int B_TILE = BN * BK * 2;            // 8 KB
-  static constexpr int A_BYTES = MAX_KB * 2 * A_TILE;   // 64 KB resident
+  static constexpr int B_TILE = BN * BK * 2;            // 8 KB for 128 rows
+  static constexpr int A_BYTES = MAX_KB * 2 * A_TILE;   // 64 KB resident for 128
   static constexpr int STAGE_BYTES = 2 * B_TILE;        // hi + lo of one K block of O_P
-  static constexpr int WARP_OUT = 2 * 64 * 32 * 2;     // one warp's staged hi + lo tiles: 64 i x 32 nu
+  static constexpr int WARP_OUT = 2 * HW * 32 * 2;      // one warp's staged hi + lo tiles: HW i x 32 nu
   static constexpr int OUT_BYTES = EPI_WARPS * WARP_OUT;
   static constexpr int SMEM_BYTES = A_BYTES + STAGES * STAGE_BYTES + OUT_BYTES + 1024 + 1024;
+  static constexpr int CTAS = BN_ == 128 ? 1 : 2;       // per SM
 };
 
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
@@ -700,19 +706,21 @@ __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.comm
 __device__ __forceinline__ void bulk_wait_read0() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
-__global__ void __launch_bounds__(320, 1)
+template <int BN_>
+__global__ void __launch_bounds__(320, ResT<BN_>::CTAS)
     tc_tgen_resident_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant__ CUtensorMap mB,
                             const __grid_constant__ CUtensorMap mTh0, const __grid_constant__ CUtensorMap mTh1,
                             const __grid_constant__ CUtensorMap mTl0, const __grid_constant__ CUtensorMap mTl1,
                             OzArgs args) {
-  constexpr int STAGES = ResT::STAGES, BN = ResT::BN;
+  using R = ResT<BN_>;
+  constexpr int STAGES = R::STAGES, BN = R::BN, HW = R::HW;
   constexpr uint32_t ACC = BN;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* ares = smem;
-  uint8_t* ring = smem + ResT::A_BYTES;
-  uint8_t* outs = ring + STAGES * ResT::STAGE_BYTES;  // per epilogue warp: [plane][64 i][32 nu] FP16
-  uint64_t* bars = reinterpret_cast<uint64_t*>(outs + ResT::OUT_BYTES);
+  uint8_t* ring = smem + R::A_BYTES;
+  uint8_t* outs = ring + STAGES * R::STAGE_BYTES;  // per epilogue warp: [plane][HW i][32 nu] FP16
+  uint64_t* bars = reinterpret_cast<uint64_t*>(outs + R::OUT_BYTES);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 6);
   const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + STAGES);
   const uint32_t accf0 = smem_u32(bars + 2 * STAGES), acce0 = smem_u32(bars + 2 * STAGES + 2);
@@ -736,7 +744,7 @@ __global__ void __launch_bounds__(320, 1)
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(accf0 + 8 * b, 1);
-      mbar_init(acce0 + 8 * b, ResT::EPI_WARPS);
+      mbar_init(acce0 + 8 * b, R::EPI_WARPS);
     }
     mbar_init(done, 1);
     mbar_init(abar, 1);
@@ -751,10 +759,10 @@ __global__ void __launch_bounds__(320, 1)
   if (nP > 0) {
     if (warp == 0 && lane == 0) {
       // resident A: every K block of both planes, once
-      mbar_expect_tx(abar, (uint32_t)(nkb * 2 * ResT::A_TILE));
+      mbar_expect_tx(abar, (uint32_t)(nkb * 2 * R::A_TILE));
       for (int kb = 0; kb < nkb; ++kb)
         for (int t = 0; t < 2; ++t)
-          tma_load_3d(smem_u32(ares + (kb * 2 + t) * ResT::A_TILE), &mA, abar, kb * BK, m0, t * args.a_depth + args.a_off);
+          tma_load_3d(smem_u32(ares + (kb * 2 + t) * R::A_TILE), &mA, abar, kb * BK, m0, t * args.a_depth + args.a_off);
       // O_P tiles of the aux range through the ring
       const int total = nP * nkb;
       int issued = 0;
@@ -763,49 +771,55 @@ __global__ void __launch_bounds__(320, 1)
         if (!mbar_wait(empty0 + 8 * s, ((it / STAGES) & 1) ^ 1, args.err)) break;
         issued = it + 1;
         const uint32_t full = full0 + 8 * s;
-        mbar_expect_tx(full, ResT::STAGE_BYTES);
+        mbar_expect_tx(full, R::STAGE_BYTES);
         const int P = p_begin + it / nkb;
         const int k0 = (it % nkb) * BK;
-        const uint32_t st = smem_u32(ring + s * ResT::STAGE_BYTES);
-        for (int t = 0; t < 2; ++t) tma_load_3d(st + t * ResT::B_TILE, &mB, full, k0, 0, t * args.b_depth + args.b_off + P);
+        const uint32_t st = smem_u32(ring + s * R::STAGE_BYTES);
+        for (int t = 0; t < 2; ++t) tma_load_3d(st + t * R::B_TILE, &mB, full, k0, 0, t * args.b_depth + args.b_off + P);
       }
       for (int it = max(0, issued - STAGES); it < issued; ++it)
         mbar_wait(full0 + 8 * (it % STAGES), (it / STAGES) & 1, nullptr);
       mbar_wait(abar, 0, nullptr);  // the resident copies have landed before the CTA may exit
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1) {
       constexpr uint32_t idesc = instr_desc_f16(BM, BN, false);
-      bool ok = mbar_wait(abar, 0, args.err);
+      const bool el = elect_one();
+      bool ok = __all_sync(0xffffffffu, mbar_wait(abar, 0, args.err));
       fence_after_sync();
       for (int p = 0; p < nP && ok; ++p) {
         const int b = p & 1;
-        if (!mbar_wait(acce0 + 8 * b, ((p >> 1) & 1) ^ 1, args.err)) break;
+        if (!__all_sync(0xffffffffu, mbar_wait(acce0 + 8 * b, ((p >> 1) & 1) ^ 1, args.err))) break;
         fence_after_sync();
         const uint32_t acc_base = tmem + (uint32_t)b * ACC;
         for (int kb = 0; kb < nkb; ++kb) {
           const int it = p * nkb + kb;
           const int s = it % STAGES;
-          if (!mbar_wait(full0 + 8 * s, (it / STAGES) & 1, args.err)) { ok = false; break; }
+          if (!__all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, (it / STAGES) & 1, args.err))) { ok = false; break; }
           fence_after_sync();
-          const uint32_t ah = smem_u32(ares + (kb * 2 + 0) * ResT::A_TILE), al = ah + ResT::A_TILE;
-          const uint32_t bh = smem_u32(ring + s * ResT::STAGE_BYTES), bl = bh + ResT::B_TILE;
+          const uint64_t da = smem_desc<64>(smem_u32(ares + (kb * 2) * R::A_TILE));
+          const uint64_t db = smem_desc<64>(smem_u32(ring + s * R::STAGE_BYTES));
+          if (el) {
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {
-            const uint64_t dk = (uint64_t)((k * 32) >> 4);
-            mma_f16(acc_base, smem_desc<64>(ah) + dk, smem_desc<64>(bh) + dk, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-            mma_f16(acc_base, smem_desc<64>(ah) + dk, smem_desc<64>(bl) + dk, idesc, 1u);
-            mma_f16(acc_base, smem_desc<64>(al) + dk, smem_desc<64>(bh) + dk, idesc, 1u);
+            for (int k = 0; k < BK / 16; ++k) {
+              const uint64_t dk = desc_off(k * 32);
+              mma_f16(acc_base, da + dk, db + dk, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+              mma_f16(acc_base, da + dk, db + (desc_off(R::B_TILE) + dk), idesc, 1u);
+              mma_f16(acc_base, da + (desc_off(R::A_TILE) + dk), db + dk, idesc, 1u);
+            }
+            mma_commit(empty0 + 8 * s);
           }
-          mma_commit(empty0 + 8 * s);
+          __syncwarp();
         }
-        if (ok) mma_commit(accf0 + 8 * b);
+        if (ok && el) mma_commit(accf0 + 8 * b);
+        __syncwarp();
       }
-      mma_commit(done);
+      if (el) mma_commit(done);
+      __syncwarp();
       mbar_wait(done, 0, nullptr);
     } else if (warp >= 2) {
-      // epilogue: TMEM lane quarter q (rows nu0 + 32 q + lane), columns i in [64 h, 64 h + ni)
+      // epilogue: TMEM lane quarter q (rows nu0 + 32 q + lane), columns i in [HW h, HW h + ni)
       const int q = warp & 3;
       const int h = (warp - 2) >> 2;
-      const int ni = min(64, no - 64 * h);  // this warp's columns (none when nocc <= 64 and h = 1)
+      const int ni = min(HW, no - HW * h);  // this warp's columns (may be none)
       const int nul = q * 32 + lane;
       const bool row_ok = nu0 + nul < nao;
       const int erow = row_ok ? args.e_row[m0 + nul] - 2 * Split2::EOFF : 0;
@@ -815,9 +829,9 @@ __global__ void __launch_bounds__(320, 1)
       // exponent of p + 1 is fetched while p is processed
       const int* const eP = args.e_col + (int64_t)(args.b_off + p_begin) * args.N;
       int e_next = eP[0];
-      uint8_t* const wst = outs + (warp - 2) * ResT::WARP_OUT;
-      __half* const sh = reinterpret_cast<__half*>(wst) + lane;  // [64 i][32 nu]
-      __half* const sl = sh + 64 * 32;
+      uint8_t* const wst = outs + (warp - 2) * R::WARP_OUT;
+      __half* const sh = reinterpret_cast<__half*>(wst) + lane;  // [HW i][32 nu]
+      __half* const sl = sh + HW * 32;
       const CUtensorMap* const mh = h == 0 ? &mTh0 : &mTh1;
       const CUtensorMap* const ml = h == 0 ? &mTl0 : &mTl1;
       const uint64_t policy = l2_evict_first();
@@ -825,48 +839,38 @@ __global__ void __launch_bounds__(320, 1)
         const int b = p & 1;
         const int e_p = e_next;
         if (p + 1 < nP) e_next = eP[(int64_t)(p + 1) * args.N];
-        // this warp's staged tiles of p - 1 have left shared memory before they are overwritten
-        if (lane == 0) bulk_wait_read0();
-        __syncwarp();
         if (!__all_sync(0xffffffffu, mbar_wait(accf0 + 8 * b, (p >> 1) & 1, args.err))) break;
         fence_after_sync();
-        float v[2][32];
-        const uint32_t tb = tmem + (uint32_t)b * ACC + ((uint32_t)(q * 32) << 16) + (uint32_t)(h * 64);
-        tmem_ld32x2(tb, tb + 32, v[0], v[1]);
+        float v[HW];
+        const uint32_t tb = tmem + (uint32_t)b * ACC + ((uint32_t)(q * 32) << 16) + (uint32_t)(h * HW);
+        if constexpr (HW == 64) tmem_ld32x2(tb, tb + 32, v, v + 32);
+        else if constexpr (HW == 32) tmem_ld32(tb, v);
+        else tmem_ld16(tb, v);
         fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(acce0 + 8 * b);  // accumulator b may take aux p + 2
         if (ni <= 0) continue;
+        // this warp's staged tiles of p - 1 have left shared memory before they are overwritten
+        if (lane == 0) bulk_wait_read0();
+        __syncwarp();
         const float f = pow2f(erow + e_p + ets);
+        // two columns per conversion (columns >= ni are staged but not stored)
 #pragma unroll
-        for (int cc = 0; cc < 2; ++cc) {
-          const int jn = min(32, ni - 32 * cc);
-          if (jn >= 32) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              const float x = v[cc][j] * f;
-              const __half hh = __float2half_rn(x);
-              sh[(32 * cc + j) * 32] = hh;
-              sl[(32 * cc + j) * 32] = __float2half_rn(x - __half2float(hh));
-            }
-          } else {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              if (j < jn) {
-                const float x = v[cc][j] * f;
-                const __half hh = __float2half_rn(x);
-                sh[(32 * cc + j) * 32] = hh;
-                sl[(32 * cc + j) * 32] = __float2half_rn(x - __half2float(hh));
-              }
-            }
-          }
+        for (int j = 0; j < HW; j += 2) {
+          const float x0 = v[j] * f, x1 = v[j + 1] * f;
+          const __half2 hh = __floats2half2_rn(x0, x1);
+          const __half2 ll = __floats2half2_rn(x0 - __low2float(hh), x1 - __high2float(hh));
+          sh[j * 32] = __low2half(hh);
+          sh[(j + 1) * 32] = __high2half(hh);
+          sl[j * 32] = __low2half(ll);
+          sl[(j + 1) * 32] = __high2half(ll);
         }
         fence_proxy_async();  // the generic-proxy writes are visible to the TMA stores
         __syncwarp();
-        if (lane == 0 && nu0 + 32 * q < nao) {  // (a box wholly past nu = nao has nothing to store)
+        if (lane == 0 && nu0 + q * 32 < nao) {
           const int Pl = p_begin + p;
-          tma_store_3d(mh, smem_u32(wst), nu0 + 32 * q, a_pert * no + 64 * h, Pl, policy);
-          tma_store_3d(ml, smem_u32(wst + ResT::WARP_OUT / 2), nu0 + 32 * q, a_pert * no + 64 * h, Pl, policy);
+          tma_store_3d(mh, smem_u32(wst), nu0 + q * 32, a_pert * no + HW * h, Pl, policy);
+          tma_store_3d(ml, smem_u32(wst + R::WARP_OUT / 2), nu0 + q * 32, a_pert * no + HW * h, Pl, policy);
           bulk_commit();
         }
       }
@@ -1296,22 +1300,35 @@ void launch_batched(cphf_ctx* c, const CUtensorMap& mA, const CUtensorMap& mB, c
 bool res_attr_ok() {
   static int state = -1;
   if (state < 0) {
-    state = cudaFuncSetAttribute(tc_tgen_resident_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 ResT::SMEM_BYTES) == cudaSuccess ? 1 : 0;
+    auto set = [](const void* f, int bytes) {
+      return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
+    };
+    state = set((const void*)tc_tgen_resident_kernel<32>, ResT<32>::SMEM_BYTES) &&
+                    set((const void*)tc_tgen_resident_kernel<64>, ResT<64>::SMEM_BYTES) &&
+                    set((const void*)tc_tgen_resident_kernel<128>, ResT<128>::SMEM_BYTES)
+                ? 1 : 0;
     if (!state) cudaGetLastError();
   }
   return state == 1;
 }
+// column tile of the resident T generation for nocc columns
+int res_bn(int64_t no) { return no <= 32 ? 32 : no <= 64 ? 64 : 128; }
 
 // row tiles: 128 nu of one perturbation (m_div = nao, M = nao nb)
 void launch_tgen_resident_raw(cphf_ctx* c, const CUtensorMap& mA, const CUtensorMap& mB, const CUtensorMap* mT,
                               OzArgs a, int waves) {
   const int64_t tiles = div_up(a.m_div, (int64_t)BM) * (a.M / a.m_div);
   if (tiles > 65535) throw Error(CPHF_ERR_ARG, "tensor-core T generation: grid too large");
-  a.p_per_cta = (int)std::max<int64_t>(1, std::min<int64_t>(a.np, a.np * tiles / (waves * (int64_t)c->num_sms)));
+  const int bn = res_bn(a.N);
+  const int64_t slots = (int64_t)c->num_sms * (bn == 128 ? 1 : 2);
+  a.p_per_cta = (int)std::max<int64_t>(1, std::min<int64_t>(a.np, a.np * tiles / (waves * slots)));
   const dim3 grid((unsigned)div_up(a.np, a.p_per_cta), (unsigned)tiles);
-  tc_tgen_resident_kernel<<<grid, ResT::THREADS, ResT::SMEM_BYTES, c->stream>>>(mA, mB, mT[0], mT[1], mT[2], mT[3],
-                                                                                 a);
+  auto launch = [&](auto kern, int smem) {
+    kern<<<grid, 320, smem, c->stream>>>(mA, mB, mT[0], mT[1], mT[2], mT[3], a);
+  };
+  if (bn == 32) launch(tc_tgen_resident_kernel<32>, ResT<32>::SMEM_BYTES);
+  else if (bn == 64) launch(tc_tgen_resident_kernel<64>, ResT<64>::SMEM_BYTES);
+  else launch(tc_tgen_resident_kernel<128>, ResT<128>::SMEM_BYTES);
   count_launch();
   CPHF_CUDA(cudaGetLastError());
 }
@@ -1695,7 +1712,7 @@ void lp_tgen_planes(cphf_ctx* c, OzState& z, int s, int64_t P0, int64_t npc, int
   launch_t_scale(mx, sA, alpha, scale, c->stream);
   if (no <= 128 && res_attr_ok()) {
     // bra tile resident, all i of a column in one tile of bn columns
-    const int bn = 128;
+    const int bn = res_bn(no);
     const CUtensorMap mO128 = make_map(z.spin[s].O.p, no, no, S2 * naux, ldj, bn, false);
     // store maps of the epilogue warps' parts: columns [0, bn / 2) and [bn / 2, nocc)
     const int64_t n0c = std::min<int64_t>(no, bn / 2), n1c = std::max<int64_t>(no - bn / 2, 1);

@@ -59,3 +59,14 @@ def test_exact_slice_residual_at_tile_edges(nao, naux, nocc, natm):
     r = (s.rhs[0] - x - y).reshape(-1, 3 * natm, order="F")
     ref = float(np.linalg.norm(r, axis=0).max())
     assert abs(ctx.last_stats["residual_max"] - ref) < 1e-9 * max(1.0, np.abs(x).max()), ref
+
+
+@pytest.mark.parametrize("nocc", [1, 31, 32, 33, 63, 64, 65, 127, 128, 129])
+def test_t_generation_at_column_tile_edges(nocc):
+    """T generation keeps the bra tile for nocc <= 128, in column tiles of 32, 64 or 128."""
+    s = _system(161, 21, nocc, 1)
+    ctx = _context(s, aux_chunk=8)
+    mo1 = np.random.default_rng(nocc).standard_normal((161, nocc, 3))
+    got = ctx.response_dimless_cphf_lowp(mo1)
+    assert ctx.tensor_cores_active
+    assert rel_err(got, _oracle(s).response_dimless_cphf(mo1)) < 1e-5
