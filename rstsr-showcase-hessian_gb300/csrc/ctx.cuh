@@ -236,6 +236,7 @@ struct cphf_ctx {
   // scratch (grown on demand)
   cphf::DevBuf ws_fx, fx_err;  // fixed-point GEMM: workspace, error flag of its bounded waits
   bool fx_used = false;        // ... launched since the flag was last read
+  cphf::DevBuf s_phid;         // dense AO values of one chunk of grid batches (FP64 XC)
   cphf::DevBuf ws_gemm, s_c1, s_resp, s_T, s_W, s_d, s_ket, s_rho, s_y, s_x, s_misc, s_host_io;
   cphf::DevBuf k_xs, k_ax, k_h, k_g, k_b, k_xacc, k_x1, k_axt, k_coef, k_ip, k_keep, k_part, k_idx,
       k_hw, k_info, k_r, k_norm, k_finite, k_pre;
@@ -277,8 +278,12 @@ struct ProfScope {
 namespace cphf {
 
 // gemm helpers bound to the context (stream, split-K workspace, SM count)
+struct FxPlan;
 void gemm64(cphf_ctx* c, const GemmDesc& d);
 double gemm64_us(cphf_ctx* c, const GemmDesc& d);      // its expected time (us)
+// fixed-point product by plan (gemm_fx.cuh); returns the device flag of non-finite operands, which
+// are left to the caller
+const int* gemm64_fx(cphf_ctx* c, const GemmDesc& d, const FxPlan& fx);
 void gemm32(cphf_ctx* c, const GemmDesc& d);  // float compute, float operands/output
 template <typename TA, typename TB, typename TC>
 void gemm32x(cphf_ctx* c, const GemmDesc& d);

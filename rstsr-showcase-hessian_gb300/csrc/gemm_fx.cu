@@ -636,7 +636,8 @@ cudaError_t slice(SliceArgs a, cudaStream_t s, int num_sms) {
 
 }  // namespace
 
-cudaError_t fx_gemm(const FxPlan& p, cudaStream_t st, void* ws, int* err, int num_sms) {
+cudaError_t fx_gemm(const FxPlan& p, cudaStream_t st, void* ws, int* err, int num_sms, const int** nonfinite) {
+  if (nonfinite != nullptr && p.m_chunk < p.d.M) return cudaErrorInvalidValue;
   const GemmDesc& d = p.d;
   char* w = static_cast<char*>(ws);
   int* flag = reinterpret_cast<int*>(w);
@@ -715,6 +716,10 @@ cudaError_t fx_gemm(const FxPlan& p, cudaStream_t st, void* ws, int* err, int nu
       fx_reduce_kernel<<<(unsigned)std::min<int64_t>(div_up(tot, 256), 8 * (int64_t)num_sms), 256, 0, st>>>(g, d.batch1);
       count_launch();
       if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
+    if (nonfinite != nullptr) {
+      *nonfinite = flag;
+      continue;
     }
     // non-finite operands: the product on the native kernel (returns at once otherwise), its split-K
     // sums over the planes

@@ -27,7 +27,10 @@ bool fx_available(int device);
 // native kernel on this shape.
 bool fx_plan(const GemmDesc& d, int num_sms, FxPlan& p);
 // C = alpha A B + beta C.  `ws`: plan.total bytes; `err`: raised when a bounded wait expired.
-// Non-finite operands are left to the native kernel, which runs only when one was met.
-cudaError_t fx_gemm(const FxPlan& p, cudaStream_t stream, void* ws, int* err, int num_sms);
+// Non-finite operands are left to the native kernel, which runs only when one was met; with
+// `nonfinite` (single-pass plans) they are left to the caller: it receives the device flag that is
+// set when one was met, C is then untouched.
+cudaError_t fx_gemm(const FxPlan& p, cudaStream_t stream, void* ws, int* err, int num_sms,
+                    const int** nonfinite = nullptr);
 
 }  // namespace cphf

@@ -46,6 +46,23 @@ double gemm64_us(cphf_ctx* c, const GemmDesc& d) {
   return gemm_f64_us(d, c->num_sms);
 }
 
+static void run_fx(cphf_ctx* c, const GemmDesc& d, const FxPlan& fx, const int** nonfinite) {
+  if (c->fx_err.p == nullptr) {
+    c->fx_err.ensure(sizeof(int), c->counter());
+    CPHF_CUDA(cudaMemsetAsync(c->fx_err.p, 0, sizeof(int), c->stream));
+  }
+  c->ws_fx.ensure(fx.total, c->counter());
+  c->fx_used = true;  // the error flag is read at the end of the API call
+  ProfScope ps(c, PROF_GEMM_FX, gemm_flops(d), 8.0 * (d.M * d.K + d.K * d.N + d.M * d.N) * d.batch1 * d.batch2);
+  CPHF_CUDA(fx_gemm(fx, c->stream, c->ws_fx.p, c->fx_err.as<int>(), c->num_sms, nonfinite));
+}
+
+const int* gemm64_fx(cphf_ctx* c, const GemmDesc& d, const FxPlan& fx) {
+  const int* flag = nullptr;
+  run_fx(c, d, fx, &flag);
+  return flag;
+}
+
 void gemm64(cphf_ctx* c, const GemmDesc& d) {
   if (c->f32_correction) {
     // FP64 operands and result, FP32 arithmetic: the GEMMs of an operator applied to a small
@@ -57,14 +74,7 @@ void gemm64(cphf_ctx* c, const GemmDesc& d) {
   // tensor_cores = 0 keeps every FP64 GEMM on the CUDA cores
   FxPlan fx;
   if (c->cfg.tensor_cores != 0 && fx_available(c->device) && fx_plan(d, c->num_sms, fx)) {
-    if (c->fx_err.p == nullptr) {
-      c->fx_err.ensure(sizeof(int), c->counter());
-      CPHF_CUDA(cudaMemsetAsync(c->fx_err.p, 0, sizeof(int), c->stream));
-    }
-    c->ws_fx.ensure(fx.total, c->counter());
-    c->fx_used = true;  // the error flag is read at the end of the API call
-    ProfScope ps(c, PROF_GEMM_FX, gemm_flops(d), 8.0 * (d.M * d.K + d.K * d.N + d.M * d.N) * d.batch1 * d.batch2);
-    CPHF_CUDA(fx_gemm(fx, c->stream, c->ws_fx.p, c->fx_err.as<int>(), c->num_sms));
+    run_fx(c, d, fx, nullptr);
     return;
   }
   const size_t need = gemm_workspace_bytes(d, 8, c->num_sms);

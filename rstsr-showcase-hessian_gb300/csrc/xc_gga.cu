@@ -102,6 +102,28 @@ __global__ void gga_q_kernel(const T* __restrict__ aob, int64_t ldg, int64_t ldc
   }
 }
 
+// out[e] = beta out[e] + sum_c planes[c n + e] (c < 4)
+__global__ void gga_sum_kernel(const double* __restrict__ planes, int64_t n, double beta, double* __restrict__ out) {
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
+    double v = planes[e] + planes[n + e] + planes[2 * n + e] + planes[3 * n + e];
+    if (beta != 0.0) v = fma(beta, out[e], v);
+    out[e] = v;
+  }
+}
+
+// FP64: the four components of a contraction as one batched GEMM where that is expected to be
+// faster than four: one set of slicing and GEMM launches, whose tiles fill the last wave together
+// (5600 points, nao 96, 15 occupied x 24: the eight products of an application 0.9 -> 0.6 ms).
+bool gemm_components(cphf_ctx* c, GemmDesc d, double extra_us, int64_t a_b, int64_t b_b, int64_t c_b) {
+  if (c->cfg.tensor_cores == 0 || c->f64_emulate || c->f32_correction) return false;
+  const double four = 4.0 * gemm64_us(c, d);
+  d.batch1 = 4;
+  d.a_b1 = a_b; d.b_b1 = b_b; d.c_b1 = c_b;
+  if (gemm64_us(c, d) + extra_us >= four) return false;
+  gemm64(c, d);
+  return true;
+}
+
 template <typename T>
 void gemm_t(cphf_ctx* c, const GemmDesc& d) {
   if constexpr (sizeof(T) == 8) gemm64(c, d);
@@ -145,7 +167,9 @@ void xc_response_gga(cphf_ctx* c, const T* const* bra, int64_t nb, T* const* out
     if (c->cfg.xc_chunk_points > 0) chunk = c->cfg.xc_chunk_points;
     chunk = std::min<int64_t>(chunk, NG);
     ket_buf.ensure((size_t)4 * chunk * no_max * nb * sizeof(T), c->counter());
-    rho_buf.ensure((size_t)ns * chunk * nvar * nb * sizeof(T), c->counter());
+    // rho1 of the spins, then (FP64) the output contraction's four component planes
+    const int64_t rho_all = ns * chunk * nvar * nb;
+    rho_buf.ensure((size_t)(rho_all + (sizeof(T) == 8 ? 4 * nao * no_max * nb : 0)) * sizeof(T), c->counter());
     T* ket = ket_buf.as<T>();
     T* rho = rho_buf.as<T>();
     for (int64_t g0 = 0; g0 < NG; g0 += chunk) {
@@ -158,7 +182,16 @@ void xc_response_gga(cphf_ctx* c, const T* const* bra, int64_t nb, T* const* out
           CPHF_CUDA(cudaMemsetAsync(rho + s * rho_ss, 0, (size_t)rho_ss * sizeof(T), c->stream));
           continue;
         }
-        for (int comp = 0; comp < 4; ++comp) {
+        bool one = false;
+        if constexpr (sizeof(T) == 8) {
+          GemmDesc d;
+          d.M = ng; d.N = N; d.K = nao;
+          d.A = phi + g0; d.a_m = 1; d.a_k = NG;
+          d.B = bra[s]; d.b_k = 1; d.b_n = nao;
+          d.C = ket; d.c_m = 1; d.c_n = ng;
+          one = gemm_components(c, d, 0.0, NG * nao, 0, ng * N);
+        }
+        for (int comp = 0; !one && comp < 4; ++comp) {
           GemmDesc d;  // ket_c = phi_c bra  (pure_eval_rho.rs:283-296)
           d.M = ng; d.N = N; d.K = nao;
           d.A = phi + g0 + NG * nao * comp; d.a_m = 1; d.a_k = NG;
@@ -178,7 +211,23 @@ void xc_response_gga(cphf_ctx* c, const T* const* bra, int64_t nb, T* const* out
             aob[so] + g0, NG, NG * no, c->weights.as<double>(), c->fxcG.as<double>(), NG, g0, ns, so, rho, rho_ss, ng,
             no, nb, nvar, ket);
         count_launch();
-        for (int comp = 0; comp < 4; ++comp) {
+        bool one = false;
+        if constexpr (sizeof(T) == 8) {
+          GemmDesc d;
+          d.M = nao; d.N = N; d.K = ng;
+          d.A = phi + g0; d.a_m = NG; d.a_k = 1;
+          d.B = ket; d.b_k = 1; d.b_n = ng;
+          d.C = rho + rho_all; d.c_m = 1; d.c_n = nao;
+          d.alpha = fac;
+          one = gemm_components(c, d, 8.0, NG * nao, ng * N, nao * N);
+          if (one) {
+            gga_sum_kernel<<<blocks(nao * N), kThreads, 0, c->stream>>>(rho + rho_all, nao * N, written[so] ? 1.0 : 0.0,
+                                                                        out[so]);
+            count_launch();
+            written[so] = true;
+          }
+        }
+        for (int comp = 0; !one && comp < 4; ++comp) {
           GemmDesc d;  // out += fac phi_c^T Q_c  (pure_xcpot.rs:331-351)
           d.M = nao; d.N = N; d.K = ng;
           d.A = phi + g0 + NG * nao * comp; d.a_m = NG; d.a_k = 1;

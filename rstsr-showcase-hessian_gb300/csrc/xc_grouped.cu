@@ -15,6 +15,7 @@
 
 #include "ctx.cuh"
 #include "dfloat.cuh"
+#include "gemm_fx.cuh"
 #include "kernels.cuh"
 #include "xc_grouped.cuh"
 
@@ -105,7 +106,8 @@ template <typename T, typename TC>
 __global__ void __launch_bounds__(256, sizeof(TC) == 4 ? 2 : 3) xc_gemm1_kernel(const XcGroupDev* __restrict__ groups, int ngroups,
                                                        const T* __restrict__ phi, const T* __restrict__ bra,
                                                        int64_t nao, int64_t N, int64_t pchunk, T* __restrict__ ket,
-                                                       int64_t total_tiles, int64_t tiles_n) {
+                                                       int64_t total_tiles, int64_t tiles_n, const int* only_if) {
+  if (only_if != nullptr && *only_if == 0) return;
   using Cfg = XcCfg<T>;
   constexpr int BM = Cfg::BM, BN = Cfg::BN, BK = Cfg::BK, TM = Cfg::TM, TN = Cfg::TN;
   constexpr int NTX = BN / TN, NTY = BM / TM;
@@ -151,7 +153,9 @@ template <typename T, typename TC>
 __global__ void __launch_bounds__(256, sizeof(TC) == 4 ? 2 : 3) xc_gemm2_kernel(const XcGroupDev* __restrict__ groups, int ngroups,
                                                        const T* __restrict__ phi, const T* __restrict__ q,
                                                        int64_t nao, int64_t N, int64_t pchunk, T* __restrict__ out,
-                                                       double alpha, double beta, int64_t tiles_m, int64_t tiles_n) {
+                                                       double alpha, double beta, int64_t tiles_m, int64_t tiles_n,
+                                                       const int* only_if) {
+  if (only_if != nullptr && *only_if == 0) return;
   using Cfg = XcCfg<T>;
   constexpr int BM = Cfg::BM, BN = Cfg::BN, BK = Cfg::BK, TM = Cfg::TM, TN = Cfg::TN;
   constexpr int NTX = BN / TN, NTY = BM / TM;
@@ -201,7 +205,7 @@ __global__ void __launch_bounds__(256, sizeof(TC) == 4 ? 2 : 3) xc_gemm2_kernel(
 
 template <typename T>
 void xc_grouped_gemm1(cphf_ctx* c, const XcGroupDev* groups_dev, int ngroups, int64_t total_tiles, const T* phi,
-                      const T* bra, int64_t N, int64_t pchunk, T* ket) {
+                      const T* bra, int64_t N, int64_t pchunk, T* ket, const int* only_if) {
   using Cfg = XcCfg<T>;
   const int64_t tiles_n = div_up(N, Cfg::BN);
   const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(total_tiles, 8 * (int64_t)c->num_sms));
@@ -209,20 +213,20 @@ void xc_grouped_gemm1(cphf_ctx* c, const XcGroupDev* groups_dev, int ngroups, in
   if constexpr (sizeof(T) == 8) {
     if (c->f64_emulate) {
       xc_gemm1_kernel<T, dfloat><<<grid, 256, 0, c->stream>>>(groups_dev, ngroups, phi, bra, c->nao, N, pchunk, ket,
-                                                              total_tiles, tiles_n);
+                                                              total_tiles, tiles_n, only_if);
       launched = true;
     }
   }
   if (!launched)
     xc_gemm1_kernel<T, T><<<grid, 256, 0, c->stream>>>(groups_dev, ngroups, phi, bra, c->nao, N, pchunk, ket,
-                                                       total_tiles, tiles_n);
+                                                       total_tiles, tiles_n, only_if);
   count_launch();
   CPHF_CUDA(cudaGetLastError());
 }
 
 template <typename T>
 void xc_grouped_gemm2(cphf_ctx* c, const XcGroupDev* groups_dev, int ngroups, const T* phi, const T* q, int64_t N,
-                      int64_t pchunk, T* out, double alpha, double beta) {
+                      int64_t pchunk, T* out, double alpha, double beta, const int* only_if) {
   using Cfg = XcCfg<T>;
   const int64_t tiles_m = div_up(c->nao, Cfg::BM), tiles_n = div_up(N, Cfg::BN);
   const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(tiles_m * tiles_n, 8 * (int64_t)c->num_sms));
@@ -230,13 +234,13 @@ void xc_grouped_gemm2(cphf_ctx* c, const XcGroupDev* groups_dev, int ngroups, co
   if constexpr (sizeof(T) == 8) {
     if (c->f64_emulate) {
       xc_gemm2_kernel<T, dfloat><<<grid, 256, 0, c->stream>>>(groups_dev, ngroups, phi, q, c->nao, N, pchunk, out,
-                                                              alpha, beta, tiles_m, tiles_n);
+                                                              alpha, beta, tiles_m, tiles_n, only_if);
       launched = true;
     }
   }
   if (!launched)
     xc_gemm2_kernel<T, T><<<grid, 256, 0, c->stream>>>(groups_dev, ngroups, phi, q, c->nao, N, pchunk, out, alpha,
-                                                       beta, tiles_m, tiles_n);
+                                                       beta, tiles_m, tiles_n, only_if);
   count_launch();
   CPHF_CUDA(cudaGetLastError());
 }
@@ -320,13 +324,51 @@ static GemmDesc batch_out(cphf_ctx* c, const XcBatch& x, int64_t g0, int64_t pts
   return d;
 }
 
-// FP64: one GEMM per batch and contraction (on the tensor cores where gemm64 finds that faster)
-// instead of the two grouped launches, when the sum of their expected times is the smaller: the
-// grouped kernels run at the FP64 pipe's rate, and the second one gives each 64 x 64 output tile
-// to one CTA for all points (nao 83, 6600 points: 16 ms an application, batches 1.1 ms); with
-// many tiny batches the launches of the batch route cost more.
-static bool batches_faster(cphf_ctx* c, const XcChunk& ch, int64_t N) {
-  if (c->cfg.tensor_cores == 0 || N <= 0) return false;
+// The two contractions of a whole chunk over its dense AO values [points, nao].
+static GemmDesc dense_ket(cphf_ctx* c, int64_t pts, int64_t N, const double* phi, const double* bra, double* ket) {
+  GemmDesc d;
+  d.M = pts; d.N = N; d.K = c->nao;
+  d.A = phi; d.a_m = 1; d.a_k = pts;
+  d.B = bra; d.b_k = 1; d.b_n = c->nao;
+  d.C = ket; d.c_m = 1; d.c_n = pts;
+  return d;
+}
+static GemmDesc dense_out(cphf_ctx* c, int64_t pts, int64_t N, const double* phi, const double* q, double* out,
+                          double fac) {
+  GemmDesc d;
+  d.M = c->nao; d.N = N; d.K = pts;
+  d.A = phi; d.a_m = pts; d.a_k = 1;
+  d.B = q; d.b_k = 1; d.b_n = pts;
+  d.C = out; d.c_m = 1; d.c_n = c->nao;
+  d.alpha = fac; d.beta = 1.0;
+  return d;
+}
+
+// dense[r + pts m] = the chunk's AO value of point r and AO m, zero outside the batch's window
+__global__ void xc_dense_phi_kernel(const XcGroupDev* __restrict__ groups, int ngroups, const double* __restrict__ phi,
+                                    int64_t nao, int64_t pts, double* __restrict__ dense) {
+  for (int g = blockIdx.y; g < ngroups; g += gridDim.y) {
+    const XcGroupDev G = groups[g];
+    const int64_t total = G.npts * nao;
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
+      const int64_t r = t % G.npts, m = t / G.npts, k = m - G.lo;
+      dense[G.p_local + r + pts * m] = k >= 0 && k < G.nwin ? phi[G.phi_off + r + G.npts * k] : 0.0;
+    }
+  }
+}
+
+// FP64 contractions of a chunk and spin, by the sum of their expected times:
+//   grouped: the two grouped launches, at the FP64 pipe's rate, the second with one CTA per 64 x 64
+//            output tile for all points;
+//   batches: one GEMM per batch and contraction (on the tensor cores where gemm64 finds that faster);
+//   dense:   one fixed-point GEMM per contraction over the chunk's dense AO values: more products,
+//            the zeros outside the windows, in two launches on the tensor cores.  Non-finite
+//            operands go to the grouped kernels, which keep to the windows.
+// nao 83, 6600 points in 6 batches, 2 spins: 16 / 1.2 / 0.36 ms an application.  Few points and many
+// AOs outside the windows favour the batches, many tiny batches the grouped kernels.
+enum class XcRoute { grouped, batches, dense };
+static XcRoute xc_route(cphf_ctx* c, const XcChunk& ch, int64_t N, FxPlan& ket_fx, FxPlan& out_fx) {
+  if (c->cfg.tensor_cores == 0 || N <= 0) return XcRoute::grouped;
   constexpr double kTile = 64.0 * 64.0 / 2.0 / 1900.0;  // us per k of a tile on one SM
   const double tn = (double)xc_tiles_n(N, true);
   double batch = 0.0, work1 = 0.0;
@@ -342,7 +384,16 @@ static bool batches_faster(cphf_ctx* c, const XcChunk& ch, int64_t N) {
   double longest = 0.0, all = 0.0;
   for (double p : pts) longest = std::max(longest, p), all += p;
   const double grouped = kTile * (work1 / c->num_sms + std::max(longest, all * tn / c->num_sms)) + 10.0;
-  return batch < grouped;
+  if (!c->f64_emulate && !c->f32_correction && fx_available(c->device) && ch.npts * c->nao <= (int64_t(1) << 28)) {
+    const GemmDesc k = dense_ket(c, ch.npts, N, nullptr, nullptr, nullptr);
+    const GemmDesc o = dense_out(c, ch.npts, N, nullptr, nullptr, nullptr, 1.0);
+    if (fx_plan(k, c->num_sms, ket_fx) && fx_plan(o, c->num_sms, out_fx) && ket_fx.m_chunk == ket_fx.d.M &&
+        out_fx.m_chunk == out_fx.d.M) {
+      const double dense = ket_fx.us + out_fx.us + 5.0 + 16.0 * (double)(ch.npts * c->nao) / 4.5e6;
+      if (dense < std::min(batch, grouped)) return XcRoute::dense;
+    }
+  }
+  return batch < grouped ? XcRoute::batches : XcRoute::grouped;
 }
 
 template <typename T>
@@ -370,6 +421,17 @@ void xc_response_grouped(cphf_ctx* c, const T* const* bra, int64_t nb, T* const*
     const int ng = (int)(ch.b1 - ch.b0);
     T* ket[2] = {ket_buf.as<T>(), ket_buf.as<T>() + ket_spin[0]};
     T* rho = rho_buf.as<T>();
+    XcRoute route[2] = {XcRoute::grouped, XcRoute::grouped};
+    if constexpr (sizeof(T) == 8) {
+      FxPlan k, o;
+      for (int s = 0; s < ns; ++s) route[s] = xc_route(c, ch, c->spin[s].nocc * nb, k, o);
+      if (route[0] == XcRoute::dense || route[1] == XcRoute::dense) {
+        c->s_phid.ensure((size_t)(ch.npts * nao) * 8, c->counter());
+        const dim3 grid((unsigned)std::max<int64_t>(1, div_up(4 * (int64_t)c->num_sms, ng)), (unsigned)std::min(ng, 65535));
+        xc_dense_phi_kernel<<<grid, 256, 0, c->stream>>>(gdev + ch.group_off, ng, phi, nao, ch.npts, c->s_phid.as<double>());
+        count_launch();
+      }
+    }
     for (int s = 0; s < ns; ++s) {
       const int64_t no = c->spin[s].nocc;
       T* rho_s = rho + s * ch.npts * nb;
@@ -379,15 +441,21 @@ void xc_response_grouped(cphf_ctx* c, const T* const* bra, int64_t nb, T* const*
       }
       // rows of batches with an empty AO window are never written: clear them first
       CPHF_CUDA(cudaMemsetAsync(ket[s], 0, (size_t)ch.npts * no * nb * sizeof(T), c->stream));
-      bool batches = false;
+      const int* only_if = nullptr;  // the grouped kernel behind the dense product
       if constexpr (sizeof(T) == 8) {
-        batches = batches_faster(c, ch, no * nb);
-        for (int64_t b = ch.b0; batches && b < ch.b1; ++b)
+        if (route[s] == XcRoute::dense) {
+          FxPlan fx;
+          const GemmDesc d = dense_ket(c, ch.npts, no * nb, c->s_phid.as<double>(), bra[s], ket[s]);
+          fx_plan(d, c->num_sms, fx);
+          only_if = gemm64_fx(c, d, fx);
+        }
+        for (int64_t b = ch.b0; route[s] == XcRoute::batches && b < ch.b1; ++b)
           if (c->xc_batches[b].npts > 0 && c->xc_batches[b].nwin > 0)
             gemm64(c, batch_ket(c, c->xc_batches[b], ch.g0, ch.npts, no * nb, phi, bra[s], ket[s]));
       }
-      if (!batches)
-        xc_grouped_gemm1<T>(c, gdev + ch.group_off + s * ng, ng, ch.tiles[s], phi, bra[s], no * nb, ch.npts, ket[s]);
+      if (route[s] != XcRoute::batches)
+        xc_grouped_gemm1<T>(c, gdev + ch.group_off + s * ng, ng, ch.tiles[s], phi, bra[s], no * nb, ch.npts, ket[s],
+                            only_if);
       launch_xc_rho<T>(aobra[s] + ch.g0, c->ngrids, ket[s], ch.npts, no, nb, rho_s, ch.npts, c->stream);
     }
     for (int s = 0; s < ns; ++s) {
@@ -395,15 +463,20 @@ void xc_response_grouped(cphf_ctx* c, const T* const* bra, int64_t nb, T* const*
       if (no == 0) continue;
       launch_xc_q<T>(aobra[s] + ch.g0, c->ngrids, c->weights.as<double>() + ch.g0, c->fxc.as<double>() + ch.g0,
                      c->ngrids, ns, s, rho, ch.npts, ch.npts * nb, ch.npts, no, nb, ket[s], c->stream);
-      bool batches = false;
+      const int* only_if = nullptr;
       if constexpr (sizeof(T) == 8) {
-        batches = batches_faster(c, ch, no * nb);
-        for (int64_t b = ch.b0; batches && b < ch.b1; ++b)
+        if (route[s] == XcRoute::dense) {
+          FxPlan fx;
+          const GemmDesc d = dense_out(c, ch.npts, no * nb, c->s_phid.as<double>(), ket[s], out[s], fac);
+          fx_plan(d, c->num_sms, fx);
+          only_if = gemm64_fx(c, d, fx);
+        }
+        for (int64_t b = ch.b0; route[s] == XcRoute::batches && b < ch.b1; ++b)
           if (c->xc_batches[b].npts > 0 && c->xc_batches[b].nwin > 0)
             gemm64(c, batch_out(c, c->xc_batches[b], ch.g0, ch.npts, no * nb, phi, ket[s], out[s], fac));
       }
-      if (!batches)
-        xc_grouped_gemm2<T>(c, gdev + ch.group_off + s * ng, ng, phi, ket[s], no * nb, ch.npts, out[s], fac, 1.0);
+      if (route[s] != XcRoute::batches)
+        xc_grouped_gemm2<T>(c, gdev + ch.group_off + s * ng, ng, phi, ket[s], no * nb, ch.npts, out[s], fac, 1.0, only_if);
     }
   }
 }
@@ -414,12 +487,12 @@ template void xc_response_grouped<float>(cphf_ctx*, const float* const*, int64_t
                                          const float* const*, DevBuf&, DevBuf&);
 
 template void xc_grouped_gemm1<double>(cphf_ctx*, const XcGroupDev*, int, int64_t, const double*, const double*,
-                                       int64_t, int64_t, double*);
+                                       int64_t, int64_t, double*, const int*);
 template void xc_grouped_gemm1<float>(cphf_ctx*, const XcGroupDev*, int, int64_t, const float*, const float*,
-                                      int64_t, int64_t, float*);
+                                      int64_t, int64_t, float*, const int*);
 template void xc_grouped_gemm2<double>(cphf_ctx*, const XcGroupDev*, int, const double*, const double*, int64_t,
-                                       int64_t, double*, double, double);
+                                       int64_t, double*, double, double, const int*);
 template void xc_grouped_gemm2<float>(cphf_ctx*, const XcGroupDev*, int, const float*, const float*, int64_t,
-                                      int64_t, float*, double, double);
+                                      int64_t, float*, double, double, const int*);
 
 }  // namespace cphf

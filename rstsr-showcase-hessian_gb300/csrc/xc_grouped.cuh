@@ -21,12 +21,13 @@ template <typename T>
 void xc_response_grouped(cphf_ctx* c, const T* const* bra, int64_t nb, T* const* out, bool accumulate,
                          const T* phi, const T* const* aobra, DevBuf& ket_buf, DevBuf& rho_buf);
 
+// The two grouped launches; with `only_if` they return at once unless the device flag is set.
 template <typename T>
 void xc_grouped_gemm1(cphf_ctx* c, const XcGroupDev* groups_dev, int ngroups, int64_t total_tiles, const T* phi,
-                      const T* bra, int64_t N, int64_t pchunk, T* ket);
+                      const T* bra, int64_t N, int64_t pchunk, T* ket, const int* only_if = nullptr);
 template <typename T>
 void xc_grouped_gemm2(cphf_ctx* c, const XcGroupDev* groups_dev, int ngroups, const T* phi, const T* q, int64_t N,
-                      int64_t pchunk, T* out, double alpha, double beta);
+                      int64_t pchunk, T* out, double alpha, double beta, const int* only_if = nullptr);
 // chunk plan of the grid batches for element size esize and nb columns (cached per width)
 XcPlan& xc_plan(cphf_ctx* c, size_t esize, int64_t nb);
 int64_t xc_tiles_m(int64_t npts, bool f64);
