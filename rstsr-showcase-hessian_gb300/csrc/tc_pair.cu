@@ -117,6 +117,7 @@ __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
 __device__ __forceinline__ double widen(float x) {
   const unsigned b = __float_as_uint(x);
   if ((b & 0x7F800000u) == 0u) return 0.0;
+  if ((b & 0x7F800000u) == 0x7F800000u) return (double)x;  // NaN slices of non-finite operands
   return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7FFFFFFFu) >> 3) + 0x38000000u)), (int)(b << 29));
 }
 // a0 + a1 + a2 + a3 (a0, a1, a2 exact integer sums, a3 rounded) through an FP32 pair
@@ -129,10 +130,12 @@ __device__ __forceinline__ double combine4(float a0, float a1, float a2, float a
   e += e2;
   return widen(s) + widen(e);
 }
-// x 2^k by the exponent field (x zero or a normal number that stays normal)
+// x 2^k by the exponent field; subnormal operands and results to zero, NaN and Inf stay
 __device__ __forceinline__ double shift_exp(double x, int k) {
-  const int hi = __double2hiint(x);
-  return (hi & 0x7FF00000) == 0 ? 0.0 : __hiloint2double(hi + (k << 20), __double2loint(x));
+  const int hi = __double2hiint(x), e = (hi >> 20) & 0x7FF, r = e + k;
+  if (e == 0x7FF) return x;
+  if (r >= 0x7FF) return x * 0x1p1023 * 0x1p1023;
+  return e == 0 || r <= 0 ? 0.0 : __hiloint2double(hi + (k << 20), __double2loint(x));
 }
 
 template <class PR>
