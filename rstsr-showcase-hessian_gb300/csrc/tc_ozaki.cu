@@ -25,14 +25,11 @@
 // adds alpha 2^(eA + eB) (hi + lo) into the FP64 output (terms 1 and 2, split over K ranges
 // across CTAs) or stores the pair 2^(eA + eB) (hi, lo) into a staging array (T, W).
 //
-// Terms 1 and 2 run on CTA pairs (tc_pair.cu); the kernels below generate T and W and evaluate the
-// XC term.  Kernel structure (one CTA per SM, 4 warps):
-//   warp 0 lane 0  -- TMA producer: 3-D tiled loads of the 6 + 6 slice tiles (K = 32 wide,
-//                     64B swizzle) into a 2-stage ring;
-//   warp 1         -- MMA issuer (warp-uniform, one elected lane): 21 x tcgen05.mma.kind::f16
-//                     (BF16, M=128, N=BN, K=16) per K step into 4 accumulators (4 x BN TMEM columns);
-//   warp 2         -- TMEM allocation and release;
-//   warps 0-3      -- epilogue.
+// Terms 1 and 2 and the XC response's contractions run on CTA pairs (tc_pair.cu); the kernels below
+// generate T and W (ten warps: TMA producer, MMA issuer, eight of epilogue) and reduce the XC
+// response's first contraction to rho1 (four warps).  TMA loads 3-D tiles (K = 32 wide, 64B swizzle)
+// into a ring of stages; the MMAs (M=128, N=BN, K=16; 21 per K step for six slices into 4
+// accumulators) are issued warp-uniformly by one elected lane.
 // Every mbarrier wait is bounded; on expiry the kernel raises the error flag and returns.
 //
 // The same kernel template also runs the split-precision operator of the inner solves
@@ -84,30 +81,24 @@ struct OzArgs {
   void* out;
   int M, N;
   int m_tiles;
-  int nkb;                  // K blocks of 32 per aux function
-  int total_kb;             // split mode: K blocks of the chunk (np * nkb)
+  int nkb;                  // K blocks of 32 (batched: per aux function)
   int a_depth, b_depth;     // plane stride of A / B in depth units (slice t at depth t * stride)
   int a_off, b_off;         // depth offset of the chunk's aux function 0
-  int a_per_p;              // A depth advances with the aux function
-  int a_row0;               // split mode: first A row of the contraction (A rows need no alignment)
-  int b_k0;                 // split mode: K offset of B (elements, a multiple of 16 bytes)
-  int store;                // split mode with one K range per tile: store instead of accumulating
-  // split-FP16 split mode, rho1 epilogue (when rho is set): instead of out, accumulate
-  // rho[m + ld_rho a] += sum_i value[m, n = i + rho_nocc a] ao[m + ld_ao i]
+  int a_row0;               // rho1: first A row of the contraction (A rows need no alignment)
+  int b_k0;                 // rho1: K offset of B (elements, a multiple of 16 bytes)
+  // rho1: rho[m + ld_rho a] += sum_i value[m, n = i + rho_nocc a] ao[m + ld_ao i]
   float* rho;
   const float* rho_ao;
   int64_t ld_rho, ld_ao;
   int rho_nocc;
   int np, p_per_cta;        // batched: aux functions of the launch, per CTA
-  int kb_per_cta;           // split: K blocks per CTA (<= KMAX / BK, the exactness bound)
   // batched split-FP16 T generation writing the FP16 hi / lo planes of T * (*tscale) for
   // tc_gemm.cu's term 1
   const float* tscale;
   void* out_lo;             // the lo plane (same layout as out, the hi plane)
-  // split mode epilogue: out [m + ld_out n] += value rowscale[m] colscale[n] (double: Exact6, float: Split2)
+  // rho1: scales of A's rows and B's
   const double* rowscale;
   const double* colscale;
-  int64_t ld_out;
   // batched mode epilogue: out [(m % m_div) s_m1 + (m / m_div) s_m2 + n s_n + Pl s_p]
   //   = 2^(e_row[m] + e_col[(b_off + Pl) N + n] - 2 EOFF) value (float2 pair: Exact6, float: Split2;
   //   EPI_SPLIT16 takes e_col uniform over an aux function's columns and reads its first)
@@ -136,12 +127,14 @@ __device__ __forceinline__ void combine4(float a0, float a1, float a2, float a3,
   lo = e - (hi - s);
 }
 
-// Split-K contractions (terms 1 and 2): one CTA per (tile, K range of at most KMAX).  ST
-// pipeline stages (fewer for short K ranges, so that two CTAs share an SM and one's epilogue
-// overlaps the other's MMAs).
-template <class PR, int BN, int ST = PR::STAGES>
+// First grid step of the split-FP16 XC response: the rows' products with bra, reduced to rho1 in the
+// epilogue.  One CTA per tile; ST pipeline stages (fewer for short K, so that two CTAs share an SM
+// and one's epilogue overlaps the other's MMAs).
+template <int ST>
 __global__ void __launch_bounds__(128, 1)
-    tc_slice_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant__ CUtensorMap mB, OzArgs args) {
+    tc_rho_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant__ CUtensorMap mB, OzArgs args) {
+  using PR = Split2;
+  constexpr int BN = 128;
   using C = Cfg<PR, BN, ST>;
   constexpr int STAGES = C::STAGES;
   extern __shared__ uint8_t smem_raw[];
@@ -151,11 +144,10 @@ __global__ void __launch_bounds__(128, 1)
   const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + STAGES), accum = smem_u32(bars + 2 * STAGES);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // x = tile (M fastest: CTAs that share a B tile run together), y = K range
+  // M fastest: CTAs that share a B tile run together
   const int m_tile = blockIdx.x % args.m_tiles, n_tile = blockIdx.x / args.m_tiles;
   const int m0 = m_tile * BM, n0 = n_tile * BN;
-  const int kb0 = blockIdx.y * args.kb_per_cta;
-  const int total = min(args.total_kb - kb0, args.kb_per_cta);
+  const int total = args.nkb;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -165,7 +157,7 @@ __global__ void __launch_bounds__(128, 1)
     mbar_init(accum, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  constexpr uint32_t TMEM_COLS = PR::NACC * BN;  // one accumulator per group
+  constexpr uint32_t TMEM_COLS = BN;
   if (warp == 2) tmem_alloc(smem_u32(tmem_slot), TMEM_COLS);
   fence_before_sync();
   __syncthreads();
@@ -183,16 +175,12 @@ __global__ void __launch_bounds__(128, 1)
         issued = it + 1;
         const uint32_t full = full0 + 8 * s;
         mbar_expect_tx(full, C::STAGE_BYTES);
-        const int kb = kb0 + it;
-        const int P = kb / args.nkb;
-        const int k0 = (kb % args.nkb) * BK;
-        const int da = args.a_off + (args.a_per_p ? P : 0);
-        const int db = args.b_off + P;
+        const int k0 = it * BK;
         const uint32_t st = smem_u32(smem + s * C::STAGE_BYTES);
 #pragma unroll
         for (int t = 0; t < PR::S; ++t) {
-          tma_load_3d(st + t * C::A_TILE, &mA, full, k0, m0 + args.a_row0, t * args.a_depth + da);
-          tma_load_3d(st + PR::S * C::A_TILE + t * C::B_TILE, &mB, full, k0 + args.b_k0, n0, t * args.b_depth + db);
+          tma_load_3d(st + t * C::A_TILE, &mA, full, k0, m0 + args.a_row0, t * args.a_depth);
+          tma_load_3d(st + PR::S * C::A_TILE + t * C::B_TILE, &mB, full, k0 + args.b_k0, n0, t * args.b_depth);
         }
       }
       for (int it = max(0, issued - STAGES); it < issued; ++it)
@@ -212,23 +200,10 @@ __global__ void __launch_bounds__(128, 1)
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k) {
             const uint64_t dk = desc_off(k * 32);  // 16 elements = 32 B along K inside the swizzle row
-            if constexpr (PR::NACC == 4) {
-#pragma unroll
-              for (int g = 0; g < PR::S; ++g) {
-#pragma unroll
-                for (int t = 0; t <= g; ++t) {
-                  const int acc = g < 3 ? g : 3;
-                  const bool first = it == 0 && k == 0 && t == 0 && g <= 3;
-                  mma_f16(tmem + (uint32_t)(acc * BN), da + (desc_off(t * C::A_TILE) + dk),
-                          db + (desc_off((g - t) * C::B_TILE) + dk), idesc, first ? 0u : 1u);
-                }
-              }
-            } else {
-              // hi*hi + hi*lo + lo*hi
-              mma_f16(tmem, da + dk, db + dk, idesc, (it > 0 || k > 0) ? 1u : 0u);
-              mma_f16(tmem, da + dk, db + (desc_off(C::B_TILE) + dk), idesc, 1u);
-              mma_f16(tmem, da + (desc_off(C::A_TILE) + dk), db + dk, idesc, 1u);
-            }
+            // hi*hi + hi*lo + lo*hi
+            mma_f16(tmem, da + dk, db + dk, idesc, (it > 0 || k > 0) ? 1u : 0u);
+            mma_f16(tmem, da + dk, db + (desc_off(C::B_TILE) + dk), idesc, 1u);
+            mma_f16(tmem, da + (desc_off(C::A_TILE) + dk), db + dk, idesc, 1u);
           }
           mma_commit(empty0 + 8 * s);
         }
@@ -245,101 +220,53 @@ __global__ void __launch_bounds__(128, 1)
       const int row = m0 + warp * 32 + lane;
       const bool row_ok = row < args.M;
       const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
-      const double rs = row_ok ? args.rowscale[row] : 0.0;
-      const float rsf = (float)rs;
-      // rho1 epilogue state: orbital i and right-hand side a of column n0, partial sum
-      int rho_i = 0, rho_a = 0;
+      const float rsf = row_ok ? (float)args.rowscale[row] : 0.f;
+      // orbital i and right-hand side a of column n0, partial sum
+      int rho_i = n0 % args.rho_nocc, rho_a = n0 / args.rho_nocc;
       float rho_acc = 0.f;
-      const float* rho_ao_row = nullptr;
-      if constexpr (PR::NACC == 1) {
-        if (args.rho != nullptr) {
-          rho_i = n0 % args.rho_nocc;
-          rho_a = n0 / args.rho_nocc;
-          rho_ao_row = args.rho_ao + (row_ok ? row : 0);
-        }
-      }
+      const float* const rho_ao_row = args.rho_ao + (row_ok ? row : 0);
       for (int c = 0; c < BN / 32; ++c) {
-        if constexpr (PR::NACC == 4) {
-          float v0[32], v1[32], v2[32], v3[32];
-          tmem_ld32(lane_base + (uint32_t)(0 * BN + c * 32), v0);
-          tmem_ld32(lane_base + (uint32_t)(1 * BN + c * 32), v1);
-          tmem_ld32(lane_base + (uint32_t)(2 * BN + c * 32), v2);
-          if constexpr (PR::S > 3) {
-            tmem_ld32(lane_base + (uint32_t)(3 * BN + c * 32), v3);
-          } else {
+        float v[32];
+        tmem_ld32(lane_base + (uint32_t)(c * 32), v);
+        // the chunk's 32 column scales: one load per lane, broadcast by shuffles (no FP64 per
+        // element); rowscale and colscale are powers of two (times a small factor), so the
+        // FP32 product equals the FP64 one
+        float cs[32];
+        {
+          const int nl = n0 + c * 32 + lane;
+          const float csl = nl < args.N ? (float)args.colscale[nl] : 0.f;
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v3[j] = 0.f;  // groups 0-2 only: the fourth accumulator is unused
-          }
-          if (row_ok) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              const int n = n0 + c * 32 + j;
-              if (n < args.N) {
-                float hi, lo;
-                combine4(v0[j], v1[j], v2[j], v3[j], hi, lo);
-                const double v = ((double)hi + (double)lo) * (rs * args.colscale[n]);
-                double* o = reinterpret_cast<double*>(args.out) + row + args.ld_out * (int64_t)n;
-                if (args.store) *o = v;
-                else atomicAdd(o, v);
-              }
-            }
-          }
-        } else {
-          float v[32];
-          tmem_ld32(lane_base + (uint32_t)(c * 32), v);
-          // the chunk's 32 column scales: one load per lane, broadcast by shuffles (no FP64 per
-          // element); rowscale and colscale are powers of two (times a small factor), so the
-          // FP32 product equals the FP64 one
-          float cs[32];
+          for (int j = 0; j < 32; ++j) cs[j] = __shfl_sync(0xffffffffu, csl, j) * rsf;
+        }
+        if (row_ok) {
+          // rho1 of this row: columns n = i + nocc a, the running i / a carried across chunks.
+          // The chunk's 32 ao values are loaded first, back to back (independent L2 loads),
+          // then reduced.
+          float aov[32];
           {
-            const int nl = n0 + c * 32 + lane;
-            const float csl = nl < args.N ? (float)args.colscale[nl] : 0.f;
+            int ii = rho_i;
 #pragma unroll
-            for (int j = 0; j < 32; ++j) cs[j] = __shfl_sync(0xffffffffu, csl, j) * rsf;
+            for (int j = 0; j < 32; ++j) {
+              aov[j] = n0 + c * 32 + j < args.N ? rho_ao_row[args.ld_ao * (int64_t)ii] : 0.f;
+              if (++ii == args.rho_nocc) ii = 0;
+            }
           }
-          if (row_ok && args.rho != nullptr) {
-            // rho1 of this row: columns n = i + nocc a, the running i / a carried across chunks.
-            // The chunk's 32 ao values are loaded first, back to back (independent L2 loads),
-            // then reduced.
-            float aov[32];
-            {
-              int ii = rho_i;
 #pragma unroll
-              for (int j = 0; j < 32; ++j) {
-                aov[j] = n0 + c * 32 + j < args.N ? rho_ao_row[args.ld_ao * (int64_t)ii] : 0.f;
-                if (++ii == args.rho_nocc) ii = 0;
-              }
-            }
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              const int n = n0 + c * 32 + j;
-              if (n < args.N) {
-                rho_acc += v[j] * cs[j] * aov[j];
-                if (++rho_i == args.rho_nocc) {
-                  atomicAdd(args.rho + row + args.ld_rho * (int64_t)rho_a, rho_acc);
-                  rho_acc = 0.f;
-                  rho_i = 0;
-                  ++rho_a;
-                }
-              }
-            }
-          } else if (row_ok) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              const int n = n0 + c * 32 + j;
-              if (n < args.N) {
-                float* o = reinterpret_cast<float*>(args.out) + row + args.ld_out * (int64_t)n;
-                const float x = v[j] * cs[j];
-                if (args.store) *o = x;
-                else atomicAdd(o, x);
+          for (int j = 0; j < 32; ++j) {
+            const int n = n0 + c * 32 + j;
+            if (n < args.N) {
+              rho_acc += v[j] * cs[j] * aov[j];
+              if (++rho_i == args.rho_nocc) {
+                atomicAdd(args.rho + row + args.ld_rho * (int64_t)rho_a, rho_acc);
+                rho_acc = 0.f;
+                rho_i = 0;
+                ++rho_a;
               }
             }
           }
         }
       }
-      if constexpr (PR::NACC == 1) {
-        if (row_ok && args.rho != nullptr && rho_i > 0) atomicAdd(args.rho + row + args.ld_rho * (int64_t)rho_a, rho_acc);
-      }
+      if (row_ok && rho_i > 0) atomicAdd(args.rho + row + args.ld_rho * (int64_t)rho_a, rho_acc);
     }
   }
   fence_before_sync();
@@ -1123,22 +1050,15 @@ CUtensorMap make_map(const void* base, int64_t K, int64_t rows, int64_t depth, i
   return m;
 }
 
-template <class PR, int BN>
-bool set_short_smem_attr() {
-  if constexpr (PR::NACC == 4) {
-    return true;
-  } else {
-    return cudaFuncSetAttribute(tc_slice_kernel<PR, BN, SHORT_STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                Cfg<PR, BN, SHORT_STAGES>::SMEM_BYTES) == cudaSuccess;
-  }
+template <int ST>
+bool set_rho_smem_attr() {
+  return cudaFuncSetAttribute(tc_rho_kernel<ST>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              Cfg<Split2, 128, ST>::SMEM_BYTES) == cudaSuccess;
 }
 
-template <class PR, int BN>
+template <class PR>
 bool set_smem_attr() {
-  bool ok = cudaFuncSetAttribute(tc_slice_kernel<PR, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 Cfg<PR, BN>::SMEM_BYTES) == cudaSuccess &&
-            set_short_smem_attr<PR, BN>() &&
-            cudaFuncSetAttribute(tc_slice_batched_kernel<PR, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  bool ok = cudaFuncSetAttribute(tc_slice_batched_kernel<PR, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  Batched<PR>::SMEM_BYTES) == cudaSuccess;
   if constexpr (PR::NACC == 4)
     ok = ok && cudaFuncSetAttribute(tc_slice_batched_kernel<PR, 64, EPI_STOREMAX>,
@@ -1199,51 +1119,6 @@ float time_launch(cudaStream_t s, F&& launch) {
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   return ms;
-}
-
-// split-K contraction: grid (tiles, K ranges)
-template <class PR, int BN, int ST = PR::STAGES>
-void launch_split_raw(cphf_ctx* c, const CUtensorMap& mA, const CUtensorMap& mB, const OzArgs& a) {
-  const unsigned tiles = (unsigned)(a.m_tiles * div_up(a.N, BN));
-  const int64_t ranges = div_up(a.total_kb, a.kb_per_cta);
-  if (ranges > 65535) throw Error(CPHF_ERR_ARG, "tensor-core K term: grid too large");
-  tc_slice_kernel<PR, BN, ST><<<dim3(tiles, (unsigned)ranges), 128, Cfg<PR, BN, ST>::SMEM_BYTES, c->stream>>>(mA, mB, a);
-  count_launch();
-  CPHF_CUDA(cudaGetLastError());
-}
-
-template <class PR, int BN>
-void launch_split(cphf_ctx* c, OzState& z, const CUtensorMap& mA, const CUtensorMap& mB, OzArgs a) {
-  const TuneKey key{PR::S * 1000 + BN, a.M, a.N, a.nkb, a.total_kb};
-  auto& tab = tune_table();
-  int best = PR::NACC == 1 ? (int)std::max<int64_t>(1, div_up(a.total_kb, 4)) : KB_PER_CTA;
-  if (!tab.find(key, best) && !capturing(c->stream)) {
-    // candidates run into a scratch output (the real one accumulates)
-    const size_t esize = PR::NACC == 4 ? 8 : 4;
-    const size_t bytes = (size_t)a.ld_out * a.N * esize;
-    z.tune_out.ensure(bytes, c->counter());
-    OzArgs t = a;
-    t.out = z.tune_out.p;
-    float best_ms = 0.f;
-    // exact slices: K ranges within the exactness bound; split FP16 (no bound): 1, 2 or 4
-    // waves of CTAs over the tiles, each K range as long as that leaves it
-    int cand[3] = {KB_PER_CTA, KB_PER_CTA / 2, KB_PER_CTA / 3};
-    if (PR::NACC == 1) {
-      const int64_t tiles = (int64_t)a.m_tiles * div_up(a.N, BN);
-      const int64_t r0 = std::max<int64_t>(1, div_up(2 * (int64_t)c->num_sms, tiles));
-      for (int q = 0; q < 3; ++q)
-        cand[q] = (int)std::max<int64_t>(1, div_up(a.total_kb, std::min<int64_t>(r0 << q, a.total_kb)));
-    }
-    for (int kb : cand) {
-      t.kb_per_cta = kb;
-      if (div_up(t.total_kb, kb) > 65535) continue;
-      const float ms = time_launch(c->stream, [&] { launch_split_raw<PR, BN>(c, mA, mB, t); });
-      if (best_ms == 0.f || ms < best_ms) best_ms = ms, best = kb;
-    }
-    tab.put(key, best);
-  }
-  a.kb_per_cta = best;
-  launch_split_raw<PR, BN>(c, mA, mB, a);
 }
 
 // exact split-K contraction on CTA pairs: K blocks per pair tuned once per shape (candidates run
@@ -1378,7 +1253,6 @@ OzArgs base_args(OzState& z, int M, int N) {
   a.M = M;
   a.N = N;
   a.m_tiles = (int)div_up(M, BM);
-  a.kb_per_cta = KB_PER_CTA;
   a.err = z.err.as<int>();
   return a;
 }
@@ -1392,8 +1266,8 @@ bool oz_available(cphf_ctx* c) {
   static bool attr_ok = false, tried = false;
   if (!tried) {
     tried = true;
-    attr_ok = set_smem_attr<Exact6, 128>() && set_smem_attr<Exact6c, 128>() && set_smem_attr<Exact6c3, 128>() &&
-              set_smem_attr<Split2, 128>();
+    attr_ok = set_smem_attr<Exact6>() && set_smem_attr<Exact6c>() && set_smem_attr<Exact6c3>() &&
+              set_smem_attr<Split2>() && set_rho_smem_attr<SHORT_STAGES>() && set_rho_smem_attr<Split2::STAGES>();
     if (!attr_ok) cudaGetLastError();
   }
   return attr_ok;
@@ -1760,79 +1634,76 @@ void lp_w_term2(cphf_ctx* c, OzState& z, int s, int64_t P0, int64_t npc, int64_t
   }
 }
 
-// Split-FP16 contraction out[m, n] += rowscale[m] colscale[n] sum_k A[a_row0 + m, k] B[n, k]
-// over FP16 hi / lo planes (plane stride rows x ld elements), K-major, FP32 atomics into out
-// [m + ld_out n]; the K range is split over CTAs as the autotuner finds best.
-template <class PR, class TOut>
-void plane_gemm(cphf_ctx* c, OzState& z, const PlaneMat& A, int64_t a_row0, const PlaneMat& B, int64_t b_k0,
-                int64_t M, int64_t N, int64_t K, const double* rowscale, const double* colscale, TOut* out,
-                int64_t ld_out, int* err, int kb_per_cta, bool store, const RhoEpilogue* rho = nullptr) {
+// out[m + ld_out n] (+)= rowscale[m] colscale[n] sum_k A[a_row0 + m, k] B[n, b_k0 + k] on CTA pairs
+static PairTerm plane_term(const PlaneMat& A, int64_t a_row0, const PlaneMat& B, int64_t b_k0, int planes, int64_t M,
+                           int64_t N, int64_t K, const double* rowscale, const double* colscale, void* out,
+                           int64_t ld_out, int* err) {
+  if (b_k0 % 8 != 0 || b_k0 < 0) throw Error(CPHF_ERR_ARG, "tensor-core contraction: B offset not 16-byte aligned");
+  // split FP16: hi and lo as separate stacks of depth 1; exact slices: one stack of six
+  const bool split = planes == 2;
+  auto stack = [&](const PlaneMat& m) {
+    const __half* p = static_cast<const __half*>(m.p);
+    return PairPlanes{{p, split ? p + m.rows * m.ld : p}, m.rows, m.ld, split ? 1 : planes, split ? 0 : 1, m.kext};
+  };
+  PairTerm t{};
+  t.x = stack(A);
+  t.y = stack(B);
+  t.np = 1;
+  t.M = M; t.N = N; t.K = K;
+  t.rowscale = rowscale;
+  t.colscale = colscale;
+  t.out = out;
+  t.ld_out = ld_out;
+  t.err = err;
+  t.x_row0 = a_row0;
+  t.y_k0 = b_k0;
+  return t;
+}
+
+void lp_gemm(cphf_ctx* c, const PlaneMat& A, int64_t a_row0, const PlaneMat& B, int64_t b_k0, int64_t M, int64_t N,
+             int64_t K, const double* rowscale, const double* colscale, float* out, int64_t ld_out, int* err) {
+  if (M <= 0 || N <= 0 || K <= 0) return;
+  pair_split2(c, plane_term(A, a_row0, B, b_k0, 2, M, N, K, rowscale, colscale, out, ld_out, err));
+}
+
+void lp_gemm_rho(cphf_ctx* c, OzState& z, const PlaneMat& A, int64_t a_row0, const PlaneMat& B, int64_t b_k0,
+                 int64_t M, int64_t N, int64_t K, const double* rowscale, const double* colscale,
+                 const RhoEpilogue& rho, int* err) {
   if (M <= 0 || N <= 0 || K <= 0) return;
   if (b_k0 % 8 != 0 || b_k0 < 0) throw Error(CPHF_ERR_ARG, "tensor-core contraction: B offset not 16-byte aligned");
-  const CUtensorMap mA = make_map(A.p, A.kext, A.rows, PR::S, A.ld, BM, PR::BF16);
-  const CUtensorMap mB = make_map(B.p, B.kext, B.rows, PR::S, B.ld, BM, PR::BF16);
+  if (rho.nocc <= 0) throw Error(CPHF_ERR_ARG, "rho1 epilogue: no occupied orbital");
+  const CUtensorMap mA = make_map(A.p, A.kext, A.rows, Split2::S, A.ld, BM, false);
+  const CUtensorMap mB = make_map(B.p, B.kext, B.rows, Split2::S, B.ld, BM, false);
   OzArgs a = base_args(z, (int)M, (int)N);
   a.err = err;
-  a.out = out;
   a.nkb = (int)div_up(K, BK);
-  a.total_kb = a.nkb;
   a.a_depth = 1;
   a.b_depth = 1;
   a.a_row0 = (int)a_row0;
   a.b_k0 = (int)b_k0;
   a.rowscale = rowscale;
   a.colscale = colscale;
-  a.ld_out = ld_out;
-  if (rho != nullptr) {
-    if (PR::NACC != 1 || rho->nocc <= 0) throw Error(CPHF_ERR_ARG, "rho1 epilogue: split-FP16 contractions only");
-    a.rho = rho->rho;
-    a.rho_ao = rho->ao;
-    a.ld_rho = rho->ld_rho;
-    a.ld_ao = rho->ld_ao;
-    a.rho_nocc = (int)rho->nocc;
-  }
-  if (kb_per_cta > 0) {
-    a.kb_per_cta = PR::NACC == 4 ? std::min(kb_per_cta, KB_PER_CTA) : kb_per_cta;
-    a.store = store && a.kb_per_cta >= a.total_kb;
-    bool launched = false;
-    if constexpr (PR::NACC == 1) {
-      if (a.kb_per_cta <= 2 * SHORT_STAGES) {
-        launch_split_raw<PR, 128, SHORT_STAGES>(c, mA, mB, a);
-        launched = true;
-      }
-    }
-    if (!launched) launch_split_raw<PR, 128>(c, mA, mB, a);
-  } else {
-    launch_split<PR, 128>(c, z, mA, mB, a);
-  }
-}
-
-void lp_gemm(cphf_ctx* c, OzState& z, const PlaneMat& A, int64_t a_row0, const PlaneMat& B, int64_t b_k0, int64_t M,
-             int64_t N, int64_t K, const double* rowscale, const double* colscale, float* out, int64_t ld_out,
-             int* err, int kb_per_cta, bool store) {
-  plane_gemm<Split2>(c, z, A, a_row0, B, b_k0, M, N, K, rowscale, colscale, out, ld_out, err, kb_per_cta, store);
-}
-
-void lp_gemm_rho(cphf_ctx* c, OzState& z, const PlaneMat& A, int64_t a_row0, const PlaneMat& B, int64_t b_k0,
-                 int64_t M, int64_t N, int64_t K, const double* rowscale, const double* colscale,
-                 const RhoEpilogue& rho, int* err, int kb_per_cta) {
-  plane_gemm<Split2>(c, z, A, a_row0, B, b_k0, M, N, K, rowscale, colscale, (float*)nullptr, 0, err, kb_per_cta, false,
-                     &rho);
-}
-
-void oz_gemm(cphf_ctx* c, OzState& z, const PlaneMat& A, int64_t a_row0, const PlaneMat& B, int64_t b_k0, int64_t M,
-             int64_t N, int64_t K, const double* rowscale, const double* colscale, double* out, int64_t ld_out,
-             int* err, int kb_per_cta, bool store) {
-  plane_gemm<Exact6>(c, z, A, a_row0, B, b_k0, M, N, K, rowscale, colscale, out, ld_out, err, kb_per_cta, store);
-}
-
-void oz_gemm_corr(cphf_ctx* c, OzState& z, int slices, const PlaneMat& A, int64_t a_row0, const PlaneMat& B,
-                  int64_t b_k0, int64_t M, int64_t N, int64_t K, const double* rowscale, const double* colscale,
-                  double* out, int64_t ld_out, int* err, int kb_per_cta, bool store) {
-  if (slices == 3)
-    plane_gemm<Exact6c3>(c, z, A, a_row0, B, b_k0, M, N, K, rowscale, colscale, out, ld_out, err, kb_per_cta, store);
+  a.rho = rho.rho;
+  a.rho_ao = rho.ao;
+  a.ld_rho = rho.ld_rho;
+  a.ld_ao = rho.ld_ao;
+  a.rho_nocc = (int)rho.nocc;
+  const unsigned tiles = (unsigned)(a.m_tiles * div_up(N, 128));
+  if (a.nkb <= 2 * SHORT_STAGES)
+    tc_rho_kernel<SHORT_STAGES><<<tiles, 128, Cfg<Split2, 128, SHORT_STAGES>::SMEM_BYTES, c->stream>>>(mA, mB, a);
   else
-    plane_gemm<Exact6c>(c, z, A, a_row0, B, b_k0, M, N, K, rowscale, colscale, out, ld_out, err, kb_per_cta, store);
+    tc_rho_kernel<Split2::STAGES><<<tiles, 128, Cfg<Split2, 128>::SMEM_BYTES, c->stream>>>(mA, mB, a);
+  count_launch();
+  CPHF_CUDA(cudaGetLastError());
+}
+
+void oz_gemm(cphf_ctx* c, int slices, const PlaneMat& A, int64_t a_row0, const PlaneMat& B, int64_t b_k0, int64_t M,
+             int64_t N, int64_t K, const double* rowscale, const double* colscale, double* out, int64_t ld_out,
+             int* err, bool store) {
+  if (M <= 0 || N <= 0 || K <= 0) return;
+  PairTerm t = plane_term(A, a_row0, B, b_k0, slices, M, N, K, rowscale, colscale, out, ld_out, err);
+  t.store = store;
+  pair_exact(c, t, slices, 0);
 }
 
 // Split-FP16 planes [t][r][ld] of FP32 rows r (K elements each, row stride rs), exponents to e_out.

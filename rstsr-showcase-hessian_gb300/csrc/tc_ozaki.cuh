@@ -44,14 +44,11 @@ struct PlaneMat {
   int64_t rows, ld, kext;
 };
 
-// Split-FP16 contraction (hi / lo planes, three products, FP32 accumulation)
+// Split-FP16 contraction (hi / lo planes, three products, FP32 accumulation) on CTA pairs
 //   out[m + ld_out n] += rowscale[m] colscale[n] sum_{k < K} A[a_row0 + m, k] B[n, b_k0 + k]
-// with FP32 atomics; b_k0 a multiple of 8.  The K range is split over CTAs in ranges of
-// kb_per_cta blocks of 32 (0: as the autotuner finds best); with store and one range per
-// tile the values are stored, not accumulated.
-void lp_gemm(cphf_ctx* c, OzState& z, const PlaneMat& A, int64_t a_row0, const PlaneMat& B, int64_t b_k0, int64_t M,
-             int64_t N, int64_t K, const double* rowscale, const double* colscale, float* out, int64_t ld_out,
-             int* err, int kb_per_cta = 0, bool store = false);
+// with FP32 atomics; b_k0 a multiple of 8.
+void lp_gemm(cphf_ctx* c, const PlaneMat& A, int64_t a_row0, const PlaneMat& B, int64_t b_k0, int64_t M, int64_t N,
+             int64_t K, const double* rowscale, const double* colscale, float* out, int64_t ld_out, int* err);
 
 // split-FP16 planes [t][r][ld] of FP32 rows r (K elements each, row stride rs); row exponents to e_out
 void lp_slice_rows(cphf_ctx* c, const float* src, int64_t rows, int64_t K, int64_t rs, __half* dst, int64_t ld,
@@ -67,22 +64,19 @@ struct RhoEpilogue {
 };
 void lp_gemm_rho(cphf_ctx* c, OzState& z, const PlaneMat& A, int64_t a_row0, const PlaneMat& B, int64_t b_k0,
                  int64_t M, int64_t N, int64_t K, const double* rowscale, const double* colscale,
-                 const RhoEpilogue& rho, int* err, int kb_per_cta);
+                 const RhoEpilogue& rho, int* err);
 
-// The same contraction on exact BF16 slice planes (six per operand, 21 products, FP64 out,
-// K ranges of at most 3072 per CTA so that the leading groups accumulate exactly); row and
-// column scales are 2^e of the slicing exponents.
-void oz_gemm(cphf_ctx* c, OzState& z, const PlaneMat& A, int64_t a_row0, const PlaneMat& B, int64_t b_k0, int64_t M,
+// The same contraction on exact BF16 slice planes (6: 21 products, 4 or 3: the leading planes, 10 / 6
+// products; FP64 out, K ranges of at most 3072 per CTA pair so that the leading groups accumulate
+// exactly); row and column scales are 2^e of the slicing exponents (columns: times any factor).
+// store (K <= 3072): the values are stored, not accumulated.
+void oz_gemm(cphf_ctx* c, int slices, const PlaneMat& A, int64_t a_row0, const PlaneMat& B, int64_t b_k0, int64_t M,
              int64_t N, int64_t K, const double* rowscale, const double* colscale, double* out, int64_t ld_out,
-             int* err, int kb_per_cta = 0, bool store = false);
+             int* err, bool store);
 // exact BF16 slice planes [t][r][ld] of FP64 rows r (K elements each, row stride rs); exponents to e_out
 void oz_slice_rows(cphf_ctx* c, const double* src, int64_t rows, int64_t K, int64_t rs, __nv_bfloat16* dst,
                    int64_t ld, int* e_out);
-// the same contraction and slicer in correction precision: the leading `slices` (3 or 4) planes,
-// the products with t + u < slices
-void oz_gemm_corr(cphf_ctx* c, OzState& z, int slices, const PlaneMat& A, int64_t a_row0, const PlaneMat& B,
-                  int64_t b_k0, int64_t M, int64_t N, int64_t K, const double* rowscale, const double* colscale,
-                  double* out, int64_t ld_out, int* err, int kb_per_cta = 0, bool store = false);
+// the leading `slices` (3 or 4) planes only
 void oz_slice_rows_corr(cphf_ctx* c, int slices, const double* src, int64_t rows, int64_t K, int64_t rs,
                         __nv_bfloat16* dst, int64_t ld, int* e_out);
 

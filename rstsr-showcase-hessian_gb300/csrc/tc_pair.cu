@@ -62,6 +62,7 @@ struct PairArgs {
   int m_tiles;
   int nkb, total_kb, kb_per_cta;
   int x_off, x_depth, y_depth;  // depth strides of the planes (exact), depth offset of X
+  int x_row0, y_k0, store;
   int stages, b_tile, stage_bytes;
   const double* rowscale;  // exact: powers of two
   const double* colscale;
@@ -112,13 +113,13 @@ __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
   const float bb = s - a;
   e = (a - (s - bb)) + (b - bb);
 }
-// float -> double on the integer pipe (subnormals, far below any group sum's unit, to zero): the
-// conversion instruction occupies the FP64 pipe like a multiplication
+// float -> double on the integer pipe (subnormals, far below any group sum's unit, to zero; NaN and
+// Inf, from non-finite operands, stay): the conversion instruction occupies the FP64 pipe like a
+// multiplication.  Branch-free: it is unrolled over an accumulator chunk.
 __device__ __forceinline__ double widen(float x) {
-  const unsigned b = __float_as_uint(x);
-  if ((b & 0x7F800000u) == 0u) return 0.0;
-  if ((b & 0x7F800000u) == 0x7F800000u) return (double)x;  // NaN slices of non-finite operands
-  return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7FFFFFFFu) >> 3) + 0x38000000u)), (int)(b << 29));
+  const unsigned b = __float_as_uint(x), e = b & 0x7F800000u;
+  const unsigned hi = (b & 0x80000000u) | (((b & 0x7FFFFFFFu) >> 3) + 0x38000000u) | (e == 0x7F800000u ? 0x7FF00000u : 0u);
+  return __hiloint2double(e == 0u ? 0 : (int)hi, e == 0u ? 0 : (int)(b << 29));
 }
 // a0 + a1 + a2 + a3 (a0, a1, a2 exact integer sums, a3 rounded) through an FP32 pair
 __device__ __forceinline__ double combine4(float a0, float a1, float a2, float a3) {
@@ -133,9 +134,9 @@ __device__ __forceinline__ double combine4(float a0, float a1, float a2, float a
 // x 2^k by the exponent field; subnormal operands and results to zero, NaN and Inf stay
 __device__ __forceinline__ double shift_exp(double x, int k) {
   const int hi = __double2hiint(x), e = (hi >> 20) & 0x7FF, r = e + k;
-  if (e == 0x7FF) return x;
-  if (r >= 0x7FF) return x * 0x1p1023 * 0x1p1023;
-  return e == 0 || r <= 0 ? 0.0 : __hiloint2double(hi + (k << 20), __double2loint(x));
+  const bool zero = e == 0 || (r <= 0 && e != 0x7FF), inf = r >= 0x7FF && e != 0x7FF;
+  const int h = e == 0x7FF ? hi : inf ? (hi & (int)0x80000000u) | 0x7FF00000 : hi + (k << 20);
+  return __hiloint2double(zero ? 0 : h, zero || inf ? 0 : __double2loint(x));
 }
 
 template <class PR>
@@ -190,12 +191,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
       const int P = kb / args.nkb, k0 = (kb - P * args.nkb) * C::BK;
       const uint32_t st = smem_u32(smem + s * args.stage_bytes);
       const uint32_t sb = st + PR::S * C::A_TILE;
-      const int mb = m0 + (int)rank * (args.NT / 2);
+      const int mb = args.x_row0 + m0 + (int)rank * (args.NT / 2);
 #pragma unroll
       for (int t = 0; t < PR::S; ++t) {
         const CUtensorMap* y = !C::EXACT && t == 1 ? &mY1 : &mY0;
         const CUtensorMap* x = !C::EXACT && t == 1 ? &mX1 : &mX0;
-        tma_load_3d_pair(st + t * C::A_TILE, y, full, k0, n0, C::EXACT ? t * args.y_depth + P : P);
+        tma_load_3d_pair(st + t * C::A_TILE, y, full, args.y_k0 + k0, n0, C::EXACT ? t * args.y_depth + P : P);
         tma_load_3d_pair(sb + t * args.b_tile, x, full, k0, mb, (C::EXACT ? t * args.x_depth : 0) + args.x_off + P);
       }
     }
@@ -279,7 +280,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
           const int k = ((__double2hiint(args.rowscale[m0 + c + wm]) >> 20) & 0x7FF) - 1023;
           double* o = reinterpret_cast<double*>(args.out) + (m0 + c + wm) + args.ld_out * (int64_t)nw;
 #pragma unroll 4
-          for (int n = wn; n < nn; n += 2) atomicAdd(o + args.ld_out * n, shift_exp(tp[wm * 33 + n], k));
+          for (int n = wn; n < nn; n += 2) {
+            const double v = shift_exp(tp[wm * 33 + n], k);
+            if (args.store) o[args.ld_out * n] = v;
+            else atomicAdd(o + args.ld_out * n, v);
+          }
         }
         __syncwarp();
       }
@@ -383,8 +388,22 @@ void launch_pair(cphf_ctx* c, const PairTerm& t, int kb_per_cta) {
   a.out = t.out;
   a.ld_out = t.ld_out;
   a.err = t.err;
+  a.x_row0 = (int)t.x_row0;
+  a.y_k0 = (int)t.y_k0;
+  a.store = t.store;
   const int64_t tiles = (int64_t)a.m_tiles * div_up(t.N, 2 * BM);
   const int64_t pairs = std::max(1, c->num_sms / 2);
+  if (kb_per_cta <= 0 && t.np == 1) {
+    // one long K (the XC batches): the range count with the shortest time, an epilogue as above
+    const int64_t r0 = C::EXACT ? div_up(a.total_kb, PAIR_EXACT_KB) : 1;
+    double best_t = 0.0;
+    for (int64_t r = r0; r <= r0 + 63 && r <= a.total_kb && !(t.store && r > 1); ++r) {
+      const int64_t kb = div_up(a.total_kb, r), used = div_up(a.total_kb, kb);
+      const double tt = (double)div_up(tiles * used, pairs) * ((double)kb + 8.0);
+      if (best_t == 0.0 || tt < best_t) best_t = tt, kb_per_cta = (int)kb;
+    }
+    if (kb_per_cta <= 0) kb_per_cta = a.total_kb;
+  }
   if (kb_per_cta <= 0) {
     // ranges of whole aux functions, long enough for the epilogue to be small beside them (each
     // tile's atomics cost about eight K blocks) and short enough to fill the SMs evenly
@@ -400,10 +419,11 @@ void launch_pair(cphf_ctx* c, const PairTerm& t, int kb_per_cta) {
   a.kb_per_cta = kb_per_cta;
   const int64_t ranges = div_up(a.total_kb, kb_per_cta);
   if (2 * tiles > INT32_MAX || ranges > 65535) throw Error(CPHF_ERR_ARG, "tensor-core K term: grid too large");
-  const CUtensorMap y0 = make_map(t.y.p[0], t.K, t.y.rows, t.y.depth, t.y.ld, C::ROW, BM, PR::BF16);
-  const CUtensorMap x0 = make_map(t.x.p[0], t.K, t.x.rows, t.x.depth, t.x.ld, C::ROW, a.NT / 2, PR::BF16);
-  const CUtensorMap y1 = C::EXACT ? y0 : make_map(t.y.p[1], t.K, t.y.rows, t.y.depth, t.y.ld, C::ROW, BM, PR::BF16);
-  const CUtensorMap x1 = C::EXACT ? x0 : make_map(t.x.p[1], t.K, t.x.rows, t.x.depth, t.x.ld, C::ROW, a.NT / 2, PR::BF16);
+  const int64_t xk = t.x.kext > 0 ? t.x.kext : t.K, yk = t.y.kext > 0 ? t.y.kext : t.K;
+  const CUtensorMap y0 = make_map(t.y.p[0], yk, t.y.rows, t.y.depth, t.y.ld, C::ROW, BM, PR::BF16);
+  const CUtensorMap x0 = make_map(t.x.p[0], xk, t.x.rows, t.x.depth, t.x.ld, C::ROW, a.NT / 2, PR::BF16);
+  const CUtensorMap y1 = C::EXACT ? y0 : make_map(t.y.p[1], yk, t.y.rows, t.y.depth, t.y.ld, C::ROW, BM, PR::BF16);
+  const CUtensorMap x1 = C::EXACT ? x0 : make_map(t.x.p[1], xk, t.x.rows, t.x.depth, t.x.ld, C::ROW, a.NT / 2, PR::BF16);
   const size_t smem = (size_t)std::max(a.stages * a.stage_bytes, C::EPI_BYTES) + 2048;
   tc_pair_kernel<PR><<<dim3((unsigned)(2 * tiles), (unsigned)ranges), PAIR_THREADS, smem, c->stream>>>(y0, y1, x0, x1, a);
   count_launch();
@@ -435,7 +455,8 @@ void pair_split2(cphf_ctx* c, const PairTerm& t) {
 
 void pair_exact(cphf_ctx* c, const PairTerm& t, int slices, int kb_per_cta) {
   if (t.M <= 0 || t.N <= 0 || t.K <= 0 || t.np <= 0) return;
-  if (kb_per_cta <= 0 || kb_per_cta > 96) throw Error(CPHF_ERR_ARG, "exact slices: K range out of bounds");
+  if (kb_per_cta > PAIR_EXACT_KB || (kb_per_cta <= 0 && t.np != 1) || (t.store && div_up(t.K, 32) > PAIR_EXACT_KB))
+    throw Error(CPHF_ERR_ARG, "exact slices: K range out of bounds");
   if (slices == 3) launch_pair<Exact6c3>(c, t, kb_per_cta);
   else if (slices == 4) launch_pair<Exact6c>(c, t, kb_per_cta);
   else launch_pair<Exact6>(c, t, kb_per_cta);

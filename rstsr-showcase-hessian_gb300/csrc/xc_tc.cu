@@ -23,6 +23,9 @@
 // is never written) and generates q's planes in one pass from column-maximum bounds; the exact
 // slices store ket, take rho1 from the SIMT path's kernel and slice q with its exact row maxima
 // (fixed-point slices are relative to the row scale, so a loose bound would cost accuracy).
+// All other contractions run on CTA pairs (tc_pair.cu), bound by the fill of shared memory and the
+// epilogue of their short K: a batch of 2500 points, 170 AOs, 2700 columns takes 79 / 56 us on
+// average for six / three slices and 18 us split (134, 106 and 33 on single CTAs).
 #include <algorithm>
 #include <type_traits>
 #include <vector>
@@ -102,30 +105,42 @@ __global__ void xc_v_kernel(const double* __restrict__ w, const double* __restri
 }
 
 // B-operand planes of GEMM 2: row n = (i, a) over the chunk's 8-padded point columns j,
-// q = v[p, a] aobra[p, i] (0 in the padding); one warp per row; column scale fac 2^(e_n - EOFF)
-template <class PR, class T>
-__global__ void q_planes_kernel(const T* __restrict__ v, const T* __restrict__ aobra, int64_t ngrids,
-                                const int* __restrict__ colmap, int64_t g0, int64_t npts, int64_t ncol, int64_t nocc,
-                                int64_t nrows, double fac, typename PR::Elem* __restrict__ dst, int64_t plane,
-                                double* __restrict__ colscale) {
-  const int lane = threadIdx.x & 31;
-  const int64_t w0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t n = w0; n < nrows; n += nw) {
-    const int64_t i = n % nocc, a = n / nocc;
-    const T* va = v + npts * a;
-    const T* ai = aobra + ngrids * i;
-    auto q = [&](int64_t j) -> T {
-      const int gp = colmap[j];
-      return gp >= 0 ? va[gp - g0] * ai[gp] : T(0);
-    };
-    unsigned long long m = 0;
-    for (int64_t j = lane; j < ncol; j += 32) m = max(m, abs_key(q(j)));
-    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-    const int e = key_exp(m, float_key<T>());
-    for (int64_t j = lane; j < ncol; j += 32) Put<PR>::put(q(j), e, dst + n * ncol + j, plane);
-    if (lane == 0) colscale[n] = fac * ldexp(1.0, e - PR::EOFF);
+// q = v[p, a] aobra[p, i] (0 in the padding), column scale fac 2^(e_n - EOFF): a warp per row and
+// segment of QSEG columns, first the row maxima, then the planes.  Bound by the FP64 products of both
+// passes and the operands' L2 reads; one warp per whole row was a chain of load latencies (nocc 30,
+// 90 right-hand sides, 75000 points, six slices: 3.9 -> 1.9 ms; four rows to a warp: 2.5).
+constexpr int64_t QSEG = 4096;
+template <class F>
+__device__ __forceinline__ void q_segment(const double* __restrict__ va, const double* __restrict__ ai,
+                                          const int* __restrict__ colmap, int64_t g0, int64_t j0, int64_t j1, F f) {
+#pragma unroll 4
+  for (int64_t j = j0 + (threadIdx.x & 31); j < j1; j += 32) {
+    const int gp = colmap[j];
+    f(j, gp >= 0 ? va[gp - g0] * ai[gp] : 0.0);
   }
+}
+__global__ void q_max_kernel(const double* __restrict__ v, const double* __restrict__ aobra, int64_t ngrids,
+                             const int* __restrict__ colmap, int64_t g0, int64_t npts, int64_t ncol, int64_t nocc,
+                             int64_t nrows, unsigned long long* __restrict__ mx) {
+  const int64_t n = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5), j0 = blockIdx.y * QSEG;
+  if (n >= nrows) return;
+  unsigned long long m = 0;
+  q_segment(v + npts * (n / nocc), aobra + ngrids * (n % nocc), colmap, g0, j0, min(ncol, j0 + QSEG),
+            [&](int64_t, double q) { m = max(m, abs_key(q)); });
+  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0 && m > 0) atomicMax(mx + n, m);
+}
+template <class PR>
+__global__ void q_planes_kernel(const double* __restrict__ v, const double* __restrict__ aobra, int64_t ngrids,
+                                const int* __restrict__ colmap, int64_t g0, int64_t npts, int64_t ncol, int64_t nocc,
+                                int64_t nrows, double fac, const unsigned long long* __restrict__ mx,
+                                typename PR::Elem* __restrict__ dst, int64_t plane, double* __restrict__ colscale) {
+  const int64_t n = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5), j0 = blockIdx.y * QSEG;
+  if (n >= nrows) return;
+  const int e = key_exp(mx[n], false);
+  q_segment(v + npts * (n / nocc), aobra + ngrids * (n % nocc), colmap, g0, j0, min(ncol, j0 + QSEG),
+            [&](int64_t j, double q) { Put<PR>::put(q, e, dst + n * ncol + j, plane); });
+  if (j0 == 0 && (threadIdx.x & 31) == 0) colscale[n] = fac * ldexp(1.0, e - PR::EOFF);
 }
 
 // mx[c] = max_r |x[r + ld c]| as ordered keys (r < nr, c = blockIdx.y); mx zeroed first
@@ -201,10 +216,10 @@ template <>
 struct XcOps<Split2> {
   using T = float;
   static constexpr int PROF = PROF_XC_TC32;
-  static void gemm(cphf_ctx* c, OzState& z, const PlaneMat& A, int64_t a_row0, const PlaneMat& B, int64_t b_k0,
+  static void gemm(cphf_ctx* c, const PlaneMat& A, int64_t a_row0, const PlaneMat& B, int64_t b_k0,
                    int64_t M, int64_t N, int64_t K, const double* rs, const double* cs, float* out, int64_t ld_out,
-                   int* err, int kb_per_cta, bool store) {
-    lp_gemm(c, z, A, a_row0, B, b_k0, M, N, K, rs, cs, out, ld_out, err, kb_per_cta, store);
+                   int* err, bool) {
+    lp_gemm(c, A, a_row0, B, b_k0, M, N, K, rs, cs, out, ld_out, err);
   }
   static void slice(cphf_ctx* c, const float* src, int64_t rows, int64_t K, int64_t rs, __half* dst, int64_t ld,
                     int* e) {
@@ -215,10 +230,10 @@ template <>
 struct XcOps<Exact6> {
   using T = double;
   static constexpr int PROF = PROF_XC_TC64;
-  static void gemm(cphf_ctx* c, OzState& z, const PlaneMat& A, int64_t a_row0, const PlaneMat& B, int64_t b_k0,
+  static void gemm(cphf_ctx* c, const PlaneMat& A, int64_t a_row0, const PlaneMat& B, int64_t b_k0,
                    int64_t M, int64_t N, int64_t K, const double* rs, const double* cs, double* out, int64_t ld_out,
-                   int* err, int kb_per_cta, bool store) {
-    oz_gemm(c, z, A, a_row0, B, b_k0, M, N, K, rs, cs, out, ld_out, err, kb_per_cta, store);
+                   int* err, bool store) {
+    oz_gemm(c, 6, A, a_row0, B, b_k0, M, N, K, rs, cs, out, ld_out, err, store);
   }
   static void slice(cphf_ctx* c, const double* src, int64_t rows, int64_t K, int64_t rs, __nv_bfloat16* dst,
                     int64_t ld, int* e) {
@@ -230,10 +245,10 @@ template <int NS>
 struct XcOps<ExactC<NS>> {  // correction precision: the leading NS planes of the exact slices
   using T = double;
   static constexpr int PROF = PROF_XC_TC64C;
-  static void gemm(cphf_ctx* c, OzState& z, const PlaneMat& A, int64_t a_row0, const PlaneMat& B, int64_t b_k0,
+  static void gemm(cphf_ctx* c, const PlaneMat& A, int64_t a_row0, const PlaneMat& B, int64_t b_k0,
                    int64_t M, int64_t N, int64_t K, const double* rs, const double* cs, double* out, int64_t ld_out,
-                   int* err, int kb_per_cta, bool store) {
-    oz_gemm_corr(c, z, NS, A, a_row0, B, b_k0, M, N, K, rs, cs, out, ld_out, err, kb_per_cta, store);
+                   int* err, bool store) {
+    oz_gemm(c, NS, A, a_row0, B, b_k0, M, N, K, rs, cs, out, ld_out, err, store);
   }
   static void slice(cphf_ctx* c, const double* src, int64_t rows, int64_t K, int64_t rs, __nv_bfloat16* dst,
                     int64_t ld, int* e) {
@@ -329,7 +344,7 @@ void xc_tc(cphf_ctx* c, XcTcState& X, OzState& z, const typename XcOps<PR>::T* p
   X.qscale.ensure((size_t)nmax * 8, c->counter());
   int64_t omax = 1;
   for (int s = 0; s < ns; ++s) omax = std::max<int64_t>(omax, c->spin[s].nocc);
-  X.qmax.ensure((size_t)(nb + omax) * 8, c->counter());
+  X.qmax.ensure((size_t)std::max<int64_t>(nb + omax, nmax) * 8, c->counter());
   const double fac = ns == 1 ? 4.0 : 2.0;  // hess_rks.rs:603, hess_uks.rs:438-439
   double nnz = 0.0;
   for (const XcBatch& x : c->xc_batches) nnz += (double)x.npts * (double)x.nwin;
@@ -370,7 +385,7 @@ void xc_tc(cphf_ctx* c, XcTcState& X, OzState& z, const typename XcOps<PR>::T* p
           if (x.npts == 0 || x.nwin == 0) continue;
           const RhoEpilogue re{rho_s + (x.g0 - g0), aobra[s] + x.g0, npts, ngrids, no};
           lp_gemm_rho(c, z, phiB, x.g0, B, x.lo8, x.npts, N, x.kw, X.phiB_scale.as<double>() + x.g0,
-                      X.bscale[s].as<double>(), re, err, (int)div_up(x.kw, 32));
+                      X.bscale[s].as<double>(), re, err);
         }
       } else {
         // GEMM 1 per batch: ket[p - g0, :] = phi[p, win] bra[win, :] (one K range: stored)
@@ -381,8 +396,8 @@ void xc_tc(cphf_ctx* c, XcTcState& X, OzState& z, const typename XcOps<PR>::T* p
             CPHF_CUDA(cudaMemset2DAsync(ket[s] + (x.g0 - g0), npts * sizeof(T), 0, x.npts * sizeof(T), N, st));
             continue;
           }
-          XcOps<PR>::gemm(c, z, phiB, x.g0, B, x.lo8, x.npts, N, x.kw, X.phiB_scale.as<double>() + x.g0,
-                          X.bscale[s].as<double>(), ket[s] + (x.g0 - g0), npts, err, (int)div_up(x.kw, 32), true);
+          XcOps<PR>::gemm(c, phiB, x.g0, B, x.lo8, x.npts, N, x.kw, X.phiB_scale.as<double>() + x.g0,
+                          X.bscale[s].as<double>(), ket[s] + (x.g0 - g0), npts, err, true);
         }
         launch_xc_rho<T>(aobra[s] + g0, ngrids, ket[s], npts, no, nb, rho_s, npts, st);
       }
@@ -407,21 +422,22 @@ void xc_tc(cphf_ctx* c, XcTcState& X, OzState& z, const typename XcOps<PR>::T* p
             X.qpl.as<__half>(), N * ncol);
         count_launch(4);
       } else {
-        q_planes_kernel<PR, T><<<blocks_for(N * 32), 256, 0, st>>>(X.v.as<T>(), aobra[s], ngrids,
-                                                                   X.colmap.as<int>() + gofs0, g0, npts, ncol, no, N,
-                                                                   fac, X.qpl.as<E>(), N * ncol, X.qscale.as<double>());
-        count_launch();
+        unsigned long long* mx = X.qmax.as<unsigned long long>();
+        CPHF_CUDA(cudaMemsetAsync(mx, 0, (size_t)N * 8, st));
+        const dim3 grid((unsigned)div_up(N, 8), (unsigned)div_up(ncol, QSEG));
+        q_max_kernel<<<grid, 256, 0, st>>>(X.v.as<T>(), aobra[s], ngrids, X.colmap.as<int>() + gofs0, g0, npts, ncol, no,
+                                           N, mx);
+        q_planes_kernel<PR><<<grid, 256, 0, st>>>(X.v.as<T>(), aobra[s], ngrids, X.colmap.as<int>() + gofs0, g0, npts,
+                                                  ncol, no, N, fac, mx, X.qpl.as<E>(), N * ncol, X.qscale.as<double>());
+        count_launch(2);
       }
       // GEMM 2 per batch: out[win, :] += fac phi[batch, win]^T q[batch, :]
       const PlaneMat Q{X.qpl.p, N, ncol, ncol};
-      const int64_t n_tiles = div_up(N, 128);
       for (int64_t b = ch.b0; b < ch.b1; ++b) {
         const XcTcBatch& x = X.hb[b];
         if (x.nwin == 0 || x.npts == 0) continue;
-        const int64_t nkb = div_up(x.npts, 32), tiles = div_up(x.nwin, 128) * n_tiles;
-        const int64_t ranges = std::min<int64_t>(nkb, div_up(2 * (int64_t)c->num_sms, tiles));
-        XcOps<PR>::gemm(c, z, phiT, x.rT, Q, x.gofs - gofs0, x.nwin, N, x.npts, X.phiT_scale.as<double>() + x.rT,
-                        X.qscale.as<double>(), out[s] + x.lo, nao, err, (int)div_up(nkb, ranges), false);
+        XcOps<PR>::gemm(c, phiT, x.rT, Q, x.gofs - gofs0, x.nwin, N, x.npts, X.phiT_scale.as<double>() + x.rT,
+                        X.qscale.as<double>(), out[s] + x.lo, nao, err, false);
       }
     }
   }

@@ -98,3 +98,25 @@ def test_gradient_components_in_one_product(nao, nocc, natm, points, window, nb,
         got.append(_run(ctx, s, bra))
     for a, b in zip(*got):
         assert rel_err(a, b) < 1e-12
+
+
+@pytest.mark.parametrize("nao,nocc,natm,points,window,nb", LDA + [(300, (6,), 2, (1500, 1801), 290, 4)])
+def test_tensor_core_xc_at_tile_edges(nao, nocc, natm, points, window, nb):
+    """Mixed-precision XC on CTA pairs: split FP16 to 1e-5 of the operator, the exact-slice residual to
+    1e-9 max(1, max |x|) (the operators' bars)."""
+    s = _system(nao, nocc, natm, points, window)
+    one = lambda v: v if s.nspin == 2 else v[0]
+    c64, lp = _context(s), _context(s, precision="mixed")
+    rng = np.random.default_rng(5)
+    mo1 = [rng.standard_normal((nao, n, nb)) for n in nocc]
+    a, b = lp.response_dimless_cphf_lowp(one(mo1)), c64.response_dimless_cphf(one(mo1))
+    for u, v in zip(a if s.nspin == 2 else [a], b if s.nspin == 2 else [b]):
+        assert rel_err(u, v) < 1e-5
+    mx = _context(s, precision="mixed", residual_dfloat=2, max_refine=1, residual_tol=1.0, verify_residual=0)
+    x = mx.solve_dimless_cphf(one(s.rhs))
+    xs = x if s.nspin == 2 else [x]
+    y = c64.response_dimless_cphf(x)
+    r = np.concatenate([(p - q - w).reshape(-1, 3 * natm, order="F")
+                        for p, q, w in zip(s.rhs, xs, y if s.nspin == 2 else [y])])
+    ref = float(np.linalg.norm(r, axis=0).max())
+    assert abs(mx.last_stats["residual_max"] - ref) < 1e-9 * max(1.0, max(np.abs(q).max() for q in xs))
