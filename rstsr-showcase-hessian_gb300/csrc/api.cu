@@ -16,8 +16,15 @@ namespace {
 
 struct CounterScope {
   int64_t* prev;
-  explicit CounterScope(cphf_ctx* c) : prev(g_launch_counter) { g_launch_counter = &c->launches; }
-  ~CounterScope() { g_launch_counter = prev; }
+  std::unique_ptr<LowpState>* parked;
+  explicit CounterScope(cphf_ctx* c) : prev(g_launch_counter), parked(g_parked) {
+    g_launch_counter = &c->launches;
+    g_parked = &c->lowp_parked;
+  }
+  ~CounterScope() {
+    g_launch_counter = prev;
+    g_parked = parked;
+  }
 };
 
 // Reads (and clears) the error flag of the fixed-point GEMMs launched during this call.
@@ -300,7 +307,8 @@ static void install_cderi(cphf_ctx* c, int64_t nao, int64_t naux, double scale_j
   launch_unpack_cderi(c->cderi_tp.as<double>(), nao, naux, c->Bd.as<double>(), c->stream);
   c->has_rijk = true;
   c->prepared = false;
-  lowp_release(c);
+  if (c->lowp && (c->lowp->shape[0] != nao || c->lowp->shape[1] != naux)) lowp_release(c);
+  else lowp_park(c);
   CPHF_CUDA(cudaStreamSynchronize(c->stream));
 }
 
@@ -530,8 +538,12 @@ cphf_status cphf_prepare(cphf_ctx* c, int32_t nspin, const double* const* mo_coe
     c->nspin = nspin;
     if (c->has_rijk) rijk_prepare(c);
     if (c->has_xc) xc_prepare(c);
-    lowp_release(c);
-    if (c->cfg.precision == CPHF_PRECISION_MIXED) lowp_prepare(c);
+    if (c->cfg.precision == CPHF_PRECISION_MIXED) {
+      lowp_park(c);
+      lowp_prepare(c);
+    } else {
+      lowp_release(c);
+    }
     CPHF_CUDA(cudaStreamSynchronize(c->stream));
     c->prepared = true;
   });

@@ -47,6 +47,10 @@ extern std::atomic<int64_t> g_state_generation;
 inline void bump_generation() { g_state_generation.fetch_add(1, std::memory_order_relaxed); }
 inline int64_t state_generation() { return g_state_generation.load(std::memory_order_relaxed); }
 
+// Frees the memory that the calling thread's context has set aside for its next preparation
+// (lowp_park); false when there is none.
+bool reclaim_parked();
+
 // Owning device allocation; byte size tracked for cphf_ctx_device_bytes.
 struct DevBuf {
   void* p = nullptr;
@@ -71,7 +75,9 @@ struct DevBuf {
     release();
     counter = cnt;
     if (n == 0) return;
-    CPHF_CUDA(cudaMalloc(&p, n));
+    cudaError_t e = cudaMalloc(&p, n);
+    if (e == cudaErrorMemoryAllocation && reclaim_parked()) e = cudaMalloc(&p, n);
+    check_cuda(e, "cudaMalloc(&p, n)");
     bump_generation();
     bytes = n;
     if (counter) *counter += (int64_t)n;

@@ -80,6 +80,7 @@ struct LowpState {
   double sA = 1.0;             // power-of-two scale of the FP16 cderi planes
   int64_t budget = int64_t(1) << 30;  // bytes per chunk of T / W intermediates (set at preparation)
   bool use_tc = true;
+  std::vector<int64_t> shape;  // the preparation's sizes
   // captured operator applications (cfg.cuda_graphs)
   std::vector<OpGraph> graphs;
   DevBuf g_x, g_y;
@@ -241,7 +242,7 @@ struct cphf_ctx {
   cphf::DevBuf k_xs, k_ax, k_h, k_g, k_b, k_xacc, k_x1, k_axt, k_coef, k_ip, k_keep, k_part, k_idx,
       k_hw, k_info, k_r, k_norm, k_finite, k_pre;
 
-  std::unique_ptr<cphf::LowpState> lowp;
+  std::unique_ptr<cphf::LowpState> lowp, lowp_parked;
   std::unique_ptr<cphf::MlpState> mlp;
   cphf::Profiler prof;
   bool f64_emulate = false;  // route the FP64 GEMMs through the double-float kernel
@@ -322,7 +323,12 @@ double fp64_residual(cphf_ctx* c, const double* b, const double* x, int64_t nset
 
 // mixed-precision support
 void lowp_prepare(cphf_ctx* c);
-void lowp_release(cphf_ctx* c);
+void lowp_release(cphf_ctx* c);  // frees the split-precision state
+// Invalidates the split-precision state and sets its buffers aside for the next preparation, which
+// takes them over if it has the same sizes and frees them otherwise (as does any allocation of the
+// context that finds no memory).
+void lowp_park(cphf_ctx* c);
+extern thread_local std::unique_ptr<LowpState>* g_parked;  // of the context whose call runs
 
 // Scope in which the FP64 operator (response_mo_fp64) runs in the FP64-accurate arithmetic of
 // the mixed context: mode 0 native FP64, 1 double-float GEMMs, 2 double-float plus the RI-K
