@@ -22,6 +22,7 @@
 #include <mutex>
 
 #include "kernels.cuh"
+#include "slices.cuh"
 #include "tc_gemm.cuh"
 #include "tc_pair.cuh"
 #include "tc_ptx.cuh"
@@ -255,36 +256,50 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
 }
 
 // ---- FP16 plane splitting --------------------------------------------------------------
-__device__ __forceinline__ void split_f16(double x, double s, __half* hi, __half* lo) {
-  const double xs = x * s;
-  const __half h = __double2half(xs);
-  *hi = h;
-  *lo = __double2half(xs - (double)__half2float(h));
+// FP16 hi / lo of x 2^k (finite, |x 2^k| < 2^15) without the FP64 pipe: x's leading 24 bits and its
+// other 29 as an FP32 pair, hi from the first, lo from the remainder (|x 2^k - hi - lo| <= 2^-23.99
+// |x 2^k| or half the least FP16 subnormal).
+__device__ __forceinline__ void split_f16(double x, int k, __half& h, __half& l) {
+  const unsigned w1 = (unsigned)__double2hiint(x), w0 = (unsigned)__double2loint(x);
+  const int e = (int)((w1 >> 20) & 0x7FF) - 1023 + k;
+  const bool tiny = e < -64;  // far below FP16's range
+  const unsigned f = (w1 & 0x80000000u) | ((unsigned)(e + 127) << 23) | ((w1 & 0xFFFFFu) << 3) | (w0 >> 29);
+  const float x1 = tiny ? 0.f : __uint_as_float(f);
+  const float u = tiny ? 0.f : __uint_as_float((w1 & 0x80000000u) | ((unsigned)(e + 127 - 52) << 23));  // +-2^(e - 52)
+  h = __float2half_rn(x1);
+  l = __float2half_rn(fmaf((float)(w0 & 0x1FFFFFFFu), u, x1 - __half2float(h)));
 }
 
-// dense symmetric cderi (FP64 [P][mu][nu]) -> planes [P][mu][ldk] (nu contiguous)
-__global__ void split_cderi_kernel(const double* __restrict__ Bd, int64_t nao, int64_t naux, int64_t ldk, double s,
+// dense symmetric cderi (FP64 [P][mu][nu]) -> planes [P][mu][ldk] (nu contiguous) of 2^k B: a warp
+// per row, two nu to a lane.  Bound by HBM (nao 400, naux 1333: 2.0 -> 0.43 ms; two FP64 products and
+// three FP64 conversions an element bounded it before)
+__global__ void split_cderi_kernel(const double* __restrict__ Bd, int64_t nao, int64_t rows, int64_t ldk, int k,
                                    __half* __restrict__ hi, __half* __restrict__ lo) {
-  const int64_t total = naux * nao * ldk;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t nu = t % ldk;
-    const int64_t r = t / ldk;  // P * nao + mu
-    if (nu < nao) {
-      const int64_t P = r / nao, mu = r % nao;
-      split_f16(Bd[nu + nao * mu + nao * nao * P], s, hi + t, lo + t);  // (symmetric: read along nu)
-    } else {
-      hi[t] = __float2half(0.f);
-      lo[t] = __float2half(0.f);
+  const int lane = threadIdx.x & 31;
+  const int64_t w0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t r = w0; r < rows; r += nw) {  // P * nao + mu (symmetric: read along nu)
+    const double* src = Bd + r * nao;
+#pragma unroll 4
+    for (int nu = 2 * lane; nu < (int)ldk; nu += 64) {  // ldk is even
+      __half h0, l0, h1, l1;
+      split_f16(nu < nao ? src[nu] : 0.0, k, h0, l0);
+      split_f16(nu + 1 < nao ? src[nu + 1] : 0.0, k, h1, l1);
+      *reinterpret_cast<__half2*>(hi + r * ldk + nu) = __halves2half2(h0, h1);
+      *reinterpret_cast<__half2*>(lo + r * ldk + nu) = __halves2half2(l0, l1);
     }
   }
 }
 
-__global__ void absmax_f64_kernel(const double* __restrict__ x, int64_t n, unsigned* out) {
-  float m = 0.f;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x)
-    m = fmaxf(m, (float)fabs(x[t]));
-  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(out, __float_as_uint(m));
+// max |x| as an ordered key (integer comparisons: an FP64 one occupies the FP64 pipe like a
+// product; 213 M elements 4.8 -> 0.26 ms)
+__global__ void absmax_f64_kernel(const double* __restrict__ x, int64_t n, unsigned long long* out) {
+  unsigned long long m = 0;
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+#pragma unroll 8
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n; t += step) m = max(m, abs_key(x[t]));
+  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0) atomicMax(out, m);
 }
 
 // power-of-two scale bringing max |x| to at most 2^14; scale[0] = s, scale[1] = alpha / (sA * s)
@@ -367,23 +382,23 @@ void tc_prepare_cderi(cphf_ctx* c, DevBuf& hi, DevBuf& lo, int64_t& ldk) {
   ldk = plane_ld(nao);
   // power-of-two scale from max |B|
   DevBuf mx;
-  mx.ensure(sizeof(unsigned), nullptr);
-  CPHF_CUDA(cudaMemsetAsync(mx.p, 0, sizeof(unsigned), c->stream));
-  absmax_f64_kernel<<<grid_for(nao * nao * naux), 256, 0, c->stream>>>(c->Bd.as<double>(), nao * nao * naux, mx.as<unsigned>());
-  unsigned bits = 0;
-  CPHF_CUDA(cudaMemcpyAsync(&bits, mx.p, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
+  mx.ensure(sizeof(unsigned long long), nullptr);
+  CPHF_CUDA(cudaMemsetAsync(mx.p, 0, sizeof(unsigned long long), c->stream));
+  absmax_f64_kernel<<<8 * c->num_sms, 256, 0, c->stream>>>(c->Bd.as<double>(), nao * nao * naux,
+                                                           mx.as<unsigned long long>());
+  double m = 0.0;
+  CPHF_CUDA(cudaMemcpyAsync(&m, mx.p, sizeof(m), cudaMemcpyDeviceToHost, c->stream));
   CPHF_CUDA(cudaStreamSynchronize(c->stream));
-  float m;
-  std::memcpy(&m, &bits, 4);
   int e = 0;
-  std::frexp((double)m, &e);
-  const double sA = (m > 0.f) ? std::ldexp(1.0, 14 - e) : 1.0;
+  std::frexp((double)(float)m, &e);
+  const int k = (float)m > 0.f ? 14 - e : 0;
+  const double sA = std::ldexp(1.0, k);
   c->lowp->sA = sA;
   const size_t bytes = (size_t)naux * nao * ldk * 2;
   hi.ensure(bytes, c->counter());
   lo.ensure(bytes, c->counter());
-  split_cderi_kernel<<<grid_for(naux * nao * ldk), 256, 0, c->stream>>>(c->Bd.as<double>(), nao, naux, ldk, sA,
-                                                                       hi.as<__half>(), lo.as<__half>());
+  split_cderi_kernel<<<16 * c->num_sms, 256, 0, c->stream>>>(c->Bd.as<double>(), nao, naux * nao, ldk, k,
+                                                             hi.as<__half>(), lo.as<__half>());
   count_launch(2);
   CPHF_CUDA(cudaGetLastError());
 }

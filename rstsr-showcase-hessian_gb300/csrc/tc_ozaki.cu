@@ -884,15 +884,27 @@ __global__ void exp_scale_kernel(const unsigned long long* __restrict__ mx, int6
   scale[i] = mult * ldexp(1.0, e - eoff);
 }
 
-// cderi slices [t][P][mu][ldk] of B_P[mu, nu] 2^-e_mu (B_P symmetric: read Bd[nu + nao mu + nao^2 P])
+// cderi slices [t][P][mu][ldk] of B_P[mu, nu] 2^-e_mu (B_P symmetric: read Bd[nu + nao mu + nao^2 P]),
+// a warp per row.  Bound by the digits' integer instructions and HBM (nao 400, naux 1333: 1.65 -> 1.1 ms;
+// an element to a thread spent half its instructions on 64-bit divisions)
 __global__ void slice_cderi_kernel(const double* __restrict__ Bd, int64_t nao, int64_t naux, int64_t ldk,
                                    const int* __restrict__ e_row, __nv_bfloat16* __restrict__ out) {
-  const int64_t total = naux * nao * nao;
-  const int64_t plane = naux * nao * ldk;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t nu = t % nao;
-    const int64_t r = t / nao;  // P * nao + mu
-    slice6(Bd[t], e_row[r % nao], out + nu + ldk * r, plane);
+  const int64_t rows = naux * nao, plane = rows * ldk;
+  const int lane = threadIdx.x & 31;
+  const int64_t w0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t r = w0; r < rows; r += nw) {  // P * nao + mu
+    const double* src = Bd + r * nao;
+    const int e = e_row[r % nao];
+#pragma unroll 2
+    for (int nu = 2 * lane; nu < (int)nao; nu += 64) {  // two nu to a lane (the odd row's last: padding, ldk is even)
+      __nv_bfloat16 d0[S], d1[S];
+      slice6(src[nu], e, d0, 1);
+      slice6(nu + 1 < nao ? src[nu + 1] : 0.0, e, d1, 1);
+#pragma unroll
+      for (int t = 0; t < S; ++t)
+        *reinterpret_cast<__nv_bfloat162*>(out + t * plane + ldk * r + nu) = __nv_bfloat162(d0[t], d1[t]);
+    }
   }
 }
 
@@ -1294,7 +1306,7 @@ void oz_prepare_cderi(cphf_ctx* c, OzState& z) {
                                                               z.mx.as<unsigned long long>());
   exp_scale_kernel<<<grid_for(nao), 256, 0, c->stream>>>(z.mx.as<unsigned long long>(), nao, 1.0, false, 0,
                                                          z.e_row.as<int>(), z.rowscale.as<double>());
-  slice_cderi_kernel<<<grid_for(naux * nao * nao), 256, 0, c->stream>>>(c->Bd.as<double>(), nao, naux, z.ldk,
+  slice_cderi_kernel<<<grid_warps(naux * nao, c->num_sms), 256, 0, c->stream>>>(c->Bd.as<double>(), nao, naux, z.ldk,
                                                                         z.e_row.as<int>(), z.A.as<__nv_bfloat16>());
   count_launch(3);
   CPHF_CUDA(cudaGetLastError());
