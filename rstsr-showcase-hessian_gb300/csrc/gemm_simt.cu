@@ -22,8 +22,7 @@ struct CfgF64S {
 struct CfgF32 {
   static constexpr int BM = 128, BN = 128, BK = 16, TM = 8, TN = 8;
 };
-// FP32 for narrow outputs (N <= 64, e.g. the occupied index of the K-term intermediates):
-// 256x64 tile, 8x8 per thread, 256 threads.
+// FP32 where 64-wide columns pad less: 256x64 tile, 8x8 per thread, 256 threads.
 struct CfgF32Tall {
   static constexpr int BM = 256, BN = 64, BK = 16, TM = 8, TN = 8;
 };
@@ -42,11 +41,19 @@ __global__ void __launch_bounds__(256) gemm_kernel(GemmDesc d, int ksplit, int64
   constexpr int BM = Cfg::BM, BN = Cfg::BN, BK = Cfg::BK, TM = Cfg::TM, TN = Cfg::TN;
   constexpr int NTX = BN / TN, NTY = BM / TM, NT = NTX * NTY;
   constexpr int LA = BM * BK / NT, LB = BK * BN / NT;
-  __shared__ T As[2][BK][BM];
-  __shared__ T Bs[2][BK][BN];
+  // rows 16 bytes longer than the tile: operands with k contiguous are stored down a column, which
+  // would meet one bank 16 times over
+  constexpr int PAD = 16 / sizeof(T);
+  __shared__ __align__(16) T As[2][BK][BM + PAD];
+  __shared__ __align__(16) T Bs[2][BK][BN + PAD];
 
   const int tid = threadIdx.x;
-  const int tx = tid % NTX, ty = tid / NTX;
+  // tile row / column of the thread's i-th: FP32 in groups of four, read as 16 bytes, and lanes along
+  // the rows, whose results are mostly contiguous
+  constexpr bool VEC = std::is_same<T, float>::value;
+  const int tx = VEC ? tid / NTY : tid % NTX, ty = VEC ? tid % NTY : tid / NTX;
+  auto row = [&](int i) { return VEC ? (i >> 2) * (4 * NTY) + ty * 4 + (i & 3) : ty + i * NTY; };
+  auto col = [&](int j) { return VEC ? (j >> 2) * (4 * NTX) + tx * 4 + (j & 3) : tx + j * NTX; };
   const int64_t m0 = (int64_t)blockIdx.x * BM;
   const int64_t n0 = (int64_t)blockIdx.y * BN;
   const int64_t z = blockIdx.z;
@@ -147,10 +154,17 @@ __global__ void __launch_bounds__(256) gemm_kernel(GemmDesc d, int ksplit, int64
 #pragma unroll
       for (int kk = 0; kk < BK; ++kk) {
         T a[TM], b[TN];
+        if constexpr (VEC) {
 #pragma unroll
-        for (int i = 0; i < TM; ++i) a[i] = As[buf][kk][ty + i * NTY];
+          for (int i = 0; i < TM; i += 4) *reinterpret_cast<float4*>(a + i) = *reinterpret_cast<const float4*>(&As[buf][kk][row(i)]);
 #pragma unroll
-        for (int j = 0; j < TN; ++j) b[j] = Bs[buf][kk][tx + j * NTX];
+          for (int j = 0; j < TN; j += 4) *reinterpret_cast<float4*>(b + j) = *reinterpret_cast<const float4*>(&Bs[buf][kk][col(j)]);
+        } else {
+#pragma unroll
+          for (int i = 0; i < TM; ++i) a[i] = As[buf][kk][row(i)];
+#pragma unroll
+          for (int j = 0; j < TN; ++j) b[j] = Bs[buf][kk][col(j)];
+        }
 #pragma unroll
         for (int i = 0; i < TM; ++i)
 #pragma unroll
@@ -166,14 +180,37 @@ __global__ void __launch_bounds__(256) gemm_kernel(GemmDesc d, int ksplit, int64
 
   if (ksplit == 1) {
     const T alpha = (T)d.alpha, beta = (T)d.beta;
+    if constexpr (VEC && std::is_same<TC, float>::value) {
+      // whole groups of four contiguous results
+      if (d.c_m == 1 && d.m_div <= 0 && m0 + BM <= d.M && d.c_n % 4 == 0 && (d.n_div <= 0 || d.c_n2 % 4 == 0) &&
+          (reinterpret_cast<uintptr_t>(C) & 15) == 0) {
+#pragma unroll
+        for (int j = 0; j < TN; ++j) {
+          const int64_t gn = n0 + col(j);
+          if (gn >= d.N) continue;
+          float* p0 = C + m0 + off2(gn, d.n_div, d.c_n, d.c_n2);
+#pragma unroll
+          for (int i = 0; i < TM; i += 4) {
+            float4* p = reinterpret_cast<float4*>(p0 + row(i));
+            float4 v = make_float4(alpha * acc[i][j], alpha * acc[i + 1][j], alpha * acc[i + 2][j], alpha * acc[i + 3][j]);
+            if (beta != 0.f) {
+              const float4 o = *p;
+              v = make_float4(madd(beta, o.x, v.x), madd(beta, o.y, v.y), madd(beta, o.z, v.z), madd(beta, o.w, v.w));
+            }
+            *p = v;
+          }
+        }
+        return;
+      }
+    }
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
-      const int64_t gm = m0 + ty + i * NTY;
+      const int64_t gm = m0 + row(i);
       if (gm >= d.M) continue;
       const int64_t cm = off2(gm, d.m_div, d.c_m, d.c_m2);
 #pragma unroll
       for (int j = 0; j < TN; ++j) {
-        const int64_t gn = n0 + tx + j * NTX;
+        const int64_t gn = n0 + col(j);
         if (gn >= d.N) continue;
         TC* p = C + cm + off2(gn, d.n_div, d.c_n, d.c_n2);
         T v = alpha * acc[i][j];
@@ -182,16 +219,16 @@ __global__ void __launch_bounds__(256) gemm_kernel(GemmDesc d, int ksplit, int64
       }
     }
   } else {
-    // split-K partial sums, [split][batch][M][N] row-major in the workspace
+    // split-K partial sums in the workspace, [split][batch][M][N] (FP32: [N][M], the lanes' order)
     T* W = ws + ((int64_t)split * (d.batch1 * d.batch2) + bidx) * d.M * d.N;
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
-      const int64_t gm = m0 + ty + i * NTY;
+      const int64_t gm = m0 + row(i);
       if (gm >= d.M) continue;
 #pragma unroll
       for (int j = 0; j < TN; ++j) {
-        const int64_t gn = n0 + tx + j * NTX;
-        if (gn < d.N) W[gm * d.N + gn] = acc[i][j];
+        const int64_t gn = n0 + col(j);
+        if (gn < d.N) W[VEC ? gn * d.M + gm : gm * d.N + gn] = acc[i][j];
       }
     }
   }
@@ -206,8 +243,9 @@ __global__ void splitk_reduce_kernel(GemmDesc d, int ksplit, const T* __restrict
   const T alpha = (T)d.alpha, beta = (T)d.beta;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
        e += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t n = e % d.N;
-    const int64_t m = (e / d.N) % d.M;
+    constexpr bool MFAST = std::is_same<T, float>::value;  // gemm_kernel's order of the partial sums
+    const int64_t n = MFAST ? (e / d.M) % d.N : e % d.N;
+    const int64_t m = MFAST ? e % d.M : (e / d.N) % d.M;
     const int64_t bidx = e / (d.N * d.M);
     const int64_t b1 = bidx % d.batch1, b2 = bidx / d.batch1;
     T s = (T)0;
@@ -318,15 +356,41 @@ cudaError_t run_f64(const GemmDesc& d, cudaStream_t stream, void* workspace, siz
   return run<double, CfgF64, double, double, double>(d, stream, workspace, ws_bytes, num_sms, only_if, f.split);
 }
 
-// narrow-output FP32 shapes take the 256 x 64 tile
-bool use_tall(const GemmDesc& d) { return d.N <= 64 && d.M >= 512; }
+// Tile and K split of an FP32 GEMM by the time they take (us): waves of blocks, one to an SM, at
+// ~0.11 us per k of a 128 x 128 or 256 x 64 tile (~65 % of the FP32 rate), the reduction of the partial
+// sums ~3 us and its traffic.  2000 x 180 x 36000 and its like: 128 x 128 tiles in 10 splits (three waves, 30 % of
+// the columns padding) 1.7 ms, 256 x 64 tiles in 19 splits @D@ ms.
+struct F32Choice {
+  bool tall;
+  int split;
+  double us;
+};
+template <typename Cfg>
+void f32_candidates(const GemmDesc& d, int num_sms, bool tall, F32Choice& best) {
+  const int64_t nb = d.batch1 * d.batch2;
+  const int64_t tiles = div_up(d.M, Cfg::BM) * div_up(d.N, Cfg::BN) * nb;
+  for (int s = 1; s <= 64; ++s) {
+    if (s > 1 && ((int64_t)s * 4 * Cfg::BK > d.K || (double)s * d.M * d.N * nb * 4 > 512e6 || tiles >= 8 * (int64_t)num_sms))
+      break;
+    const double kc = (double)div_up(div_up(d.K, s), Cfg::BK) * Cfg::BK;
+    const double t = (double)div_up(tiles * s, num_sms) * (kc * 0.11 + 3.0) +
+                     (s > 1 ? 3.0 + (double)(s + 2) * d.M * d.N * nb * 4 / 4.5e6 : 0.0);
+    if (best.us < 0.0 || t < best.us) best = F32Choice{tall, s, t};
+  }
+}
+F32Choice f32_choice(const GemmDesc& d, int num_sms) {
+  F32Choice best{false, 1, -1.0};
+  f32_candidates<CfgF32>(d, num_sms, false, best);
+  f32_candidates<CfgF32Tall>(d, num_sms, true, best);
+  return best;
+}
 
 }  // namespace
 
 size_t gemm_workspace_bytes(const GemmDesc& d, size_t elem_bytes, int num_sms) {
   int s;
   if (elem_bytes == 8) s = std::max(choose_split<CfgF64>(d, num_sms), f64_choice(d, num_sms).split);
-  else s = use_tall(d) ? choose_split<CfgF32Tall>(d, num_sms) : choose_split<CfgF32>(d, num_sms);
+  else s = f32_choice(d, num_sms).split;
   if (s <= 1) return 0;
   return (size_t)s * d.batch1 * d.batch2 * d.M * d.N * elem_bytes;
 }
@@ -348,8 +412,9 @@ cudaError_t gemm(const GemmDesc& d, cudaStream_t stream, void* workspace, size_t
   } else if constexpr (sizeof(T) == 8) {
     return run<T, CfgF64, TA, TB, TC>(d, stream, workspace, ws_bytes, num_sms);
   } else {
-    if (use_tall(d)) return run<T, CfgF32Tall, TA, TB, TC>(d, stream, workspace, ws_bytes, num_sms);
-    return run<T, CfgF32, TA, TB, TC>(d, stream, workspace, ws_bytes, num_sms);
+    const F32Choice f = f32_choice(d, num_sms);
+    if (f.tall) return run<T, CfgF32Tall, TA, TB, TC>(d, stream, workspace, ws_bytes, num_sms, nullptr, f.split);
+    return run<T, CfgF32, TA, TB, TC>(d, stream, workspace, ws_bytes, num_sms, nullptr, f.split);
   }
 }
 
