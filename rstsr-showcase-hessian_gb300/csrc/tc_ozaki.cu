@@ -588,23 +588,26 @@ __global__ void __launch_bounds__(320, PR::NACC == 4 ? 1 : 2)
 // tile, range of aux functions).  A row tile is 128 consecutive nu of one perturbation
 // a (the last tile of each a is partial), so that T_P's tile is one box of the planes' layout.
 // The A tile -- every K block of the bra rows, both planes -- is loaded once and stays in
-// shared memory; O_P's tile (all i of a column, BN = 32, 64 or 128 >= nocc rows) streams through a
-// 4-stage ring.  Double-buffered TMEM accumulators (2 x BN columns) let the epilogue of aux
-// function p overlap the MMAs of p + 1.  Each epilogue warp (32 nu x BN / 2 i) writes the FP16
-// hi / lo planes of T * tscale of its part into its own shared-memory tile [BN / 2 i][32 nu] and
-// stores them with TMA (cp.async.bulk.tensor, clipped at nu = nao): the global writes are bulk
-// transfers off the warps' issue path, and a warp waits only for its own previous stores to
-// have left shared memory, so the stores of aux function p drain while p + 1 is computed.
+// shared memory; the O_P tiles (all i of a column, BN = 32, 64 or 128 >= nocc rows each) of
+// PG = 128 / BN aux functions stream through a ring as one operand of 128 columns.  Double-buffered
+// TMEM accumulators (2 x 128 columns) let the epilogue of one group overlap the MMAs of the next.
+// Each epilogue warp (32 nu x BN / 2 i) writes the FP16 hi / lo planes of T * tscale of its part
+// into its own shared-memory tile [BN / 2 i][32 nu] and stores them with TMA
+// (cp.async.bulk.tensor, clipped at nu = nao): the global writes are bulk transfers off the warps'
+// issue path, and a warp waits only for its own previous stores to have left shared memory.
 // Warp 0: TMA loads, warp 1: MMA issuer and TMEM owner, warps 2-9: epilogue.
-// The epilogue's serial chain per aux function (load, convert, stage, store) bounds it, so the
-// column tile follows nocc: with a fixed 128 half of the warps idled for nocc <= 64, and the smaller
-// tiles leave room for two CTAs per SM whose chains overlap (nao 243, nocc 27: 5.0 -> 3.1 ms of a
-// solve).  Staging 128 nu per half (256-byte rows) instead of 32 measured the same.
+// Bounds: shared memory (per 128 nu x 64 i of one P, clocks at 128 B/clk: the MMAs' operands 576 as
+// 64-column products and 384 as 128-column ones, the staging 512 as 2-byte stores and 256 as
+// transposed 8 x 8 matrices, the TMA copies 384) and the writes, 4.1 TB/s at nao 600; stored with an
+// evict-first policy they reach 3.4.  nao 600 (nocc 60): 98 -> 84 ms of a solve, nao 243 (nocc 27): 3.1
+// -> 2.7 (5.0 with one column tile of 128 for every nocc); 256-byte staged rows measured the same as
+// these of 64.
 template <int BN_>
 struct ResT {
-  static constexpr int BN = BN_, HW = BN_ / 2, STAGES = 4, MAX_KB = BN_ / 32, THREADS = 320, EPI_WARPS = 8;
+  static constexpr int BN = BN_, HW = BN_ / 2, PG = 128 / BN_, MAX_KB = BN_ / 32, THREADS = 320, EPI_WARPS = 8;
+  static constexpr int STAGES = BN_ == 64 ? 2 : 4;      // (two CTAs per SM for 32 and 64)
   static constexpr int A_TILE = BM * BK * 2;            // 8 KB: one K block of one plane
-  static constexpr int B_TILE = BN * BK * 2;            // 8 KB for 128 rows
+  static constexpr int B_TILE = 128 * BK * 2;           // 8 KB: PG aux functions
   static constexpr int A_BYTES = MAX_KB * 2 * A_TILE;   // 64 KB resident for 128
   static constexpr int STAGE_BYTES = 2 * B_TILE;        // hi + lo of one K block of O_P
   static constexpr int WARP_OUT = 2 * HW * 32 * 2;      // one warp's staged hi + lo tiles: HW i x 32 nu
@@ -614,20 +617,11 @@ struct ResT {
 };
 
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-// L2 policy that evicts the lines written first (T is streamed: read once, by term 1, after
-// the chunk is complete), so that the O tiles the next aux functions read stay in L2
-__device__ __forceinline__ uint64_t l2_evict_first() {
-  uint64_t p;
-  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
-  return p;
-}
-__device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, uint32_t src, int c0, int c1, int c2,
-                                             uint64_t policy) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.global.shared::cta.bulk_group.L2::cache_hint [%0, {%2, %3, %4}], [%1], %5;" ::"l"(
-          reinterpret_cast<uint64_t>(map)),
-      "r"(src), "r"(c0), "r"(c1), "r"(c2), "l"(policy)
-      : "memory");
+__device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, uint32_t src, int c0, int c1, int c2) {
+  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(
+                   reinterpret_cast<uint64_t>(map)),
+               "r"(src), "r"(c0), "r"(c1), "r"(c2)
+               : "memory");
 }
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_read0() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
@@ -641,7 +635,8 @@ __global__ void __launch_bounds__(320, ResT<BN_>::CTAS)
                             OzArgs args) {
   using R = ResT<BN_>;
   constexpr int STAGES = R::STAGES, BN = R::BN, HW = R::HW;
-  constexpr uint32_t ACC = BN;
+  constexpr int PG = R::PG;
+  constexpr uint32_t ACC = 128;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* ares = smem;
@@ -691,7 +686,7 @@ __global__ void __launch_bounds__(320, ResT<BN_>::CTAS)
         for (int t = 0; t < 2; ++t)
           tma_load_3d(smem_u32(ares + (kb * 2 + t) * R::A_TILE), &mA, abar, kb * BK, m0, t * args.a_depth + args.a_off);
       // O_P tiles of the aux range through the ring
-      const int total = nP * nkb;
+      const int total = (nP + PG - 1) / PG * nkb;
       int issued = 0;
       for (int it = 0; it < total; ++it) {
         const int s = it % STAGES;
@@ -699,7 +694,7 @@ __global__ void __launch_bounds__(320, ResT<BN_>::CTAS)
         issued = it + 1;
         const uint32_t full = full0 + 8 * s;
         mbar_expect_tx(full, R::STAGE_BYTES);
-        const int P = p_begin + it / nkb;
+        const int P = p_begin + it / nkb * PG;  // (past the range: other planes or zeros, not read)
         const int k0 = (it % nkb) * BK;
         const uint32_t st = smem_u32(ring + s * R::STAGE_BYTES);
         for (int t = 0; t < 2; ++t) tma_load_3d(st + t * R::B_TILE, &mB, full, k0, 0, t * args.b_depth + args.b_off + P);
@@ -708,11 +703,12 @@ __global__ void __launch_bounds__(320, ResT<BN_>::CTAS)
         mbar_wait(full0 + 8 * (it % STAGES), (it / STAGES) & 1, nullptr);
       mbar_wait(abar, 0, nullptr);  // the resident copies have landed before the CTA may exit
     } else if (warp == 1) {
-      constexpr uint32_t idesc = instr_desc_f16(BM, BN, false);
+      constexpr uint32_t idesc = instr_desc_f16(BM, 128, false);
       const bool el = elect_one();
       bool ok = __all_sync(0xffffffffu, mbar_wait(abar, 0, args.err));
       fence_after_sync();
-      for (int p = 0; p < nP && ok; ++p) {
+      const int groups = (nP + PG - 1) / PG;
+      for (int p = 0; p < groups && ok; ++p) {
         const int b = p & 1;
         if (!__all_sync(0xffffffffu, mbar_wait(acce0 + 8 * b, ((p >> 1) & 1) ^ 1, args.err))) break;
         fence_after_sync();
@@ -743,61 +739,74 @@ __global__ void __launch_bounds__(320, ResT<BN_>::CTAS)
       __syncwarp();
       mbar_wait(done, 0, nullptr);
     } else if (warp >= 2) {
-      // epilogue: TMEM lane quarter q (rows nu0 + 32 q + lane), columns i in [HW h, HW h + ni)
+      // epilogue: TMEM lane quarter q (rows nu0 + 32 q ..), columns i in [HW h, HW h + ni) of each P
       const int q = warp & 3;
       const int h = (warp - 2) >> 2;
       const int ni = min(HW, no - HW * h);  // this warp's columns (may be none)
-      const int nul = q * 32 + lane;
-      const bool row_ok = nu0 + nul < nao;
-      const int erow = row_ok ? args.e_row[m0 + nul] - 2 * Split2::EOFF : 0;
-      // T's scale is a power of two: its exponent joins the row's and the aux function's
+      // a lane's fragments: rows 32 q + lane / 4 + {0, 8, 16, 24}, columns 2 (lane % 4) + {0, 1} of
+      // every eight; T's scale is a power of two: its exponent joins the row's and the aux function's
       const int ets = pow2_exponent(*args.tscale);
-      // O_P's planes carry one exponent per aux function, so the row has one factor per P; the
+      int erow[4];
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const int nu = q * 32 + (lane >> 2) + 8 * t;
+        erow[t] = nu0 + nu < nao ? args.e_row[m0 + nu] - 2 * Split2::EOFF + ets : -1000;
+      }
+      // O_P's planes carry one exponent per aux function, so a row has one factor per P; the
       // exponent of p + 1 is fetched while p is processed
       const int* const eP = args.e_col + (int64_t)(args.b_off + p_begin) * args.N;
       int e_next = eP[0];
-      uint8_t* const wst = outs + (warp - 2) * R::WARP_OUT;
-      __half* const sh = reinterpret_cast<__half*>(wst) + lane;  // [HW i][32 nu]
-      __half* const sl = sh + HW * 32;
+      uint8_t* const wst = outs + (warp - 2) * R::WARP_OUT;  // [plane][HW i][32 nu], 64-byte swizzled rows
+      // stmatrix row of this lane: matrix (eight nu) lane / 8, column i = lane % 8
+      const uint32_t srow = smem_u32(wst) + (lane & 7) * 64 + (((lane >> 3) ^ ((lane >> 1) & 3)) << 4);
       const CUtensorMap* const mh = h == 0 ? &mTh0 : &mTh1;
       const CUtensorMap* const ml = h == 0 ? &mTl0 : &mTl1;
-      const uint64_t policy = l2_evict_first();
       for (int p = 0; p < nP; ++p) {
-        const int b = p & 1;
+        const int u = p / PG, g = p - u * PG, b = u & 1;
         const int e_p = e_next;
         if (p + 1 < nP) e_next = eP[(int64_t)(p + 1) * args.N];
-        if (!__all_sync(0xffffffffu, mbar_wait(accf0 + 8 * b, (p >> 1) & 1, args.err))) break;
-        fence_after_sync();
-        float v[HW];
-        const uint32_t tb = tmem + (uint32_t)b * ACC + ((uint32_t)(q * 32) << 16) + (uint32_t)(h * HW);
-        if constexpr (HW == 64) tmem_ld32x2(tb, tb + 32, v, v + 32);
-        else if constexpr (HW == 32) tmem_ld32(tb, v);
-        else tmem_ld16(tb, v);
-        fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(acce0 + 8 * b);  // accumulator b may take aux p + 2
+        if (g == 0) {
+          if (!__all_sync(0xffffffffu, mbar_wait(accf0 + 8 * b, (u >> 1) & 1, args.err))) break;
+          fence_after_sync();
+        }
+        float v[2][HW / 2];  // lanes 0-15 and 16-31 of the quarter
+        const uint32_t tb = tmem + (uint32_t)b * ACC + ((uint32_t)(q * 32) << 16) + (uint32_t)(g * BN + h * HW);
+        tmem_ld_16x256<HW / 8>(tb, v[0]);
+        tmem_ld_16x256<HW / 8>(tb + (16u << 16), v[1]);
+        if (g == PG - 1 || p + 1 == nP) {
+          fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(acce0 + 8 * b);  // accumulator b may take the group after next
+        }
         if (ni <= 0) continue;
         // this warp's staged tiles of p - 1 have left shared memory before they are overwritten
         if (lane == 0) bulk_wait_read0();
         __syncwarp();
-        const float f = pow2f(erow + e_p + ets);
-        // two columns per conversion (columns >= ni are staged but not stored)
+        float f[4];
 #pragma unroll
-        for (int j = 0; j < HW; j += 2) {
-          const float x0 = v[j] * f, x1 = v[j + 1] * f;
-          const __half2 hh = __floats2half2_rn(x0, x1);
-          const __half2 ll = __floats2half2_rn(x0 - __low2float(hh), x1 - __high2float(hh));
-          sh[j * 32] = __low2half(hh);
-          sh[(j + 1) * 32] = __high2half(hh);
-          sl[j * 32] = __low2half(ll);
-          sl[(j + 1) * 32] = __high2half(ll);
+        for (int t = 0; t < 4; ++t) f[t] = pow2f(erow[t] + e_p);
+        // eight columns at a time (of the last eight, those >= ni are staged but not stored)
+#pragma unroll
+        for (int j = 0; j < HW / 8; ++j) {
+          if (8 * j >= ni) break;
+          uint32_t hi[4], lo[4];
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            const float x0 = v[t >> 1][4 * j + 2 * (t & 1)] * f[t], x1 = v[t >> 1][4 * j + 2 * (t & 1) + 1] * f[t];
+            const __half2 hh = __floats2half2_rn(x0, x1);
+            const __half2 ll = __floats2half2_rn(x0 - __low2float(hh), x1 - __high2float(hh));
+            hi[t] = *reinterpret_cast<const uint32_t*>(&hh);
+            lo[t] = *reinterpret_cast<const uint32_t*>(&ll);
+          }
+          stmatrix_x4_trans(srow + j * 512, hi);
+          stmatrix_x4_trans(srow + R::WARP_OUT / 2 + j * 512, lo);
         }
         fence_proxy_async();  // the generic-proxy writes are visible to the TMA stores
         __syncwarp();
         if (lane == 0 && nu0 + q * 32 < nao) {
           const int Pl = p_begin + p;
-          tma_store_3d(mh, smem_u32(wst), nu0 + q * 32, a_pert * no + HW * h, Pl, policy);
-          tma_store_3d(ml, smem_u32(wst + R::WARP_OUT / 2), nu0 + q * 32, a_pert * no + HW * h, Pl, policy);
+          tma_store_3d(mh, smem_u32(wst), nu0 + q * 32, a_pert * no + HW * h, Pl);
+          tma_store_3d(ml, smem_u32(wst + R::WARP_OUT / 2), nu0 + q * 32, a_pert * no + HW * h, Pl);
           bulk_commit();
         }
       }
@@ -1042,17 +1051,17 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   return fn;
 }
 
-// 3-D BF16 / FP16 tensor map: dims {K, rows, depth}, row stride ld elements, box {32, box_rows, 1},
-// 64B swizzle.
+// 3-D BF16 / FP16 tensor map: dims {K, rows, depth}, row stride ld elements, box {32, box_rows,
+// box_depth}, 64B swizzle.
 CUtensorMap make_map(const void* base, int64_t K, int64_t rows, int64_t depth, int64_t ld, int box_rows,
-                     bool bf16 = true) {
+                     bool bf16 = true, int box_depth = 1) {
   CUtensorMap m;
   std::memset(&m, 0, sizeof(m));
   auto fn = encode_fn();
   if (!fn) throw Error(CPHF_ERR_CUDA, "cuTensorMapEncodeTiled unavailable");
   cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)rows, (cuuint64_t)depth};
   cuuint64_t strides[2] = {(cuuint64_t)(ld * 2), (cuuint64_t)(ld * 2 * rows)};
-  cuuint32_t box[3] = {(cuuint32_t)BK, (cuuint32_t)box_rows, 1};
+  cuuint32_t box[3] = {(cuuint32_t)BK, (cuuint32_t)box_rows, (cuuint32_t)box_depth};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = fn(&m, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3,
                   const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -1208,7 +1217,8 @@ void launch_tgen_resident_raw(cphf_ctx* c, const CUtensorMap& mA, const CUtensor
   if (tiles > 65535) throw Error(CPHF_ERR_ARG, "tensor-core T generation: grid too large");
   const int bn = res_bn(a.N);
   const int64_t slots = (int64_t)c->num_sms * (bn == 128 ? 1 : 2);
-  a.p_per_cta = (int)std::max<int64_t>(1, std::min<int64_t>(a.np, a.np * tiles / (waves * slots)));
+  const int64_t pg = 128 / bn;  // whole groups of aux functions
+  a.p_per_cta = (int)(div_up(std::max<int64_t>(1, std::min<int64_t>(a.np, a.np * tiles / (waves * slots))), pg) * pg);
   const dim3 grid((unsigned)div_up(a.np, a.p_per_cta), (unsigned)tiles);
   auto launch = [&](auto kern, int smem) {
     kern<<<grid, 320, smem, c->stream>>>(mA, mB, mT[0], mT[1], mT[2], mT[3], a);
@@ -1241,7 +1251,7 @@ void launch_tgen_resident(cphf_ctx* c, const CUtensorMap& mA, const CUtensorMap&
 
 // 3-D FP16 map of T's planes for the TMA stores of the resident T generation: dims {nu (nao),
 // n = i + nocc a (N), Pl (npc)}, row stride ldt, box {32 nu, ni, 1} (one epilogue warp's part,
-// ni of its columns), no swizzle (the staged tile is [ni][32] dense)
+// ni of its columns) of 64-byte rows, swizzled as they are staged
 CUtensorMap make_t_store_map(const __half* base, int64_t nao, int64_t N, int64_t npc, int64_t ldt, int64_t ni) {
   CUtensorMap m;
   std::memset(&m, 0, sizeof(m));
@@ -1252,7 +1262,7 @@ CUtensorMap make_t_store_map(const __half* base, int64_t nao, int64_t N, int64_t
   cuuint32_t box[3] = {32, (cuuint32_t)ni, 1};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = fn(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<__half*>(base), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) throw Error(CPHF_ERR_CUDA, "cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")");
   return m;
@@ -1599,7 +1609,7 @@ void lp_tgen_planes(cphf_ctx* c, OzState& z, int s, int64_t P0, int64_t npc, int
   if (no <= 128 && res_attr_ok()) {
     // bra tile resident, all i of a column in one tile of bn columns
     const int bn = res_bn(no);
-    const CUtensorMap mO128 = make_map(z.spin[s].O.p, no, no, S2 * naux, ldj, bn, false);
+    const CUtensorMap mO128 = make_map(z.spin[s].O.p, no, no, S2 * naux, ldj, bn, false, 128 / bn);
     // store maps of the epilogue warps' parts: columns [0, bn / 2) and [bn / 2, nocc)
     const int64_t n0c = std::min<int64_t>(no, bn / 2), n1c = std::max<int64_t>(no - bn / 2, 1);
     const CUtensorMap mT[4] = {make_t_store_map(hi, nao, N, npc, ldt, n0c), make_t_store_map(hi, nao, N, npc, ldt, n1c),
