@@ -115,14 +115,17 @@ __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
   e = (a - (s - bb)) + (b - bb);
 }
 
-// (hi, lo) ~ a0 + a1 + a2 + a3 (a0, a1, a2 exact integer sums, a3 rounded)
+// (hi, lo) ~ a0 + a1 + a2 + a3 (a0, a1, a2 exact integer sums, a3 rounded; three slices: no a3)
+template <int NS>
 __device__ __forceinline__ void combine4(float a0, float a1, float a2, float a3, float& hi, float& lo) {
   float s, e, e2;
   two_sum(a0, a1, s, e);
   two_sum(s, a2, s, e2);
   e += e2;
-  two_sum(s, a3, s, e2);
-  e += e2;
+  if constexpr (NS > 3) {
+    two_sum(s, a3, s, e2);
+    e += e2;
+  }
   hi = s + e;
   lo = e - (hi - s);
 }
@@ -515,7 +518,7 @@ __global__ void __launch_bounds__(320, PR::NACC == 4 ? 1 : 2)
                 const int j = 16 * hf + jj;
                 const float f = __uint_as_float((unsigned)(eb + __shfl_sync(0xffffffffu, ec, j)) << 23);
                 float hi, lo;
-                combine4(v0[jj], v1[jj], v2[jj], v3[jj], hi, lo);
+                combine4<PR::S>(v0[jj], v1[jj], v2[jj], v3[jj], hi, lo);
                 __stcs(o + j * sn, make_float2(hi * f, lo * f));
                 if constexpr (EPI == EPI_STOREMAX) cmax[j] = fmaxf(cmax[j], fabsf(hi * f));
               }
@@ -526,7 +529,7 @@ __global__ void __launch_bounds__(320, PR::NACC == 4 ? 1 : 2)
                 const float f = pow2f(erow + __shfl_sync(0xffffffffu, ec, j));
                 if (row_ok && n0 + c * 32 + j < args.N) {
                   float hi, lo;
-                  combine4(v0[jj], v1[jj], v2[jj], v3[jj], hi, lo);
+                  combine4<PR::S>(v0[jj], v1[jj], v2[jj], v3[jj], hi, lo);
                   __stcs(o + j * sn, make_float2(hi * f, lo * f));
                   if constexpr (EPI == EPI_STOREMAX) cmax[j] = fmaxf(cmax[j], fabsf(hi * f));
                 }

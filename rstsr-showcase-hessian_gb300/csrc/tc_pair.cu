@@ -121,14 +121,17 @@ __device__ __forceinline__ double widen(float x) {
   const unsigned hi = (b & 0x80000000u) | (((b & 0x7FFFFFFFu) >> 3) + 0x38000000u) | (e == 0x7F800000u ? 0x7FF00000u : 0u);
   return __hiloint2double(e == 0u ? 0 : (int)hi, e == 0u ? 0 : (int)(b << 29));
 }
-// a0 + a1 + a2 + a3 (a0, a1, a2 exact integer sums, a3 rounded) through an FP32 pair
+// a0 + a1 + a2 + a3 (a0, a1, a2 exact integer sums, a3 rounded; three slices: no a3) through an FP32 pair
+template <int NS>
 __device__ __forceinline__ double combine4(float a0, float a1, float a2, float a3) {
   float s, e, e2;
   two_sum(a0, a1, s, e);
   two_sum(s, a2, s, e2);
   e += e2;
-  two_sum(s, a3, s, e2);
-  e += e2;
+  if constexpr (NS > 3) {
+    two_sum(s, a3, s, e2);
+    e += e2;
+  }
   return widen(s) + widen(e);
 }
 // x 2^k by the exponent field; subnormal operands and results to zero, NaN and Inf stay
@@ -274,7 +277,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
           for (int j = 0; j < 16; ++j) v3[j] = 0.f;  // groups 0-2 only: the fourth accumulator is unused
         }
 #pragma unroll
-        for (int j = 0; j < 16; ++j) tp[j * 33 + lane] = combine4(v0[j], v1[j], v2[j], v3[j]) * cs;
+        for (int j = 0; j < 16; ++j) tp[j * 33 + lane] = combine4<PR::S>(v0[j], v1[j], v2[j], v3[j]) * cs;
         __syncwarp();
         if (c + wm < c_end) {
           const int k = ((__double2hiint(args.rowscale[m0 + c + wm]) >> 20) & 0x7FF) - 1023;
