@@ -91,7 +91,8 @@ struct OzArgs {
   const float* rho_ao;
   int64_t ld_rho, ld_ao;
   int rho_nocc;
-  int np, p_per_cta;        // batched: aux functions of the launch, per CTA
+  int np, p_per_cta;        // batched: aux functions of the launch, per CTA (a multiple of pg)
+  int pg;                   // batched: aux functions per 64-column tile (2: N <= 32, 32 columns each)
   // batched split-FP16 T generation writing the FP16 hi / lo planes of T * (*tscale) for
   // tc_gemm.cu's term 1
   const float* tscale;
@@ -360,7 +361,8 @@ __global__ void __launch_bounds__(320, PR::NACC == 4 ? 1 : 2)
   const int m0 = m_tile * BM, n0 = n_tile * BN;
   const int p_begin = blockIdx.x * args.p_per_cta;
   const int nP = min(args.np - p_begin, args.p_per_cta);
-  const int nkb = args.nkb;
+  const int nkb = args.nkb, pg = args.pg;
+  const int groups = (nP + pg - 1) / pg;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -383,7 +385,7 @@ __global__ void __launch_bounds__(320, PR::NACC == 4 ? 1 : 2)
   if (nP > 0) {
     if (warp == 0 && lane == 0) {
       // producer: K blocks of every aux function of the range, back to back through the ring
-      const int total = nP * nkb;
+      const int total = groups * nkb;
       int issued = 0;
       for (int it = 0; it < total; ++it) {
         const int s = it % STAGES;
@@ -392,7 +394,7 @@ __global__ void __launch_bounds__(320, PR::NACC == 4 ? 1 : 2)
         issued = it + 1;
         const uint32_t full = full0 + 8 * s;
         mbar_expect_tx(full, C::STAGE_BYTES);
-        const int P = p_begin + it / nkb;
+        const int P = p_begin + it / nkb * pg;
         const int k0 = (it % nkb) * BK;
         const int db = args.b_off + P;
         const uint32_t st = smem_u32(smem + s * C::STAGE_BYTES);
@@ -409,7 +411,7 @@ __global__ void __launch_bounds__(320, PR::NACC == 4 ? 1 : 2)
       constexpr uint32_t idesc = instr_desc_f16(BM, BN, PR::BF16);
       const bool el = elect_one();
       bool ok = true;
-      for (int p = 0; p < nP && ok; ++p) {
+      for (int p = 0; p < groups && ok; ++p) {
         const int b = p & 1;
         if (!__all_sync(0xffffffffu, mbar_wait(acce0 + 8 * b, ((p >> 1) & 1) ^ 1, args.err))) break;
         fence_after_sync();
@@ -454,9 +456,12 @@ __global__ void __launch_bounds__(320, PR::NACC == 4 ? 1 : 2)
       __syncwarp();
       mbar_wait(done, 0, nullptr);
     } else if (warp >= 2) {
-      // epilogue: TMEM lane quarter q, 32-column chunk c
+      // epilogue: TMEM lane quarter q, 32-column chunk c: columns col0 .. of every aux function, or of
+      // the group's c-th
       const int q = warp & 3;
       const int c = (warp - 2) >> 2;
+      const int dp = pg == 2 ? c : 0, col0 = pg == 2 ? 0 : n0 + c * 32;
+      const int jn = min(32, args.N - col0);  // columns inside (none: <= 0)
       const int row = m0 + q * 32 + lane;
       const bool row_ok = row < args.M;
       int erow = 0;
@@ -465,7 +470,7 @@ __global__ void __launch_bounds__(320, PR::NACC == 4 ? 1 : 2)
         erow = args.e_row[row] - 2 * PR::EOFF;
         base = args.m_div > 0 ? (row % args.m_div) * args.s_m1 + (row / args.m_div) * args.s_m2 : row * args.s_m1;
       }
-      const int ncol = n0 + c * 32 + lane;  // the column whose exponent this lane fetches
+      const int ncol = jn > 0 ? col0 + min(lane, jn - 1) : 0;  // the column whose exponent this lane fetches
       // EPI_STOREMAX: the row's block index a = row / m_div selects the staging column n + N a
       const int64_t arow = (row_ok && args.m_div > 0) ? row / args.m_div : 0;
       float cmax[EPI == EPI_STOREMAX ? 32 : 1];
@@ -475,31 +480,32 @@ __global__ void __launch_bounds__(320, PR::NACC == 4 ? 1 : 2)
       }
       // the column exponent of aux function p + 1 is fetched while p is processed (its load
       // latency would otherwise stall every aux function's epilogue)
-      const int* const ecp = args.e_col + (int64_t)(args.b_off + p_begin) * args.N + ncol;
-      int ec_next = (nP > 0 && ncol < args.N) ? ecp[0] : 0;
-      for (int p = 0; p < nP; ++p) {
+      const int* const ecp = args.e_col + (int64_t)(args.b_off + p_begin + dp) * args.N + ncol;
+      int ec_next = dp < nP ? ecp[0] : 0;
+      for (int p = 0; p < groups; ++p) {
         const int b = p & 1;
         const int ec = ec_next;
-        if (p + 1 < nP && ncol < args.N) ec_next = ecp[(int64_t)(p + 1) * args.N];
+        const bool live = p * pg + dp < nP && jn > 0;  // (warp-uniform)
+        if ((p + 1) * pg + dp < nP) ec_next = ecp[(int64_t)(p + 1) * pg * args.N];
         // warp-uniform decision: tcgen05.ld is a whole-warp instruction
         if (!__all_sync(0xffffffffu, mbar_wait(accf0 + 8 * b, (p >> 1) & 1, args.err))) break;
         fence_after_sync();
-        const int Pl = p_begin + p;
+        const int Pl = p_begin + p * pg + dp;
         const uint32_t lane_base = tmem + (uint32_t)b * ACC + ((uint32_t)(q * 32) << 16);
         const int64_t pbase = base + (int64_t)Pl * args.s_p;
-        if constexpr (PR::NACC == 4) {
-          float2* const o = reinterpret_cast<float2*>(args.out) + pbase + (int64_t)(n0 + c * 32) * args.s_n;
+        if (!live) {
+          // nothing of the chunk is inside
+        } else if constexpr (PR::NACC == 4) {
+          float2* const o = reinterpret_cast<float2*>(args.out) + pbase + (int64_t)col0 * args.s_n;
           const int sn = (int)args.s_n;
-          // the common case without per-element predicates or range checks: every row and
-          // column of the chunk in range, every factor 2^(erow + ec) a normal float (its bit
-          // pattern (erow + ec + 127) << 23)
+          // the common case without range checks: every factor 2^(erow + ec) of the chunk a normal
+          // float (its bit pattern (erow + ec + 127) << 23); rows outside hold zeros
           int emn = ec, emx = ec;
           for (int o2 = 16; o2 > 0; o2 >>= 1) {
             emn = min(emn, __shfl_xor_sync(0xffffffffu, emn, o2));
             emx = max(emx, __shfl_xor_sync(0xffffffffu, emx, o2));
           }
-          const bool fast = __all_sync(0xffffffffu, row_ok && erow + emn >= -126 && erow + emx <= 127) &&
-                            args.N - (n0 + c * 32) >= 32;
+          const bool fast = __all_sync(0xffffffffu, !row_ok || (erow + emn >= -126 && erow + emx <= 127));
           const int eb = erow + 127;
           // two halves of 16 columns: four accumulators of 16 columns in registers at a time
 #pragma unroll
@@ -516,10 +522,11 @@ __global__ void __launch_bounds__(320, PR::NACC == 4 ? 1 : 2)
 #pragma unroll
               for (int jj = 0; jj < 16; ++jj) {
                 const int j = 16 * hf + jj;
+                if (j >= jn) break;
                 const float f = __uint_as_float((unsigned)(eb + __shfl_sync(0xffffffffu, ec, j)) << 23);
                 float hi, lo;
                 combine4<PR::S>(v0[jj], v1[jj], v2[jj], v3[jj], hi, lo);
-                __stcs(o + j * sn, make_float2(hi * f, lo * f));
+                if (row_ok) __stcs(o + j * sn, make_float2(hi * f, lo * f));
                 if constexpr (EPI == EPI_STOREMAX) cmax[j] = fmaxf(cmax[j], fabsf(hi * f));
               }
             } else {
@@ -527,7 +534,7 @@ __global__ void __launch_bounds__(320, PR::NACC == 4 ? 1 : 2)
               for (int jj = 0; jj < 16; ++jj) {
                 const int j = 16 * hf + jj;
                 const float f = pow2f(erow + __shfl_sync(0xffffffffu, ec, j));
-                if (row_ok && n0 + c * 32 + j < args.N) {
+                if (row_ok && j < jn) {
                   float hi, lo;
                   combine4<PR::S>(v0[jj], v1[jj], v2[jj], v3[jj], hi, lo);
                   __stcs(o + j * sn, make_float2(hi * f, lo * f));
@@ -543,16 +550,16 @@ __global__ void __launch_bounds__(320, PR::NACC == 4 ? 1 : 2)
           tmem_ld32(lane_base + (uint32_t)(c * 32), v);
           // (every column of O_P carries the aux function's exponent: lane 0's, fetched ahead)
           const float f = pow2f(erow + __shfl_sync(0xffffffffu, ec, 0) + pow2_exponent(*args.tscale));
-          const int64_t off = pbase + (int64_t)(n0 + c * 32) * args.s_n;
+          const int64_t off = pbase + (int64_t)col0 * args.s_n;
           if (row_ok)
             store_split32(v, f, reinterpret_cast<__half*>(args.out) + off, reinterpret_cast<__half*>(args.out_lo) + off,
-                          (int)args.s_n, min(32, args.N - (n0 + c * 32)));
+                          (int)args.s_n, jn);
         } else {
           float v[32];
           tmem_ld32(lane_base + (uint32_t)(c * 32), v);
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
-            const int n = n0 + c * 32 + j;
+            const int n = col0 + j;
             const float f = pow2f(erow + __shfl_sync(0xffffffffu, ec, j));
             if (row_ok && n < args.N) __stcs(reinterpret_cast<float*>(args.out) + pbase + n * args.s_n, v[j] * f);
           }
@@ -568,7 +575,7 @@ __global__ void __launch_bounds__(320, PR::NACC == 4 ? 1 : 2)
         const bool uniform = __all_sync(0xffffffffu, !row_ok || arow == a0) && __any_sync(0xffffffffu, row_ok);
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
-          const int n = n0 + c * 32 + j;
+          const int n = col0 + j;
           if (n >= args.N) continue;
           float m = row_ok ? cmax[j] : 0.f;
           if (uniform) {
@@ -1172,6 +1179,7 @@ void launch_batched_raw(cphf_ctx* c, const CUtensorMap& mA, const CUtensorMap& m
   const int64_t tiles = (int64_t)a.m_tiles * div_up(a.N, 64);
   if (tiles > 65535) throw Error(CPHF_ERR_ARG, "tensor-core K term: grid too large");
   a.p_per_cta = (int)std::max<int64_t>(1, std::min<int64_t>(a.np, a.np * tiles / (waves * (int64_t)c->num_sms)));
+  a.p_per_cta = (int)div_up(a.p_per_cta, a.pg) * a.pg;
   const dim3 grid((unsigned)div_up(a.np, a.p_per_cta), (unsigned)tiles);
   tc_slice_batched_kernel<PR, 64, EPI><<<grid, Batched<PR>::THREADS, Batched<PR>::SMEM_BYTES, c->stream>>>(mA, mB, a);
   count_launch();
@@ -1278,6 +1286,7 @@ OzArgs base_args(OzState& z, int M, int N) {
   a.M = M;
   a.N = N;
   a.m_tiles = (int)div_up(M, BM);
+  a.pg = 1;
   a.err = z.err.as<int>();
   return a;
 }
@@ -1407,9 +1416,13 @@ static void oz_k_terms_t(cphf_ctx* c, OzState& z, int s, const double* bra, int6
   z.mxc.ensure((size_t)N * 8, c->counter());
 
   const CUtensorMap mBt = make_map(z.brat.p, no, nao * nb, S, ldj, BM);            // T-gen A
-  const CUtensorMap mO = make_map(os.O.p, no, no, S * naux, ldj, 64);               // T-gen B
+  // a 64-column tile of T and W generation holds two aux functions where nocc <= 32, half the MMAs and
+  // loads (T generation, six / three slices: nao 243, nocc 27 2.1 / 1.9 -> 1.1 / 0.87 ms; with the
+  // ragged columns off the slow epilogue nao 600, nocc 60 51 / 39.5 -> 42 / 28)
+  const int pg = no <= 32 ? 2 : 1;
+  const CUtensorMap mO = make_map(os.O.p, no, no, S * naux, ldj, 64 / pg, true, pg);   // T-gen B
   const CUtensorMap mBw = make_map(z.braw.p, nao, N, S, ldk, BM);                  // W-gen A
-  const CUtensorMap mZ = make_map(os.Z.p, nao, no, S * naux, ldk, 64);             // W-gen B
+  const CUtensorMap mZ = make_map(os.Z.p, nao, no, S * naux, ldk, 64 / pg, true, pg);  // W-gen B
   const int nkb_nao = (int)div_up(nao, BK), nkb_no = (int)div_up(no, BK);
 
   for (int64_t P0 = 0; P0 < naux; P0 += np) {
@@ -1426,6 +1439,7 @@ static void oz_k_terms_t(cphf_ctx* c, OzState& z, int s, const double* bra, int6
       a.e_row = z.ebrat.as<int>();
       a.e_col = os.eO.as<int>();
       a.m_div = nao; a.s_m1 = 1; a.s_m2 = ldk * no; a.s_n = ldk; a.s_p = N * ldk;
+      a.pg = pg;
       a.colmax = z.mxc.as<unsigned long long>();  // T's column maxima, reduced in the epilogue
       ProfScope ps(c, tP, 2.0 * nao * nb * no * no * npc, 0.0);
       a.np = (int)npc;
@@ -1467,6 +1481,7 @@ static void oz_k_terms_t(cphf_ctx* c, OzState& z, int s, const double* bra, int6
       a.e_col = os.eZ.as<int>();
       a.m_div = no; a.s_m1 = 1; a.s_m2 = ldj * no; a.s_n = ldj; a.s_p = N * ldj;
       // W's staging column (i, a) = i + nocc (row / nocc): its maxima reduced in the epilogue
+      a.pg = pg;
       a.colmax = z.mxc.as<unsigned long long>();
       ProfScope ps(c, wP, 2.0 * N * no * nao * npc, 0.0);
       a.np = (int)npc;

@@ -70,3 +70,16 @@ def test_t_generation_at_column_tile_edges(nocc):
     got = ctx.response_dimless_cphf_lowp(mo1)
     assert ctx.tensor_cores_active
     assert rel_err(got, _oracle(s).response_dimless_cphf(mo1)) < 1e-5
+
+
+@pytest.mark.parametrize("naux,chunk", [(21, 8), (20, 7), (1, 0)])
+@pytest.mark.parametrize("nocc", [1, 31, 32, 33, 64, 65])
+def test_exact_generation_at_column_tile_edges(nocc, naux, chunk):
+    """T and W of the exact slices come two aux functions to a column tile for nocc <= 32."""
+    s = _system(131, naux, nocc, 2)
+    ctx = _context(s, residual_dfloat=2, max_refine=1, residual_tol=1.0, verify_residual=0, aux_chunk=chunk)
+    x = ctx.solve_dimless_cphf(s.rhs[0])
+    assert ctx.last_stats["residual_mode"] == 2
+    r = (s.rhs[0] - x - _oracle(s).response_dimless_cphf(x)).reshape(-1, 6, order="F")
+    ref = float(np.linalg.norm(r, axis=0).max())
+    assert abs(ctx.last_stats["residual_max"] - ref) < 1e-9 * max(1.0, np.abs(x).max())
