@@ -56,7 +56,9 @@ void lowp_park(cphf_ctx* c) {
 }
 
 void lowp_prepare(cphf_ctx* c) {
-  std::vector<int64_t> shape{c->nao, c->naux, c->has_rijk, c->has_xc, c->ngrids, c->xc_den, c->xc_nvar, c->nspin};
+  std::vector<int64_t> shape{c->nao,       c->naux, c->has_rijk,           c->has_xc,         c->ngrids,
+                             c->xc_den,    c->xc_nvar, c->cfg.tensor_cores, c->cfg.aux_chunk, c->cfg.xc_chunk_points,
+                             c->nspin};
   for (int s = 0; s < c->nspin; ++s) shape.insert(shape.end(), {c->spin[s].nmo, c->spin[s].nocc});
   bool fresh = false;
   if (!c->lowp && c->lowp_parked && c->lowp_parked->shape == shape) c->lowp = std::move(c->lowp_parked);
