@@ -642,8 +642,8 @@ def run_gpu(args, world, rank, local):
                                  f"counts algorithmic FLOPs") + (f"; {note}" if note else ""))
     # DRAM bytes per launch: the ratio of ncu-measured DRAM bytes to the algorithmic bytes of
     # the same kernel on a small case (profiles/), times this run's algorithmic bytes per launch
-    traffic_ratio = {"kterm_tcgen05_f16x3": 9.99 / 9.25,         # tc_term1_kernel, rhf_nao384_occ120
-                     "kterm_tcgen05_bf16x6_exact": 5.954 / 5.22}  # tc_slice_kernel<Exact6>, rhf_nao300
+    traffic_ratio = {"kterm_tcgen05_f16x3": 1.123 / 1.121,       # tc_pair_kernel<Split2>, nao 384, naux 400
+                     "kterm_tcgen05_bf16x6_exact": 3.67 / 3.36}   # tc_pair_kernel<Exact6>, nao 384, naux 400
     traffic = None
     if dom_name in traffic_ratio and dom.get("bytes", 0) > 0:
         traffic = traffic_ratio[dom_name] * dom["bytes"] / dom["launches"]
