@@ -30,6 +30,7 @@ struct PairTerm {
   int64_t x_row0 = 0;  // X row of m = 0
   int64_t y_k0 = 0;    // Y column of k = 0, a multiple of 8
   bool store = false;  // exact slices, one K range: out = the value (no accumulation)
+  int64_t max_k = 0;   // split FP16, np > 1: products an FP32 accumulator sums at most (0: any number)
 };
 
 bool pair_available(int device);
