@@ -21,6 +21,7 @@ def test_exchange_sums_stay_short(nao, naux, nocc, natm):
     draw = lambda *shape: torch.randn(shape, generator=gen, dtype=torch.float64, device="cuda")
     nu, mu = torch.tril_indices(nao, nao, device="cuda")
     cderi = draw(naux, mu.numel()) * 0.3 * torch.exp((mu - nu).double() / 20.0)
+    torch.cuda.synchronize()  # the context reads it on a stream of its own
     occ = np.zeros(nao)
     occ[:nocc] = 2.0
     ctx = Context(precision="mixed")
