@@ -751,9 +751,8 @@ bool fx_plan(const GemmDesc& d0, int num_sms, FxPlan& p) {
   t.c_m = d0.c_n; t.c_m2 = d0.c_n2; t.c_n = d0.c_m; t.c_n2 = d0.c_m2;
   const int64_t tiles0 = div_up(d0.M, BM) * div_up(d0.N, BN), tiles1 = div_up(t.M, BM) * div_up(t.N, BN);
   // fewest padded tiles; equal: rows of the tile along the unit stride of C
-  const bool swap = div_up(t.N, 64) <= 65535 && (tiles1 < tiles0 || (tiles1 == tiles0 && d0.c_m != 1 && d0.c_n == 1));
+  const bool swap = tiles1 < tiles0 || (tiles1 == tiles0 && d0.c_m != 1 && d0.c_n == 1);
   p.d = swap ? t : d0;
-  if (div_up(p.d.N, 64) > 65535) return false;  // grid limit of the native kernel behind the flag
   const GemmDesc& d = p.d;
   p.ldk = div_up(d.K, 8) * 8;
   p.n_tiles = (int)div_up(d.N, BN);
