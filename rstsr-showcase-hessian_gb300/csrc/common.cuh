@@ -9,6 +9,7 @@
 #include <string>
 
 #include "../../include/cphf.h"
+#include "per_device.cuh"
 
 namespace cphf {
 
@@ -90,6 +91,18 @@ struct DevBuf {
 extern thread_local int64_t* g_launch_counter;
 inline void count_launch(int64_t n = 1) {
   if (g_launch_counter) *g_launch_counter += n;
+}
+
+// Lets `kernel` use `bytes` of shared memory on the current device.
+inline void allow_smem(PerDevice& done, const void* kernel, int bytes) {
+  int dev = 0;
+  CPHF_CUDA(cudaGetDevice(&dev));
+  cudaError_t e = cudaSuccess;
+  done.once(dev, [&] {
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    return e == cudaSuccess;
+  });
+  CPHF_CUDA(e);
 }
 
 inline int64_t div_up(int64_t a, int64_t b) { return (a + b - 1) / b; }

@@ -140,11 +140,8 @@ __global__ void __launch_bounds__(kThreads) tri_rows_kernel(TriArgs a) {
 }
 constexpr int kTriSmem = (TB * TB + TB * kTriRows + TB) * 8;
 void launch_tri_rows(cphf_ctx* c, const TriArgs& a, int64_t rows, int64_t blocks) {
-  static bool attr = false;
-  if (!attr) {
-    CPHF_CUDA(cudaFuncSetAttribute(tri_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTriSmem));
-    attr = true;
-  }
+  static PerDevice smem;
+  allow_smem(smem, (const void*)tri_rows_kernel, kTriSmem);
   tri_rows_kernel<<<dim3((unsigned)div_up(rows, kTriRows), (unsigned)blocks), kThreads, kTriSmem, c->stream>>>(a);
   count_launch();
   CPHF_CUDA(cudaGetLastError());

@@ -775,12 +775,8 @@ void launch_mgs(double* V, int64_t n, int64_t m, double lindep, double* ip, int*
   a.coef = partials + kMgsPanel * m * nblk;
   a.bar = reinterpret_cast<unsigned*>(a.coef + kMgsPanel * m + 1);
   const size_t smem = (size_t)kMgsPanel * (2 * a.stage + std::min(m, kMgsCoefs)) * 8;
-  static bool attr = false;
-  if (!attr) {
-    CPHF_CUDA(cudaFuncSetAttribute(mgs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   kMgsPanel * (int)(2 * kMgsStage + kMgsCoefs) * 8));
-    attr = true;
-  }
+  static PerDevice limit;
+  allow_smem(limit, (const void*)mgs_kernel, kMgsPanel * (int)(2 * kMgsStage + kMgsCoefs) * 8);
   CPHF_CUDA(cudaMemsetAsync(a.bar, 0, sizeof(unsigned), s));
   void* args[] = {&a};
   CPHF_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(mgs_kernel), dim3((unsigned)nblk),
@@ -814,11 +810,8 @@ void launch_lu_solve(double* h, int64_t ldh, double* g, int64_t ldg, int64_t m, 
   LuMoves* moves = reinterpret_cast<LuMoves*>(info + 1);
   CPHF_CUDA(cudaMemsetAsync(info, 0, sizeof(int), s));
   constexpr int kMaxSmem = 200 * 1024;
-  static bool attr = false;
-  if (!attr) {
-    CPHF_CUDA(cudaFuncSetAttribute(lu_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
-    attr = true;
-  }
+  static PerDevice limit;
+  allow_smem(limit, (const void*)lu_panel_kernel, kMaxSmem);
   for (int64_t k0 = 0; k0 < m; k0 += kLuPanel) {
     const int w = (int)std::min<int64_t>(kLuPanel, m - k0);
     const int64_t bytes = (m - k0) * w * 8, k1 = k0 + w, cols = (m - k1) + nrhs;

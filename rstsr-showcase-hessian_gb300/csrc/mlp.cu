@@ -345,11 +345,8 @@ void mlp_forward(cphf_ctx* c, const float* feat, int64_t n, float* out, bool bf1
 
 float mlp_loss_grad(cphf_ctx* c, const float* feat, const float* target, const int* idx, int64_t n, float* grad) {
   mlp_require(c);
-  static bool attr = false;
-  if (!attr) {
-    CPHF_CUDA(cudaFuncSetAttribute(mlp_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TRAIN_SMEM));
-    attr = true;
-  }
+  static PerDevice smem;
+  allow_smem(smem, (const void*)mlp_grad_kernel, TRAIN_SMEM);
   MlpState& M = *c->mlp;
   const int64_t nblk = div_up(n, BS);
   M.part.ensure((size_t)nblk * (NW + 1) * 4, c->counter());

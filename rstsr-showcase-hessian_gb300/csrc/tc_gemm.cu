@@ -365,16 +365,12 @@ bool tc_available(cphf_ctx* c) {
   cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, c->device);
   cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, c->device);
   if (major != 10 || encode_fn() == nullptr) return false;
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (!pair_available(c->device) ||
-        cudaFuncSetAttribute(tc_wgen_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess) {
-      cudaGetLastError();
-      return false;
-    }
-    attr_set = true;
-  }
-  return true;
+  static PerDevice attr;
+  const bool ok = pair_available(c->device) && attr.once(c->device, [] {
+    return cudaFuncSetAttribute(tc_wgen_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) == cudaSuccess;
+  });
+  if (!ok) cudaGetLastError();
+  return ok;
 }
 
 void tc_prepare_cderi(cphf_ctx* c, DevBuf& hi, DevBuf& lo, int64_t& ldk) {

@@ -1204,19 +1204,18 @@ void launch_batched(cphf_ctx* c, const CUtensorMap& mA, const CUtensorMap& mB, c
   launch_batched_raw<PR, EPI>(c, mA, mB, a, best);
 }
 
-bool res_attr_ok() {
-  static int state = -1;
-  if (state < 0) {
+bool res_attr_ok(int device) {
+  static PerDevice attr;
+  const bool ok = attr.once(device, [] {
     auto set = [](const void* f, int bytes) {
       return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
     };
-    state = set((const void*)tc_tgen_resident_kernel<32>, ResT<32>::SMEM_BYTES) &&
-                    set((const void*)tc_tgen_resident_kernel<64>, ResT<64>::SMEM_BYTES) &&
-                    set((const void*)tc_tgen_resident_kernel<128>, ResT<128>::SMEM_BYTES)
-                ? 1 : 0;
-    if (!state) cudaGetLastError();
-  }
-  return state == 1;
+    return set((const void*)tc_tgen_resident_kernel<32>, ResT<32>::SMEM_BYTES) &&
+           set((const void*)tc_tgen_resident_kernel<64>, ResT<64>::SMEM_BYTES) &&
+           set((const void*)tc_tgen_resident_kernel<128>, ResT<128>::SMEM_BYTES);
+  });
+  if (!ok) cudaGetLastError();
+  return ok;
 }
 // column tile of the resident T generation for nocc columns
 int res_bn(int64_t no) { return no <= 32 ? 32 : no <= 64 ? 64 : 128; }
@@ -1297,14 +1296,13 @@ bool oz_available(cphf_ctx* c) {
   int major = 0;
   cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, c->device);
   if (major != 10 || encode_fn() == nullptr) return false;
-  static bool attr_ok = false, tried = false;
-  if (!tried) {
-    tried = true;
-    attr_ok = set_smem_attr<Exact6>() && set_smem_attr<Exact6c>() && set_smem_attr<Exact6c3>() &&
-              set_smem_attr<Split2>() && set_rho_smem_attr<SHORT_STAGES>() && set_rho_smem_attr<Split2::STAGES>();
-    if (!attr_ok) cudaGetLastError();
-  }
-  return attr_ok;
+  static PerDevice attr;
+  const bool ok = attr.once(c->device, [] {
+    return set_smem_attr<Exact6>() && set_smem_attr<Exact6c>() && set_smem_attr<Exact6c3>() &&
+           set_smem_attr<Split2>() && set_rho_smem_attr<SHORT_STAGES>() && set_rho_smem_attr<Split2::STAGES>();
+  });
+  if (!ok) cudaGetLastError();
+  return ok;
 }
 
 bool oz_supported(const cphf_ctx* c) {
@@ -1624,7 +1622,7 @@ void lp_tgen_planes(cphf_ctx* c, OzState& z, int s, int64_t P0, int64_t npc, int
   tbound_kernel<<<1, 256, 0, c->stream>>>(z.braS.as<unsigned>(), z.spin[s].Omax.as<unsigned>() + P0, npc, mx);
   count_launch();
   launch_t_scale(mx, sA, alpha, scale, c->stream);
-  if (no <= 128 && res_attr_ok()) {
+  if (no <= 128 && res_attr_ok(c->device)) {
     // bra tile resident, all i of a column in one tile of bn columns
     const int bn = res_bn(no);
     const CUtensorMap mO128 = make_map(z.spin[s].O.p, no, no, S2 * naux, ldj, bn, false, 128 / bn);
