@@ -16,14 +16,14 @@ namespace {
 
 struct CounterScope {
   int64_t* prev;
-  std::unique_ptr<LowpState>* parked;
-  explicit CounterScope(cphf_ctx* c) : prev(g_launch_counter), parked(g_parked) {
+  cphf_ctx* ctx;
+  explicit CounterScope(cphf_ctx* c) : prev(g_launch_counter), ctx(g_call_ctx) {
     g_launch_counter = &c->launches;
-    g_parked = &c->lowp_parked;
+    g_call_ctx = c;
   }
   ~CounterScope() {
     g_launch_counter = prev;
-    g_parked = parked;
+    g_call_ctx = ctx;
   }
 };
 

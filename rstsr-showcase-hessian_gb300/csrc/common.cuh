@@ -48,9 +48,9 @@ extern std::atomic<int64_t> g_state_generation;
 inline void bump_generation() { g_state_generation.fetch_add(1, std::memory_order_relaxed); }
 inline int64_t state_generation() { return g_state_generation.load(std::memory_order_relaxed); }
 
-// Frees the memory that the calling thread's context has set aside for its next preparation
-// (lowp_park); false when there is none.
-bool reclaim_parked();
+// Frees memory that the calling thread's context only keeps for later calls: the buffers set aside
+// for its next preparation (lowp_park), the fixed-point GEMM's workspace; false when there is none.
+bool reclaim_spare();
 
 // Owning device allocation; byte size tracked for cphf_ctx_device_bytes.
 struct DevBuf {
@@ -77,11 +77,22 @@ struct DevBuf {
     counter = cnt;
     if (n == 0) return;
     cudaError_t e = cudaMalloc(&p, n);
-    if (e == cudaErrorMemoryAllocation && reclaim_parked()) e = cudaMalloc(&p, n);
+    if (e == cudaErrorMemoryAllocation && reclaim_spare()) e = cudaMalloc(&p, n);
     check_cuda(e, "cudaMalloc(&p, n)");
     bump_generation();
     bytes = n;
     if (counter) *counter += (int64_t)n;
+  }
+  // The same for a buffer that the call can do without: false when there is no memory for it.
+  bool try_ensure(size_t n, int64_t* cnt) {
+    try {
+      ensure(n, cnt);
+    } catch (const Error& e) {
+      if (e.status != CPHF_ERR_OOM) throw;
+      p = nullptr;
+      return false;
+    }
+    return true;
   }
   template <typename T>
   T* as() const { return static_cast<T*>(p); }

@@ -283,7 +283,7 @@ struct FxPlan;
 void gemm64(cphf_ctx* c, const GemmDesc& d);
 double gemm64_us(cphf_ctx* c, const GemmDesc& d);      // its expected time (us)
 // fixed-point product by plan (gemm_fx.cuh); returns the device flag of non-finite operands, which
-// are left to the caller
+// are left to the caller, or null when there was no memory for its digit planes: nothing is computed
 const int* gemm64_fx(cphf_ctx* c, const GemmDesc& d, const FxPlan& fx);
 void gemm32(cphf_ctx* c, const GemmDesc& d);  // float compute, float operands/output
 template <typename TA, typename TB, typename TC>
@@ -328,7 +328,7 @@ void lowp_release(cphf_ctx* c);  // frees the split-precision state
 // takes them over if it has the same sizes and frees them otherwise (as does any allocation of the
 // context that finds no memory).
 void lowp_park(cphf_ctx* c);
-extern thread_local std::unique_ptr<LowpState>* g_parked;  // of the context whose call runs
+extern thread_local cphf_ctx* g_call_ctx;  // the context whose call runs
 
 // Scope in which the FP64 operator (response_mo_fp64) runs in the FP64-accurate arithmetic of
 // the mixed context: mode 0 native FP64, 1 double-float GEMMs, 2 double-float plus the RI-K

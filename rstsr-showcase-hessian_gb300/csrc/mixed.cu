@@ -25,12 +25,14 @@
 namespace cphf {
 
 
-thread_local std::unique_ptr<LowpState>* g_parked = nullptr;
+thread_local cphf_ctx* g_call_ctx = nullptr;
 
-bool reclaim_parked() {
-  if (g_parked == nullptr || !*g_parked) return false;
+bool reclaim_spare() {
+  cphf_ctx* const c = g_call_ctx;
+  if (c == nullptr || (!c->lowp_parked && c->ws_fx.p == nullptr)) return false;
   cudaGetLastError();
-  g_parked->reset();
+  c->lowp_parked.reset();
+  c->ws_fx.release();  // (held by no launch that is still to come: gemm64 takes it anew)
   return true;
 }
 

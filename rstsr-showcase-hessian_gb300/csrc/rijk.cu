@@ -46,15 +46,18 @@ double gemm64_us(cphf_ctx* c, const GemmDesc& d) {
   return gemm_f64_us(d, c->num_sms);
 }
 
-static void run_fx(cphf_ctx* c, const GemmDesc& d, const FxPlan& fx, const int** nonfinite) {
+// false when there is no memory for its digit planes
+static bool run_fx(cphf_ctx* c, const GemmDesc& d, const FxPlan& fx, const int** nonfinite) {
   if (c->fx_err.p == nullptr) {
-    c->fx_err.ensure(sizeof(int), c->counter());
+    if (!c->fx_err.try_ensure(sizeof(int), c->counter())) return false;
     CPHF_CUDA(cudaMemsetAsync(c->fx_err.p, 0, sizeof(int), c->stream));
   }
-  c->ws_fx.ensure(fx.total, c->counter());
+  // (last: an allocation that finds no memory gives this one back)
+  if (!c->ws_fx.try_ensure(fx.total, c->counter())) return false;
   c->fx_used = true;  // the error flag is read at the end of the API call
   ProfScope ps(c, PROF_GEMM_FX, gemm_flops(d), 8.0 * (d.M * d.K + d.K * d.N + d.M * d.N) * d.batch1 * d.batch2);
   CPHF_CUDA(fx_gemm(fx, c->stream, c->ws_fx.p, c->fx_err.as<int>(), c->num_sms, nonfinite));
+  return true;
 }
 
 const int* gemm64_fx(cphf_ctx* c, const GemmDesc& d, const FxPlan& fx) {
@@ -73,12 +76,10 @@ void gemm64(cphf_ctx* c, const GemmDesc& d) {
   // large products on the tensor cores as exact sums of fixed-point digit products (gemm_fx.cu);
   // tensor_cores = 0 keeps every FP64 GEMM on the CUDA cores
   FxPlan fx;
-  if (c->cfg.tensor_cores != 0 && fx_available(c->device) && fx_plan(d, c->num_sms, fx)) {
-    run_fx(c, d, fx, nullptr);
+  if (c->cfg.tensor_cores != 0 && fx_available(c->device) && fx_plan(d, c->num_sms, fx) && run_fx(c, d, fx, nullptr))
     return;
-  }
   const size_t need = gemm_workspace_bytes(d, 8, c->num_sms);
-  if (need) c->ws_gemm.ensure(need, c->counter());
+  if (need) c->ws_gemm.try_ensure(need, c->counter());  // (no memory: one K range)
   if (c->f64_emulate) {
     ProfScope ps(c, PROF_GEMM_F64E, gemm_flops(d), 8.0 * (d.M * d.K + d.K * d.N + d.M * d.N) * d.batch1 * d.batch2);
     CPHF_CUDA(gemm_f64_emulated(d, c->stream, c->ws_gemm.p, c->ws_gemm.bytes, c->num_sms));
@@ -93,7 +94,7 @@ void gemm32(cphf_ctx* c, const GemmDesc& d) { gemm32x<float, float, float>(c, d)
 template <typename TA, typename TB, typename TC>
 void gemm32x(cphf_ctx* c, const GemmDesc& d) {
   const size_t need = gemm_workspace_bytes(d, 4, c->num_sms);
-  if (need) c->ws_gemm.ensure(need, c->counter());
+  if (need) c->ws_gemm.try_ensure(need, c->counter());  // (no memory: one K range)
   ProfScope ps(c, PROF_GEMM_F32, gemm_flops(d), 4.0 * (d.M * d.K + d.K * d.N + d.M * d.N) * d.batch1 * d.batch2);
   CPHF_CUDA((gemm<float, TA, TB, TC>(d, c->stream, c->ws_gemm.p, c->ws_gemm.bytes, c->num_sms)));
 }

@@ -115,7 +115,6 @@ __global__ void gga_sum_kernel(const double* __restrict__ planes, int64_t n, dou
 // faster than four: one set of slicing and GEMM launches, whose tiles fill the last wave together
 // (5600 points, nao 96, 15 occupied x 24: the eight products of an application 0.9 -> 0.6 ms).
 bool gemm_components(cphf_ctx* c, GemmDesc d, double extra_us, int64_t a_b, int64_t b_b, int64_t c_b) {
-  if (c->cfg.tensor_cores == 0 || c->f64_emulate || c->f32_correction) return false;
   const double four = 4.0 * gemm64_us(c, d);
   d.batch1 = 4;
   d.a_b1 = a_b; d.b_b1 = b_b; d.c_b1 = c_b;
@@ -167,9 +166,12 @@ void xc_response_gga(cphf_ctx* c, const T* const* bra, int64_t nb, T* const* out
     if (c->cfg.xc_chunk_points > 0) chunk = c->cfg.xc_chunk_points;
     chunk = std::min<int64_t>(chunk, NG);
     ket_buf.ensure((size_t)4 * chunk * no_max * nb * sizeof(T), c->counter());
-    // rho1 of the spins, then (FP64) the output contraction's four component planes
-    const int64_t rho_all = ns * chunk * nvar * nb;
-    rho_buf.ensure((size_t)(rho_all + (sizeof(T) == 8 ? 4 * nao * no_max * nb : 0)) * sizeof(T), c->counter());
+    // rho1 of the spins, then the output contraction's four component planes where they may be batched
+    // (FP64 on the tensor cores) and there is memory for them
+    const int64_t rho_all = ns * chunk * nvar * nb, planes = 4 * nao * no_max * nb;
+    const bool batched = sizeof(T) == 8 && c->cfg.tensor_cores != 0 && !c->f64_emulate && !c->f32_correction &&
+                         rho_buf.try_ensure((size_t)(rho_all + planes) * sizeof(T), c->counter());
+    if (!batched) rho_buf.ensure((size_t)rho_all * sizeof(T), c->counter());
     T* ket = ket_buf.as<T>();
     T* rho = rho_buf.as<T>();
     for (int64_t g0 = 0; g0 < NG; g0 += chunk) {
@@ -189,7 +191,7 @@ void xc_response_gga(cphf_ctx* c, const T* const* bra, int64_t nb, T* const* out
           d.A = phi + g0; d.a_m = 1; d.a_k = NG;
           d.B = bra[s]; d.b_k = 1; d.b_n = nao;
           d.C = ket; d.c_m = 1; d.c_n = ng;
-          one = gemm_components(c, d, 0.0, NG * nao, 0, ng * N);
+          one = batched && gemm_components(c, d, 0.0, NG * nao, 0, ng * N);
         }
         for (int comp = 0; !one && comp < 4; ++comp) {
           GemmDesc d;  // ket_c = phi_c bra  (pure_eval_rho.rs:283-296)
@@ -219,7 +221,7 @@ void xc_response_gga(cphf_ctx* c, const T* const* bra, int64_t nb, T* const* out
           d.B = ket; d.b_k = 1; d.b_n = ng;
           d.C = rho + rho_all; d.c_m = 1; d.c_n = nao;
           d.alpha = fac;
-          one = gemm_components(c, d, 8.0, NG * nao, ng * N, nao * N);
+          one = batched && gemm_components(c, d, 8.0, NG * nao, ng * N, nao * N);
           if (one) {
             gga_sum_kernel<<<blocks(nao * N), kThreads, 0, c->stream>>>(rho + rho_all, nao * N, written[so] ? 1.0 : 0.0,
                                                                         out[so]);

@@ -426,10 +426,14 @@ void xc_response_grouped(cphf_ctx* c, const T* const* bra, int64_t nb, T* const*
       FxPlan k, o;
       for (int s = 0; s < ns; ++s) route[s] = xc_route(c, ch, c->spin[s].nocc * nb, k, o);
       if (route[0] == XcRoute::dense || route[1] == XcRoute::dense) {
-        c->s_phid.ensure((size_t)(ch.npts * nao) * 8, c->counter());
-        const dim3 grid((unsigned)std::max<int64_t>(1, div_up(4 * (int64_t)c->num_sms, ng)), (unsigned)std::min(ng, 65535));
-        xc_dense_phi_kernel<<<grid, 256, 0, c->stream>>>(gdev + ch.group_off, ng, phi, nao, ch.npts, c->s_phid.as<double>());
-        count_launch();
+        if (c->s_phid.try_ensure((size_t)(ch.npts * nao) * 8, c->counter())) {
+          const dim3 grid((unsigned)std::max<int64_t>(1, div_up(4 * (int64_t)c->num_sms, ng)), (unsigned)std::min(ng, 65535));
+          xc_dense_phi_kernel<<<grid, 256, 0, c->stream>>>(gdev + ch.group_off, ng, phi, nao, ch.npts, c->s_phid.as<double>());
+          count_launch();
+        } else {  // no memory for the dense values
+          for (XcRoute& r : route)
+            if (r == XcRoute::dense) r = XcRoute::grouped;
+        }
       }
     }
     for (int s = 0; s < ns; ++s) {

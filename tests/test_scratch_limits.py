@@ -1,0 +1,63 @@
+"""FP64 calls with little device memory left: the fixed-point products' scratch is not needed to answer."""
+
+import numpy as np
+import pytest
+
+from conftest import rel_err
+from cphf_gb300 import Context, synth
+
+pytestmark = pytest.mark.gpu
+
+RIJK = dict(nao=200, naux=600, nocc=(20,), natm=18, decay=12.0)
+LDA = dict(nao=83, naux=40, nocc=(11, 10), natm=6, decay=12.0, grid=True, points=(900, 1201), window=27)
+
+
+class _Filled:
+    """All device memory but about 24 MiB held by torch."""
+
+    def __enter__(self):
+        import torch
+        torch.cuda.empty_cache()
+        self.held = []
+        for keep in (1 << 30, 256 << 20, 24 << 20):
+            n = torch.cuda.mem_get_info()[0] - keep
+            if n > 0:
+                self.held.append(torch.empty(n, dtype=torch.uint8, device="cuda"))
+        assert torch.cuda.mem_get_info()[0] < 64 << 20
+
+    def __exit__(self, *exc):
+        import torch
+        self.held = None
+        torch.cuda.empty_cache()
+
+
+def _context(s, kind):
+    ctx = Context(tensor_cores=0)
+    ctx.set_cderi(s.cderi, s.scale_j, s.scale_k)
+    if kind == "lda":
+        ctx.set_grid(s.grid.ao, s.grid.weights, s.grid.fxc, s.nspin, s.grid.atom_offsets)
+    elif kind == "sigma":
+        ao, fx = synth.make_mgga_grid(s.grid, "sigma", seed=3, nspin=s.nspin)
+        ctx.set_grid_ex("sigma", ao, s.grid.weights, fx, s.nspin, s.grid.atom_offsets)
+    one = lambda v: v if s.nspin == 2 else v[0]
+    ctx.make_response_preparation(one(s.mo_coeff), one(s.mo_occ), one(s.mo_energy))
+    return ctx
+
+
+@pytest.mark.parametrize("dims,kind", [(RIJK, "rijk"), (LDA, "lda"), (LDA, "sigma")])
+def test_no_memory_for_digit_planes(dims, kind):
+    s = synth.make_system(dims, seed=4)
+    ctx = _context(s, kind)
+    rng = np.random.default_rng(1)
+    bra = [rng.standard_normal((s.nao, n, 54)) for n in s.nocc]
+    bra = bra if s.nspin == 2 else bra[0]
+    plugin = "rijk" if kind == "rijk" else "xc"
+    ref = ctx.get_response_bra(bra, plugin=plugin)  # (the native route's scratch is in place now)
+    ctx.set_config(tensor_cores=1)
+    with _Filled():
+        got = ctx.get_response_bra(bra, plugin=plugin)
+    ctx.profile(True)
+    ctx.get_response_bra(bra, plugin=plugin)
+    assert ctx.profile_report()["gemm_fp64_tcgen05"]["launches"] > 0  # (with memory the digits are used)
+    for a, b in zip(got if s.nspin == 2 else [got], ref if s.nspin == 2 else [ref]):
+        assert rel_err(a, b) < 1e-12
