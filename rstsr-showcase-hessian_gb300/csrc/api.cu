@@ -236,7 +236,7 @@ cphf_status cphf_ctx_set_config(cphf_ctx* c, const cphf_config* cfg) {
 
 const char* cphf_last_error(const cphf_ctx* c) { return c ? c->last_error.c_str() : "null context"; }
 void* cphf_ctx_stream(const cphf_ctx* c) { return c ? (void*)c->stream : nullptr; }
-int64_t cphf_ctx_device_bytes(const cphf_ctx* c) { return c ? c->device_bytes : 0; }
+int64_t cphf_ctx_device_bytes(const cphf_ctx* c) { return c ? c->device_bytes.load() : 0; }
 int64_t cphf_ctx_kernel_launches(const cphf_ctx* c) { return c ? c->launches : 0; }
 
 int32_t cphf_ctx_tensor_cores_active(const cphf_ctx* c) {
@@ -308,7 +308,7 @@ static void install_cderi(cphf_ctx* c, int64_t nao, int64_t naux, double scale_j
   c->has_rijk = true;
   c->prepared = false;
   if (c->lowp && (c->lowp->shape[0] != nao || c->lowp->shape[1] != naux)) lowp_release(c);
-  else lowp_park(c);
+  else lowp_park(c, false);
   CPHF_CUDA(cudaStreamSynchronize(c->stream));
 }
 
@@ -539,7 +539,7 @@ cphf_status cphf_prepare(cphf_ctx* c, int32_t nspin, const double* const* mo_coe
     if (c->has_rijk) rijk_prepare(c);
     if (c->has_xc) xc_prepare(c);
     if (c->cfg.precision == CPHF_PRECISION_MIXED) {
-      lowp_park(c);
+      lowp_park(c, true);
       lowp_prepare(c);
     } else {
       lowp_release(c);

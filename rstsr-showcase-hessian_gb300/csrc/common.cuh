@@ -48,15 +48,18 @@ extern std::atomic<int64_t> g_state_generation;
 inline void bump_generation() { g_state_generation.fetch_add(1, std::memory_order_relaxed); }
 inline int64_t state_generation() { return g_state_generation.load(std::memory_order_relaxed); }
 
-// Frees memory that the calling thread's context only keeps for later calls: the buffers set aside
-// for its next preparation (lowp_park), the fixed-point GEMM's workspace; false when there is none.
+// Frees memory that is only kept for later calls: the buffers that contexts of the current device
+// have set aside for their next preparation (lowp_park) and the fixed-point GEMM's workspace of the
+// calling thread's context; false when there is none.
 bool reclaim_spare();
+
+using ByteCount = std::atomic<int64_t>;  // (reclaim_spare frees buffers of other threads' contexts)
 
 // Owning device allocation; byte size tracked for cphf_ctx_device_bytes.
 struct DevBuf {
   void* p = nullptr;
   size_t bytes = 0;
-  int64_t* counter = nullptr;
+  ByteCount* counter = nullptr;
   DevBuf() = default;
   DevBuf(const DevBuf&) = delete;
   DevBuf& operator=(const DevBuf&) = delete;
@@ -71,7 +74,7 @@ struct DevBuf {
     bytes = 0;
   }
   // Grow to at least n bytes (contents are not preserved when growing).
-  void ensure(size_t n, int64_t* cnt) {
+  void ensure(size_t n, ByteCount* cnt) {
     if (n <= bytes && p) return;
     release();
     counter = cnt;
@@ -84,7 +87,7 @@ struct DevBuf {
     if (counter) *counter += (int64_t)n;
   }
   // The same for a buffer that the call can do without: false when there is no memory for it.
-  bool try_ensure(size_t n, int64_t* cnt) {
+  bool try_ensure(size_t n, ByteCount* cnt) {
     try {
       ensure(n, cnt);
     } catch (const Error& e) {

@@ -205,7 +205,7 @@ struct cphf_ctx {
   int num_sms = 152;
   cudaStream_t stream = nullptr;
   std::string last_error;
-  int64_t device_bytes = 0;
+  cphf::ByteCount device_bytes{0};
   int64_t launches = 0;
 
   // RI-JK plugin
@@ -242,7 +242,8 @@ struct cphf_ctx {
   cphf::DevBuf k_xs, k_ax, k_h, k_g, k_b, k_xacc, k_x1, k_axt, k_coef, k_ip, k_keep, k_part, k_idx,
       k_hw, k_info, k_r, k_norm, k_finite, k_pre;
 
-  std::unique_ptr<cphf::LowpState> lowp, lowp_parked;
+  std::unique_ptr<cphf::LowpState> lowp;
+  std::unique_ptr<cphf::LowpState> lowp_parked;  // under mixed.cu's lock
   std::unique_ptr<cphf::MlpState> mlp;
   cphf::Profiler prof;
   bool f64_emulate = false;  // route the FP64 GEMMs through the double-float kernel
@@ -251,7 +252,7 @@ struct cphf_ctx {
   bool f32_correction = false; // FP64 GEMMs of a correction-precision application run in FP32
   bool oz_xc = false;        // FP64 XC response on the tensor cores (exact BF16 slices)
 
-  int64_t* counter() { return &device_bytes; }
+  cphf::ByteCount* counter() { return &device_bytes; }
 };
 
 namespace cphf {
@@ -325,9 +326,11 @@ double fp64_residual(cphf_ctx* c, const double* b, const double* x, int64_t nset
 void lowp_prepare(cphf_ctx* c);
 void lowp_release(cphf_ctx* c);  // frees the split-precision state
 // Invalidates the split-precision state and sets its buffers aside for the next preparation, which
-// takes them over if it has the same sizes and frees them otherwise (as does any allocation of the
-// context that finds no memory).
-void lowp_park(cphf_ctx* c);
+// takes them over if it has the same sizes and frees them otherwise.  Until then they may be wanted
+// elsewhere: any allocation of a context of the device that finds no memory frees them, and they are
+// kept only while a quarter of the device's memory stays free (unless the preparation follows at
+// once): other allocators of the process cannot ask for them.
+void lowp_park(cphf_ctx* c, bool at_once);
 extern thread_local cphf_ctx* g_call_ctx;  // the context whose call runs
 
 // Scope in which the FP64 operator (response_mo_fp64) runs in the FP64-accurate arithmetic of

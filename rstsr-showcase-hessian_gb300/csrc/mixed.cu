@@ -11,6 +11,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <mutex>
 #include <vector>
 
 #include "ctx.cuh"
@@ -27,24 +28,52 @@ namespace cphf {
 
 thread_local cphf_ctx* g_call_ctx = nullptr;
 
+// Contexts with parked buffers.  The lock covers lowp_parked of every context, also while the buffers
+// are freed: a context cannot go away meanwhile (its destruction takes the lock in lowp_release).
+static std::mutex g_park_mu;
+static std::vector<cphf_ctx*> g_park_ctxs;
+
+static std::unique_ptr<LowpState> take_parked(cphf_ctx* c) {
+  std::lock_guard<std::mutex> lock(g_park_mu);
+  g_park_ctxs.erase(std::remove(g_park_ctxs.begin(), g_park_ctxs.end(), c), g_park_ctxs.end());
+  return std::move(c->lowp_parked);
+}
+
 bool reclaim_spare() {
-  cphf_ctx* const c = g_call_ctx;
-  if (c == nullptr || (!c->lowp_parked && c->ws_fx.p == nullptr)) return false;
   cudaGetLastError();
-  c->lowp_parked.reset();
-  c->ws_fx.release();  // (held by no launch that is still to come: gemm64 takes it anew)
-  return true;
+  bool any = false;
+  int dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess) {
+    std::lock_guard<std::mutex> lock(g_park_mu);
+    for (size_t i = g_park_ctxs.size(); i-- > 0;) {
+      if (g_park_ctxs[i]->device != dev) continue;
+      g_park_ctxs[i]->lowp_parked.reset();
+      g_park_ctxs.erase(g_park_ctxs.begin() + i);
+      any = true;
+    }
+  }
+  if (cphf_ctx* const c = g_call_ctx; c != nullptr && c->ws_fx.p != nullptr) {
+    c->ws_fx.release();  // (held by no launch that is still to come: gemm64 takes it anew)
+    any = true;
+  }
+  return any;
 }
 
 void lowp_release(cphf_ctx* c) {
   c->lowp.reset();
-  c->lowp_parked.reset();
+  take_parked(c);
 }
 
 // A new geometry of a molecule repeats the sizes of the last one; freeing and allocating the planes
 // and chunks took 19 of its 85 ms at nao 400 (18 GB).
-void lowp_park(cphf_ctx* c) {
+void lowp_park(cphf_ctx* c, bool at_once) {
   if (!c->lowp) return;
+  size_t free_b = 0, total_b = 0;
+  if (!at_once && (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || free_b < total_b / 4)) {
+    cudaGetLastError();
+    lowp_release(c);
+    return;
+  }
   LowpState& L = *c->lowp;
   L.drop_graphs();
   L.graphs_off = false;
@@ -54,7 +83,9 @@ void lowp_park(cphf_ctx* c) {
     for (OzSpin& s : z->spin) s.ready = false;
   }
   L.xctc.ready = L.xctc64.ready = false;
+  std::lock_guard<std::mutex> lock(g_park_mu);
   c->lowp_parked = std::move(c->lowp);
+  if (std::find(g_park_ctxs.begin(), g_park_ctxs.end(), c) == g_park_ctxs.end()) g_park_ctxs.push_back(c);
 }
 
 void lowp_prepare(cphf_ctx* c) {
@@ -63,8 +94,10 @@ void lowp_prepare(cphf_ctx* c) {
                              c->nspin};
   for (int s = 0; s < c->nspin; ++s) shape.insert(shape.end(), {c->spin[s].nmo, c->spin[s].nocc});
   bool fresh = false;
-  if (!c->lowp && c->lowp_parked && c->lowp_parked->shape == shape) c->lowp = std::move(c->lowp_parked);
-  c->lowp_parked.reset();
+  {
+    std::unique_ptr<LowpState> parked = take_parked(c);
+    if (!c->lowp && parked && parked->shape == shape) c->lowp = std::move(parked);
+  }
   if (!c->lowp) {
     c->lowp.reset(new LowpState());
     fresh = true;

@@ -61,3 +61,46 @@ def test_no_memory_for_digit_planes(dims, kind):
     assert ctx.profile_report()["gemm_fp64_tcgen05"]["launches"] > 0  # (with memory the digits are used)
     for a, b in zip(got if s.nspin == 2 else [got], ref if s.nspin == 2 else [ref]):
         assert rel_err(a, b) < 1e-12
+
+
+SMALL = dict(nao=96, naux=150, nocc=(12,), natm=3, decay=12.0)
+MIXED = dict(nao=200, naux=600, nocc=(20,), natm=6, decay=12.0)
+
+
+def _mixed(s, ctx=None):
+    ctx = ctx or Context(precision="mixed")
+    ctx.set_cderi(s.cderi, s.scale_j, s.scale_k)
+    ctx.make_response_preparation(s.mo_coeff[0], s.mo_occ[0], s.mo_energy[0])
+    return ctx
+
+
+def test_parked_buffers_serve_another_context():
+    """The buffers that one context keeps for its next preparation are freed for another's allocation."""
+    s, t = synth.make_system(MIXED, seed=1), synth.make_system(SMALL, seed=2)
+    ctx, other = _mixed(s), Context()
+    ref = ctx.solve_dimless_cphf(s.rhs[0])
+    ctx.set_cderi(s.cderi, s.scale_j, s.scale_k)
+    kept = ctx.device_bytes
+    with _Filled():
+        _mixed(t, other)
+        # (the buffers that other now needs in earnest come to more than the memory left)
+        other.krylov_block(np.asfortranarray(0.1 * np.eye(40)), np.ones((40, 2)))
+        big = np.zeros((3000, 3000), order="F")
+        other.krylov_block(big, np.ones((3000, 1)))  # 72 MB
+        assert ctx.device_bytes < kept
+    ctx.make_response_preparation(s.mo_coeff[0], s.mo_occ[0], s.mo_energy[0])
+    assert np.abs(ctx.solve_dimless_cphf(s.rhs[0]) - ref).max() < 1e-7  # (residual 1e-8)
+
+
+def test_buffers_are_parked_only_while_memory_is_plenty():
+    s = synth.make_system(MIXED, seed=1)
+    ctx = _mixed(s)
+    ctx.solve_dimless_cphf(s.rhs[0])
+    held = ctx.device_bytes
+    ctx.set_cderi(s.cderi, s.scale_j, s.scale_k)
+    assert ctx.device_bytes == held
+    ctx = _mixed(s)
+    ctx.solve_dimless_cphf(s.rhs[0])
+    with _Filled():
+        ctx.set_cderi(s.cderi, s.scale_j, s.scale_k)
+        assert ctx.device_bytes < held // 2
