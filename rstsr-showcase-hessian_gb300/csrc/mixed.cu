@@ -93,15 +93,11 @@ void lowp_prepare(cphf_ctx* c) {
                              c->xc_den,    c->xc_nvar, c->cfg.tensor_cores, c->cfg.aux_chunk, c->cfg.xc_chunk_points,
                              c->nspin};
   for (int s = 0; s < c->nspin; ++s) shape.insert(shape.end(), {c->spin[s].nmo, c->spin[s].nocc});
-  bool fresh = false;
   {
     std::unique_ptr<LowpState> parked = take_parked(c);
     if (!c->lowp && parked && parked->shape == shape) c->lowp = std::move(parked);
   }
-  if (!c->lowp) {
-    c->lowp.reset(new LowpState());
-    fresh = true;
-  }
+  if (!c->lowp) c->lowp.reset(new LowpState());
   LowpState& L = *c->lowp;
   L.shape = shape;
   const int64_t nao = c->nao, naux = c->naux;
@@ -149,13 +145,15 @@ void lowp_prepare(cphf_ctx* c) {
     }
   }
   // Chunk budget of the K term's T / W intermediates: up to 8 GiB, at most a quarter of the
-  // memory still free once the resident operand planes are in place (fewer, longer launches).
-  if (!fresh) return;  // the chunks in place keep their size
+  // memory still free, or taken by the chunks of the last preparation, once the resident operand planes
+  // are in place (fewer, longer launches).
   size_t free_b = 0, total_b = 0;
-  if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess)
+  if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) {
+    for (const DevBuf* b : {&L.s_Thi, &L.s_Tlo, &L.oz.T, &L.oz.B, &L.oz.W, &L.oz.Ws, &L.lp.Ws}) free_b += b->bytes;
     L.budget = std::max<int64_t>(int64_t(256) << 20, std::min<int64_t>(int64_t(8) << 30, (int64_t)(free_b / 4)));
-  else
+  } else {
     cudaGetLastError();
+  }
 }
 
 static int64_t k_chunk_lowp(const cphf_ctx* c, int64_t no, int64_t nb) {

@@ -13,17 +13,20 @@ LDA = dict(nao=83, naux=40, nocc=(11, 10), natm=6, decay=12.0, grid=True, points
 
 
 class _Filled:
-    """All device memory but about 24 MiB held by torch."""
+    """All device memory but about ``left`` bytes (24 MiB) held by torch."""
+
+    def __init__(self, left=24 << 20):
+        self.left = left
 
     def __enter__(self):
         import torch
         torch.cuda.empty_cache()
         self.held = []
-        for keep in (1 << 30, 256 << 20, 24 << 20):
-            n = torch.cuda.mem_get_info()[0] - keep
+        for keep in (1 << 30, 256 << 20, 0):
+            n = torch.cuda.mem_get_info()[0] - self.left - keep
             if n > 0:
                 self.held.append(torch.empty(n, dtype=torch.uint8, device="cuda"))
-        assert torch.cuda.mem_get_info()[0] < 64 << 20
+        assert torch.cuda.mem_get_info()[0] < self.left + (40 << 20)
 
     def __exit__(self, *exc):
         import torch
@@ -104,3 +107,23 @@ def test_buffers_are_parked_only_while_memory_is_plenty():
     with _Filled():
         ctx.set_cderi(s.cderi, s.scale_j, s.scale_k)
         assert ctx.device_bytes < held // 2
+
+
+def test_chunks_follow_the_memory_of_each_preparation():
+    """Prepared while memory was short, a context works in small chunks; prepared again, as a fresh one."""
+    s = synth.make_system(dict(MIXED, natm=18), seed=1)
+    mo1 = np.random.default_rng(2).standard_normal((s.nao, 20, 54))
+
+    def launches(ctx):
+        ctx.response_dimless_cphf_lowp(mo1)  # (the first call of a shape also tunes its launches)
+        before = ctx.kernel_launches
+        ctx.response_dimless_cphf_lowp(mo1)
+        return ctx.kernel_launches - before
+
+    ctx = Context(precision="mixed")
+    ctx.set_cderi(s.cderi, s.scale_j, s.scale_k)
+    with _Filled(left=3 << 29):  # planes and chunks: T alone is 0.6 GB in one chunk
+        _mixed(s, ctx)
+        short = launches(ctx)
+    again, fresh = launches(_mixed(s, ctx)), launches(_mixed(s))
+    assert again == fresh < short
