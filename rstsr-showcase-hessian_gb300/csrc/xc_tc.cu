@@ -34,6 +34,7 @@
 #include "kernels.cuh"
 #include "slices.cuh"
 #include "tc_ozaki.cuh"
+#include "tc_pair.cuh"
 #include "xc_grouped.cuh"
 #include "xc_tc.cuh"
 
@@ -388,16 +389,17 @@ void xc_tc(cphf_ctx* c, XcTcState& X, OzState& z, const typename XcOps<PR>::T* p
                       X.bscale[s].as<double>(), re, err);
         }
       } else {
-        // GEMM 1 per batch: ket[p - g0, :] = phi[p, win] bra[win, :] (one K range: stored)
+        // GEMM 1 per batch: ket[p - g0, :] = phi[p, win] bra[win, :], stored; a window beyond the exact
+        // sums of one K range (3072 AOs) accumulates its ranges into zeros
         for (int64_t b = ch.b0; b < ch.b1; ++b) {
           const XcTcBatch& x = X.hb[b];
           if (x.npts == 0) continue;
-          if (x.nwin == 0) {
+          const bool store = x.nwin > 0 && div_up(x.kw, 32) <= PAIR_EXACT_KB;
+          if (!store)
             CPHF_CUDA(cudaMemset2DAsync(ket[s] + (x.g0 - g0), npts * sizeof(T), 0, x.npts * sizeof(T), N, st));
-            continue;
-          }
+          if (x.nwin == 0) continue;
           XcOps<PR>::gemm(c, phiB, x.g0, B, x.lo8, x.npts, N, x.kw, X.phiB_scale.as<double>() + x.g0,
-                          X.bscale[s].as<double>(), ket[s] + (x.g0 - g0), npts, err, true);
+                          X.bscale[s].as<double>(), ket[s] + (x.g0 - g0), npts, err, store);
         }
         launch_xc_rho<T>(aobra[s] + g0, ngrids, ket[s], npts, no, nb, rho_s, npts, st);
       }
