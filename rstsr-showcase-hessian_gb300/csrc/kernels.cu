@@ -754,7 +754,7 @@ void launch_residual_norms(const double* b, const double* x, const double* ax, d
 // partial dot products, the coefficients and the barrier's counter
 int64_t mgs_partials_size(int64_t n, int64_t m) {
   const int64_t mm = std::max<int64_t>(m, 1);
-  return kMgsPanel * mm * (std::min<int64_t>(kMgsMaxBlocks, div_up(n, 32)) + 1) + 4;
+  return kMgsPanel * mm * (std::max<int64_t>(1, std::min<int64_t>(kMgsMaxBlocks, div_up(n, 32))) + 1) + 4;
 }
 
 void launch_mgs(double* V, int64_t n, int64_t m, double lindep, double* ip, int* keep, double* partials, int num_sms,
@@ -765,8 +765,8 @@ void launch_mgs(double* V, int64_t n, int64_t m, double lindep, double* ip, int*
   a.V = V;
   a.n = n;
   a.m = m;
-  a.rows = div_up(n, nblk);
-  nblk = div_up(n, a.rows);
+  a.rows = std::max<int64_t>(1, div_up(n, nblk));  // (n = 0, no occupied orbital: one block without rows)
+  nblk = std::max<int64_t>(1, div_up(n, a.rows));
   a.stage = std::min(a.rows, kMgsStage);
   a.lindep = lindep;
   a.ip = ip;
