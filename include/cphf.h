@@ -72,9 +72,13 @@ typedef struct cphf_config {
   int64_t aux_chunk;         /* aux functions per K-term chunk (default 0 = automatic) */
   int32_t tensor_cores;      /* mixed: 1 = tcgen05 split-FP16 K term (default), 0 = FP32 CUDA cores.
                                 FP64 GEMMs (either precision): 1 = large ones on the tensor cores as exact
-                                sums of 62-bit fixed-point digit products, rounded to FP64 once (error
-                                2^-62 |a||b| plus one rounding, below that of a chain of FP64 FMAs);
-                                0 = every one on the FP64 CUDA cores */
+                                sums of products of 62-bit fixed-point digits, relative to the maximum of
+                                each row of A and column of B.  The error of an element of a K-term
+                                product is at most K 2^-57 max|a| max|b| (maxima of its row and column)
+                                plus a rounding per K range: below that of a chain of FP64 FMAs unless
+                                its large factors all meet factors some 2^-9 or less of their maxima, whose
+                                low bits are lost (below 2^-62 of the maximum all of them);
+                                0 = every one on the FP64 CUDA cores, accurate to sum |a||b| */
   int32_t verify_residual;   /* mixed: how the residual of every correction after the first is obtained and
                                 convergence decided.  0 = updated with the split-precision operator,
                                 r -= (I + A_lowp) d (no FP64-accurate application);  1 = recomputed with

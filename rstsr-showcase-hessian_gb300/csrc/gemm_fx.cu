@@ -10,19 +10,24 @@
 // rounded to F = round(v 2^BITS), BITS = 8 (S - 1) + 6, and cut into S balanced base-256 digits
 // F = sum_t q_t 256^(S-1-t), |q_0| <= 64, q_t in [-128, 127], each exact in BF16.  With S = 8
 // (62 bits) every FP64 element within 2^-9 of its row's maximum is represented exactly, all
-// others to 2^-63 of that maximum.  The products of digits t + u <= S - 1 are formed (36 for
-// S = 8); what is dropped is below 2^-63 of the maxima's product.
+// others to 2^-63 of the power of two above that maximum: an element 2^-40 of the maximum keeps 22 bits.
+// The products of digits t + u <= S - 1 are formed (36 for S = 8); the seven pairs with t + u = 8
+// that are dropped come to at most 7 2^-62 of the two powers of two a product (to 2^-62 for random digits).
 // Accumulation.  Products of one weight g = t + u share one FP32 accumulator in TMEM (S x 64 of
 // the 512 columns).  Over 64 k (more for the leading weights, group_kb) their integer sum stays
 // below 2^23, so the FP32 sums are exact; then the epilogue adds them as integers into two 64-bit
-// registers per element (weights 0-3 and 4-7).  The sum over all of K is therefore exact and is
-// rounded to FP64 once, at the end, with integer arithmetic (an FP64 instruction per element
-// and group would cost more than the MMAs of a round).
+// registers per element (weights 0-3 and 4-7).  The sum of these products over a K range is therefore
+// exact and is rounded to FP64 once, at the end, with integer arithmetic (an FP64 instruction per
+// element and group would cost more than the MMAs of a round); the sums of several K ranges (at
+// most 64) are then added in FP64.
 //
-// Error against 64 bits: 2^-62 |a||b| normwise, plus one rounding of the result, instead of the
-// ~2^-53 per step of a chain of FMAs.  Measured (max error / sum |a||b|; fixed point, FMAs):
+// Error: at most K 2^-57 max_k |A(m, k)| max_k |B(k, n)| (for random digits about sqrt(K) 2^-60 of
+// it), plus a rounding per K range and per addition of ranges.  A chain of FMAs errs by ~2^-53 of sum |a||b|
+// a step instead: the digits are the more accurate where that sum is above ~2^-9 of the maxima's product,
+// the less accurate for an element whose large factors all meet small ones.
+// Measured (max error / sum |a||b|; fixed point, FMAs):
 // Gaussian 300 x 200 x 500: 1.1e-17, 2.4e-16; entries over 12 octaves, K = 36000: 4.7e-17, 1.1e-15;
-// K = 17: 1.1e-16, 3.8e-16.  The bound is normwise: where large entries of A meet small ones of B
+// K = 17: 1.1e-16, 3.8e-16.  Where large entries of A meet small ones of B
 // throughout (the Krylov basis, whose vectors shrink, and its growing coefficients; a triangular
 // solve), GemmDesc::k_balance divides A(:, k) and multiplies B(k, :) by a power of two first.
 //
@@ -308,7 +313,8 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map
       : "memory");
 }
 
-// (hi 2^32 + lo) 2^e rounded to nearest FP64 (ties to even), in branch-free integer arithmetic;
+// (hi 2^32 + lo) 2^e rounded to nearest FP64, in branch-free integer arithmetic (from its leading 64
+// bits: to 2^-11 of the last place, ties among them to even);
 // EDGE: also for results outside the normal range of FP64.
 template <bool EDGE>
 __device__ __forceinline__ double fx_round(long long hi, long long lo, int e, unsigned flip) {
