@@ -254,13 +254,29 @@ __global__ void __launch_bounds__(kMgsThreads) mgs_kernel(MgsArgs a) {
   }
   __syncthreads();
   for (int64_t j = wid; j < m; j += kMgsWarps) {
-    double acc[B] = {0.0, 0.0, 0.0, 0.0};
-    for (int64_t r = lane; r < len; r += 32) {
+    // four sums a lane: shorter chains round less (these columns may be the most correlated ones)
+    double acc[B] = {0.0, 0.0, 0.0, 0.0}, part[3][B] = {};
+    int64_t r = lane;
+    for (; r + 96 < len; r += 128) {
+      double v[4];
+#pragma unroll
+      for (int h = 0; h < 4; ++h) v[h] = Vb[r + 32 * h + n * j];
+#pragma unroll
+      for (int q = 0; q < B; ++q)
+        if (q < w) {
+          acc[q] = fma(v[0], panel(cur, 0, q, r), acc[q]);
+#pragma unroll
+          for (int h = 1; h < 4; ++h) part[h - 1][q] = fma(v[h], panel(cur, 0, q, r + 32 * h), part[h - 1][q]);
+        }
+    }
+    for (; r < len; r += 32) {
       const double v = Vb[r + n * j];
 #pragma unroll
       for (int q = 0; q < B; ++q)
         if (q < w) acc[q] = fma(v, panel(cur, 0, q, r), acc[q]);
     }
+#pragma unroll
+    for (int q = 0; q < B; ++q) acc[q] = (acc[q] + part[0][q]) + (part[1][q] + part[2][q]);
     publish(acc, j, w);
   }
   while (true) {
