@@ -92,7 +92,6 @@ void require_prepared(cphf_ctx* c) {
 }
 
 int64_t bra_elems(cphf_ctx* c, int s, int64_t nprop) { return c->nao * c->spin[s].nocc * nprop; }
-int64_t mo_elems(cphf_ctx* c, int s, int64_t nprop) { return c->spin[s].nmo * c->spin[s].nocc * nprop; }
 
 // Staging of spin-resolved arrays into one device buffer; returns per-spin device pointers.
 void stage_in(cphf_ctx* c, DevBuf& buf, const double* const* src, const std::vector<int64_t>& elems,

@@ -47,7 +47,6 @@
 // Every mbarrier wait is bounded; on expiry the kernel raises the error flag and returns.
 #include <cuda.h>
 #include <cuda_bf16.h>
-#include <cudaTypedefs.h>
 
 #include <algorithm>
 #include <cmath>
@@ -56,6 +55,7 @@
 
 #include "common.cuh"
 #include "gemm_fx.cuh"
+#include "tc_map.cuh"
 #include "tc_ptx.cuh"
 
 namespace cphf {
@@ -584,21 +584,6 @@ __global__ void __launch_bounds__(256) fx_reduce_kernel(FxArgs a, int64_t batch)
 }
 
 // ---- host side ------------------------------------------------------------------------------
-PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-    else
-      cudaGetLastError();
-  });
-  return fn;
-}
-
 // 4-D map {K, rows, batch, S} of BF16 planes, box {32, box_rows, 1, S}, 64B swizzle
 bool make_map(CUtensorMap& m, const void* base, int64_t K, int64_t rows, int64_t batch, int64_t ldk, int S, int box_rows) {
   std::memset(&m, 0, sizeof(m));

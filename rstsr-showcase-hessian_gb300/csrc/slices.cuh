@@ -13,7 +13,7 @@ namespace cphf {
 // Operand representations: exact BF16 slices (FP64-accurate residual) and split FP16 hi/lo
 // (the inner solves' operator).  EOFF: exponent offset of the stored planes (x 2^(EOFF - e)).
 struct Exact6 {
-  static constexpr int S = 6, NACC = 4, EOFF = 0, STAGES = 2;
+  static constexpr int S = 6, NACC = 4, EOFF = 0;
   static constexpr bool BF16 = true;
   using Elem = __nv_bfloat16;
 };
@@ -25,19 +25,24 @@ struct Exact6 {
 // accumulation bounds; with NS = 3 the fourth accumulator stays unused.
 template <int NS>
 struct ExactC {
-  // split-K stages of 16 KB per plane pair: 3 x 64 KB (NS = 4) or 4 x 48 KB (NS = 3), so the
-  // fewer products per stage still cover the loads' latency
-  static constexpr int S = NS, NACC = 4, EOFF = 0, STAGES = NS == 3 ? 4 : 3;
+  static constexpr int S = NS, NACC = 4, EOFF = 0;
   static constexpr bool BF16 = true;
   using Elem = __nv_bfloat16;
 };
 using Exact6c = ExactC<4>;
 using Exact6c3 = ExactC<3>;
 struct Split2 {
-  static constexpr int S = 2, NACC = 1, EOFF = 14, STAGES = 6;
+  static constexpr int S = 2, NACC = 1, EOFF = 14;
   static constexpr bool BF16 = false;
   using Elem = __half;
 };
+
+// s + e = a + b exactly
+__device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
+  s = a + b;
+  const float bb = s - a;
+  e = (a - (s - bb)) + (b - bb);
+}
 
 // ---- slicing (integer arithmetic on the bit patterns; the FP64 pipe is not used) ----------
 // |x| as an ordered integer key (non-negative floats order like their bit patterns)

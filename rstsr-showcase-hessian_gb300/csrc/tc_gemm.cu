@@ -14,17 +14,16 @@
 // cderi, the chunking over aux functions and the W generation.
 #include <cuda.h>
 #include <cuda_fp16.h>
-#include <cudaTypedefs.h>
 
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <mutex>
 
 #include "kernels.cuh"
 #include "slices.cuh"
 #include "tc_gemm.cuh"
 #include "tc_pair.cuh"
+#include "tc_map.cuh"
 #include "tc_ptx.cuh"
 
 namespace cphf {
@@ -317,21 +316,6 @@ __global__ void t_scale_kernel(const unsigned* mx, float sA, float alpha, float*
 }
 
 // ---- host side ---------------------------------------------------------------------------
-PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-    else
-      cudaGetLastError();
-  });
-  return fn;
-}
-
 // 3-D FP16 tensor map: dims {K (= nao), rows, planes}, row stride ldk elements, box {64, rows, 1},
 // 128B swizzle.
 CUtensorMap make_map(const void* base, int64_t K, int64_t rows, int64_t depth, int64_t ldk, int box_rows) {
@@ -349,8 +333,6 @@ CUtensorMap make_map(const void* base, int64_t K, int64_t rows, int64_t depth, i
   if (r != CUDA_SUCCESS) throw Error(CPHF_ERR_CUDA, "cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")");
   return m;
 }
-
-unsigned grid_for(int64_t total) { return (unsigned)std::max<int64_t>(1, std::min<int64_t>(div_up(total, 256), 1 << 20)); }
 
 }  // namespace
 

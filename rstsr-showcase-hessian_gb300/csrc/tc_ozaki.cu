@@ -38,7 +38,6 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
-#include <cudaTypedefs.h>
 
 #include <algorithm>
 #include <cmath>
@@ -53,6 +52,7 @@
 #include "tc_ozaki.cuh"
 #include "tc_pair.cuh"
 #include "slices.cuh"
+#include "tc_map.cuh"
 #include "tc_ptx.cuh"
 
 namespace cphf {
@@ -62,11 +62,12 @@ using namespace tcx;
 constexpr int BM = 128, BK = 32;
 constexpr int KMAX = 3072;         // exactness bound of the K range of one CTA
 constexpr int KB_PER_CTA = KMAX / BK;
-constexpr int SHORT_STAGES = 3;    // split-FP16 stages for K ranges of a few blocks (two CTAs per SM)
+constexpr int RHO_STAGES = 6;      // stages of tc_rho_kernel,
+constexpr int SHORT_STAGES = 3;    // ... for K of a few blocks (two CTAs per SM)
 
 constexpr int S = Exact6::S;
 
-template <class PR, int BN, int ST = PR::STAGES>
+template <class PR, int BN, int ST>
 struct Cfg {
   static constexpr int A_TILE = BM * BK * 2;                 // 8 KB
   static constexpr int B_TILE = BN * BK * 2;                 // 8 / 4 KB
@@ -109,12 +110,6 @@ struct OzArgs {
   unsigned long long* colmax;  // EPI_STOREMAX: column maxima (float bits of |value|)
   int* err;
 };
-
-__device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
-  s = a + b;
-  const float bb = s - a;
-  e = (a - (s - bb)) + (b - bb);
-}
 
 // (hi, lo) ~ a0 + a1 + a2 + a3 (a0, a1, a2 exact integer sums, a3 rounded; three slices: no a3)
 template <int NS>
@@ -292,7 +287,7 @@ struct Batched {
   static constexpr int STAGES = PR::NACC == 4 ? (PR::S == 6 ? 3 : PR::S == 4 ? 4 : 5) : 3;
   static constexpr int THREADS = 320;
   static constexpr int EPI_WARPS = 8;
-  static constexpr int SMEM_BYTES = STAGES * Cfg<PR, BN>::STAGE_BYTES + 1024 + 1024;
+  static constexpr int SMEM_BYTES = STAGES * Cfg<PR, BN, STAGES>::STAGE_BYTES + 1024 + 1024;
 };
 
 // 2^e as a float for any int e, exact: normal, subnormal below 2^-126, 0 below 2^-149, inf
@@ -342,7 +337,7 @@ template <class PR, int BN, int EPI = EPI_STORE>
 __global__ void __launch_bounds__(320, PR::NACC == 4 ? 1 : 2)
     tc_slice_batched_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant__ CUtensorMap mB,
                             OzArgs args) {
-  using C = Cfg<PR, BN>;
+  using C = Cfg<PR, BN, Batched<PR>::STAGES>;
   static_assert(BN == Batched<PR>::BN, "batched tile width");
   constexpr int STAGES = Batched<PR>::STAGES;
   constexpr uint32_t ACC = PR::NACC * BN;  // TMEM columns of one accumulator set
@@ -614,7 +609,7 @@ __global__ void __launch_bounds__(320, PR::NACC == 4 ? 1 : 2)
 // these of 64.
 template <int BN_>
 struct ResT {
-  static constexpr int BN = BN_, HW = BN_ / 2, PG = 128 / BN_, MAX_KB = BN_ / 32, THREADS = 320, EPI_WARPS = 8;
+  static constexpr int BN = BN_, HW = BN_ / 2, PG = 128 / BN_, MAX_KB = BN_ / 32, EPI_WARPS = 8;
   static constexpr int STAGES = BN_ == 64 ? 2 : 4;      // (two CTAs per SM for 32 and 64)
   static constexpr int A_TILE = BM * BK * 2;            // 8 KB: one K block of one plane
   static constexpr int B_TILE = 128 * BK * 2;           // 8 KB: PG aux functions
@@ -1045,22 +1040,6 @@ unsigned grid_warps(int64_t rows, int num_sms) {
   return (unsigned)std::max<int64_t>(1, std::min<int64_t>(div_up(rows * 32, 256), 16 * (int64_t)num_sms));
 }
 
-PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-  static bool tried = false;
-  if (!tried) {
-    tried = true;
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-    else
-      cudaGetLastError();
-  }
-  return fn;
-}
-
 // 3-D BF16 / FP16 tensor map: dims {K, rows, depth}, row stride ld elements, box {32, box_rows,
 // box_depth}, 64B swizzle.
 CUtensorMap make_map(const void* base, int64_t K, int64_t rows, int64_t depth, int64_t ld, int box_rows,
@@ -1299,7 +1278,7 @@ bool oz_available(cphf_ctx* c) {
   static PerDevice attr;
   const bool ok = attr.once(c->device, [] {
     return set_smem_attr<Exact6>() && set_smem_attr<Exact6c>() && set_smem_attr<Exact6c3>() &&
-           set_smem_attr<Split2>() && set_rho_smem_attr<SHORT_STAGES>() && set_rho_smem_attr<Split2::STAGES>();
+           set_smem_attr<Split2>() && set_rho_smem_attr<SHORT_STAGES>() && set_rho_smem_attr<RHO_STAGES>();
   });
   if (!ok) cudaGetLastError();
   return ok;
@@ -1730,7 +1709,7 @@ void lp_gemm_rho(cphf_ctx* c, OzState& z, const PlaneMat& A, int64_t a_row0, con
   if (a.nkb <= 2 * SHORT_STAGES)
     tc_rho_kernel<SHORT_STAGES><<<tiles, 128, Cfg<Split2, 128, SHORT_STAGES>::SMEM_BYTES, c->stream>>>(mA, mB, a);
   else
-    tc_rho_kernel<Split2::STAGES><<<tiles, 128, Cfg<Split2, 128>::SMEM_BYTES, c->stream>>>(mA, mB, a);
+    tc_rho_kernel<RHO_STAGES><<<tiles, 128, Cfg<Split2, 128, RHO_STAGES>::SMEM_BYTES, c->stream>>>(mA, mB, a);
   count_launch();
   CPHF_CUDA(cudaGetLastError());
 }

@@ -27,7 +27,6 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
-#include <cudaTypedefs.h>
 
 #include <algorithm>
 #include <cstring>
@@ -35,6 +34,7 @@
 
 #include "slices.cuh"
 #include "tc_pair.cuh"
+#include "tc_map.cuh"
 #include "tc_ptx.cuh"
 
 namespace cphf {
@@ -108,11 +108,6 @@ __device__ __forceinline__ void commit_pair(uint32_t bar) {
       : "memory");
 }
 
-__device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
-  s = a + b;
-  const float bb = s - a;
-  e = (a - (s - bb)) + (b - bb);
-}
 // float -> double on the integer pipe (subnormals, far below any group sum's unit, to zero; NaN and
 // Inf, from non-finite operands, stay): the conversion instruction occupies the FP64 pipe like a
 // multiplication.  Branch-free: it is unrolled over an accumulator chunk.
@@ -322,21 +317,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
 }
 
 // ---- host side ------------------------------------------------------------------------------
-PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-    else
-      cudaGetLastError();
-  });
-  return fn;
-}
-
 // 3-D map: dims {K, rows, depth}, row stride ld, box {row / 2 elements, box_rows, 1}, swizzle = row bytes
 CUtensorMap make_map(const void* base, int64_t K, int64_t rows, int64_t depth, int64_t ld, int row, int box_rows,
                      bool bf16) {
