@@ -40,13 +40,13 @@ unsigned grid1(int64_t n) { return (unsigned)std::max<int64_t>(1, std::min<int64
 // Factor the b x b diagonal block A[k0:k0+b, k0:k0+b] (lower triangle, col-major, ld lda) in
 // shared memory: A = L L^T.  info (device) receives k0 + j + 1 at the first pivot that is not
 // positive and finite (unchanged when an earlier failure was recorded).  Bound by the serial chain
-// of its columns (square root, scaling, rank-one update); one reciprocal square root per column,
-// multiplied into the rows, instead of a division per row, and no index division in the update:
-// 100 -> 45 us for b = 64.
+// of its columns (reciprocal square root, scaling, rank-one update): the reciprocal is multiplied into
+// the rows instead of a division per row, another warp takes the square root meanwhile, and no index is
+// divided in the update: 100 -> 84 us for b = 64.
 __global__ void chol_diag_kernel(double* __restrict__ A, int64_t lda, int64_t k0, int b, int* info) {
   __shared__ double a[CB][CB + 1];  // a[j][i]: column j, row i
   __shared__ int bad;
-  __shared__ double rs;
+  __shared__ double rs, diag[CB];
   const int t = threadIdx.x;
   for (int e = t; e < b * b; e += blockDim.x) {
     const int i = e % b, j = e / b;
@@ -56,17 +56,17 @@ __global__ void chol_diag_kernel(double* __restrict__ A, int64_t lda, int64_t k0
   __syncthreads();
   const int i = t % CB, l0 = t / CB;
   for (int j = 0; j < b; ++j) {
-    if (t == 0) {
+    if (t == 0 || t == kThreads - 32) {
       double d = a[j][j];
       if (!(d > 0.0) || !isfinite(d)) {
-        if (!bad) atomicCAS(info, 0, (int)(k0 + j + 1));
-        bad = 1;
+        if (t == 0) {
+          if (!bad) atomicCAS(info, 0, (int)(k0 + j + 1));
+          bad = 1;
+        }
         d = 1.0;  // keep the arithmetic finite; the result is discarded by the host
       }
-      // sqrt(d) from its reciprocal, corrected by one Newton step
-      const double r = rsqrt(d), s = d * r;
-      rs = r;
-      a[j][j] = fma(0.5 * r, fma(-s, s, d), s);
+      if (t == 0) rs = rsqrt(d);
+      else diag[j] = sqrt(d);
     }
     __syncthreads();
     if (t < b && t > j) a[j][t] *= rs;
@@ -78,15 +78,15 @@ __global__ void chol_diag_kernel(double* __restrict__ A, int64_t lda, int64_t k0
   }
   for (int e = t; e < b * b; e += blockDim.x) {
     const int r = e % b, j = e / b;
-    if (r >= j) A[(k0 + r) + lda * (k0 + j)] = a[j][r];
+    if (r >= j) A[(k0 + r) + lda * (k0 + j)] = r == j ? diag[j] : a[j][r];
   }
 }
 
 // Forward substitutions x_j = (v_j - sum_{q<j} L[j][q] x_q) / L[j][j] with a w x w lower factor
 // (w <= TB) for many vectors v: kTriRows vectors per CTA, vectors and factor in shared memory, the
 // update of the later elements spread over the block (a thread per vector leaves the chain of
-// w^2 / 2 FMAs and their loads to one lane: 221 us for 600 rows of 64, now ~20; the inverse of a
-// 128 block 493 us, now ~45).  Vector r's element j sits at v + r vr + j vj; with `identity` the
+// w^2 / 2 FMAs and their loads to one lane: 221 us for 600 rows of 64, now 28; the inverses of the 128
+// blocks 493 us, now 77).  Vector r's element j sits at v + r vr + j vj; with `identity` the
 // vectors start as the unit vectors e_r and are only written (the columns of inv(L)).  blockIdx.y:
 // diagonal blocks of width TB of the factor L [n, n] (ldl), one after the other.
 constexpr int kTriRows = 16;
