@@ -82,7 +82,7 @@ typedef struct cphf_config {
   int32_t verify_residual;   /* mixed: how the residual of every correction after the first is obtained and
                                 convergence decided.  0 = updated with the split-precision operator,
                                 r -= (I + A_lowp) d (no FP64-accurate application);  1 = recomputed with
-                                the native FP64 operator;  2 (default) = computed with the FP64-accurate
+                                the plain FP64 operator;  2 (default) = computed with the FP64-accurate
                                 operator of residual_dfloat: with the exact-slice tensor cores (residual_dfloat
                                 = 2) as r -= (I + A) d, the correction d applied in correction precision:
                                 the fewest BF16 slices per operand whose error bound (3 slices, 6
@@ -92,13 +92,15 @@ typedef struct cphf_config {
                                 < residual_tol. */
   int32_t fp64_every_step;   /* mixed: FP64 residual after every correction, not only the first (default 0) */
   int64_t xc_chunk_points;   /* grid points per XC chunk (default 0 = 8 GiB of intermediates) */
-  int32_t residual_dfloat;   /* mixed: arithmetic of the correction residuals.  0 = native FP64;
-                                1 = double-float GEMMs on the FP32 pipes (~1e-14 relative);
+  int32_t residual_dfloat;   /* mixed: arithmetic of the correction residuals.  0 = plain FP64
+                                (its GEMMs as tensor_cores says);
+                                1 = double-float GEMMs on the FP32 pipes (~1e-14 relative), large ones as
+                                fixed-point digits;
                                 2 = as 1, with the whole RI-K term and the XC grid contractions on the
                                 tensor cores as exact BF16 slice products (6 x 6 bits, ~1e-10 relative
                                 to the operand row maxima; default; without tensor cores it behaves
                                 as 1).
-                                verify_residual = 1 recomputes the later residuals in native FP64. */
+                                verify_residual = 1 recomputes the later residuals in plain FP64. */
   int32_t cuda_graphs;       /* mixed: replay each block width's split-precision operator application
                                 from a captured CUDA graph (default 1); bypassed while profiling */
 } cphf_config;
@@ -115,7 +117,7 @@ typedef struct cphf_stats {
   int64_t lowp_matvec_columns;  /* columns pushed through the split-precision operator */
   int64_t refine_steps;         /* defect-correction steps (mixed precision) */
   double seconds;               /* wall time of the call */
-  int64_t residual_mode;        /* how residual_max was computed: 0 native FP64, 1 double-float GEMMs,
+  int64_t residual_mode;        /* how residual_max was computed: 0 plain FP64, 1 double-float GEMMs,
                                    2 double-float + exact BF16 slice products on the tensor cores,
                                    3 updated with the split-precision operator, 4 as 2 for the first
                                    correction, later corrections subtracted with the exact-slice operator
@@ -269,7 +271,7 @@ cphf_status cphf_compute_dimless_cphf_rhs(cphf_ctx* ctx, const double* f1ao_core
                                           double* const* s1mo);
 /* finalize_cphf (rscf.rs:328-353, uscf.rs:365-406): f1mo[s], s1mo[s] [nmo, nocc_s, 3, natm];
  * mo1[s] in/out; mo_e1[s] [nocc_s, nocc_s, 3, natm] out.  Its one response_mo (rscf.rs:342)
- * runs in native FP64 on an FP64 context and in the FP64-accurate arithmetic selected by
+ * runs in plain FP64 on an FP64 context and in the FP64-accurate arithmetic selected by
  * residual_dfloat on a MIXED context. */
 cphf_status cphf_finalize_cphf(cphf_ctx* ctx, const double* const* f1mo, const double* const* s1mo,
                                int64_t natm, double* const* mo1, double* const* mo_e1);

@@ -751,7 +751,7 @@ cphf_status cphf_finalize_cphf(cphf_ctx* c, const double* const* f1mo, const dou
     {
       // rscf.rs:342.  A mixed-precision context evaluates this response with its FP64-accurate
       // operator (residual_dfloat: exact-slice tensor cores + double-float by default), a
-      // plain FP64 context with native FP64.
+      // plain FP64 context with plain FP64.
       const bool mixed = c->cfg.precision == CPHF_PRECISION_MIXED && c->lowp;
       AccurateScope scope(c, mixed ? c->cfg.residual_dfloat : 0);
       response_mo_fp64(c, x, nprop, resp, false);

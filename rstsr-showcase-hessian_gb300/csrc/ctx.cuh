@@ -334,7 +334,7 @@ void lowp_park(cphf_ctx* c, bool at_once);
 extern thread_local cphf_ctx* g_call_ctx;  // the context whose call runs
 
 // Scope in which the FP64 operator (response_mo_fp64) runs in the FP64-accurate arithmetic of
-// the mixed context: mode 0 native FP64, 1 double-float GEMMs, 2 double-float plus the RI-K
+// the mixed context: mode 0 plain FP64, 1 double-float GEMMs, 2 double-float plus the RI-K
 // term and XC contractions as exact BF16 slice products on the tensor cores.  `used` is the
 // mode in effect (2 falls back to 1 where no tensor-core contraction applies).
 struct AccurateScope {

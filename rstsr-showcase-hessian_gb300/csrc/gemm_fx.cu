@@ -90,7 +90,13 @@ __host__ __device__ constexpr int group_kb(int g) {
   while (p > ROUND_KB && group_bound(g) * BK * p > 1 << 23) p >>= 1;
   return p;
 }
-static_assert(group_bound(S - 1) * BK * ROUND_KB <= 1 << 23, "exact FP32 sums of a round");
+constexpr bool sums_exact() {
+  for (int g = 0; g < S; ++g)
+    if (group_bound(g) * BK * group_kb(g) > 1 << 23) return false;
+  return true;
+}
+static_assert(sums_exact(), "FP32 sums between two drains");
+static_assert(SPLIT_KB % ROUND_KB == 0, "K ranges of whole rounds");
 
 // element offset of row r with the optional two-level index r = r0 + div r1
 __host__ __device__ __forceinline__ int64_t off2(int64_t r, int64_t div, int64_t s1, int64_t s2) {
@@ -288,7 +294,7 @@ struct FxArgs {
   int64_t K;
   int m_tiles, n_tiles, batch;
   int items;               // m_tiles n_tiles splits batch
-  int nkb, kb_per_split;   // K blocks of 32, per split (a multiple of the longest accumulation)
+  int nkb, kb_per_split;   // K blocks of 32, per split (a multiple of SPLIT_KB)
   int splits;
   const int* eA;           // [batch][M], [batch][N]
   const int* eB;

@@ -7,7 +7,7 @@
 // correction: each step solves (I + A_lowp) d = r with the device Krylov solver (FP64
 // basis, orthogonalisation and projected solve), then recomputes r = b - (I + A) x with
 // an FP64-accurate operator (exact BF16 slice products on the tensor cores plus
-// double-float GEMMs by default, or native FP64), until max_j ||r_j||_2 < residual_tol.
+// double-float GEMMs by default, or plain FP64), until max_j ||r_j||_2 < residual_tol.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -494,7 +494,7 @@ bool solve_mixed(cphf_ctx* c, const double* b, const double* x0, int64_t nset, d
   };
   // Defect correction.  Step 0 solves with the full right-hand side; its residual is the one
   // that must be exact, so it is recomputed with the FP64-accurate operator (residual_dfloat):
-  // r1 = b - (I + A) x1.  With verify_residual on (1 native FP64, 2 the residual_dfloat
+  // r1 = b - (I + A) x1.  With verify_residual on (1 plain FP64, 2 the residual_dfloat
   // operator) every later residual is recomputed the same way and convergence is decided only
   // on a recomputed residual, so the solve measures its own final ||b - (I+A)x||.  With it off,
   // later corrections d are O(|r1|) and the update r -= (I + A_lowp) d carries an error of
