@@ -35,8 +35,8 @@ __device__ __forceinline__ int64_t off2(int64_t m, int64_t div, int64_t s1, int6
 }
 
 template <typename T, typename Cfg, typename TA, typename TB, typename TC>
-__global__ void __launch_bounds__(256) gemm_kernel(GemmDesc d, unsigned m_tiles, int ksplit, int64_t kchunk,
-                                                   T* ws, const int* only_if) {
+__global__ void __launch_bounds__(256) gemm_kernel(GemmDesc d, int ksplit, int64_t kchunk, T* ws,
+                                                   const int* only_if) {
   if (only_if != nullptr && *only_if == 0) return;
   constexpr int BM = Cfg::BM, BN = Cfg::BN, BK = Cfg::BK, TM = Cfg::TM, TN = Cfg::TN;
   constexpr int NTX = BN / TN, NTY = BM / TM, NT = NTX * NTY;
@@ -54,9 +54,8 @@ __global__ void __launch_bounds__(256) gemm_kernel(GemmDesc d, unsigned m_tiles,
   const int tx = VEC ? tid / NTY : tid % NTX, ty = VEC ? tid % NTY : tid / NTX;
   auto row = [&](int i) { return VEC ? (i >> 2) * (4 * NTY) + ty * 4 + (i & 3) : ty + i * NTY; };
   auto col = [&](int j) { return VEC ? (j >> 2) * (4 * NTX) + tx * 4 + (j & 3) : tx + j * NTX; };
-  // tiles in x alone, rows fastest: y and z hold 65535, which millions of columns exceed
-  const int64_t m0 = (int64_t)(blockIdx.x % m_tiles) * BM;
-  const int64_t n0 = (int64_t)(blockIdx.x / m_tiles) * BN;
+  const int64_t m0 = (int64_t)blockIdx.x * BM;
+  const int64_t n0 = (int64_t)blockIdx.y * BN;
   const int64_t z = blockIdx.z;
   const int split = (int)(z % ksplit);
   const int64_t bidx = z / ksplit;
@@ -319,7 +318,24 @@ cudaError_t run(const GemmDesc& d, cudaStream_t stream, void* workspace, size_t 
   ksplit = (int)((d.K + kchunk - 1) / kchunk);
   const int64_t gx = (d.M + Cfg::BM - 1) / Cfg::BM;
   const int64_t gy = (d.N + Cfg::BN - 1) / Cfg::BN;
-  if (gx * gy > INT32_MAX) return cudaErrorInvalidConfiguration;
+  if (gy > 65535) {
+    // more column tiles than the grid's y holds (an output of millions of columns): several launches, on
+    // whole blocks of a two-level column index
+    int64_t step = (int64_t)65535 * Cfg::BN;
+    if (d.n_div > 0) step = step / d.n_div * d.n_div;
+    if (step == 0) return cudaErrorInvalidConfiguration;
+    for (int64_t n0 = 0; n0 < d.N; n0 += step) {
+      GemmDesc s = d;
+      s.N = std::min(step, d.N - n0);
+      const int64_t ob = d.n_div > 0 ? n0 / d.n_div * d.b_n2 : n0 * d.b_n;
+      const int64_t oc = d.n_div > 0 ? n0 / d.n_div * d.c_n2 : n0 * d.c_n;
+      s.B = static_cast<const char*>(d.B) + ob * (int64_t)sizeof(TB);
+      s.C = static_cast<char*>(d.C) + oc * (int64_t)sizeof(TC);
+      const cudaError_t err = run<T, Cfg, TA, TB, TC>(s, stream, workspace, ws_bytes, num_sms, only_if, split);
+      if (err != cudaSuccess) return err;
+    }
+    return cudaSuccess;
+  }
   // batches beyond the grid z limit are issued in several launches
   const int64_t zmax = 65535 / ksplit;
   for (int64_t b0 = 0; b0 < nb; b0 += zmax) {
@@ -332,9 +348,8 @@ cudaError_t run(const GemmDesc& d, cudaStream_t stream, void* workspace, size_t 
       s.C = static_cast<char*>(d.C) + b0 * d.c_b1 * (int64_t)sizeof(TC);
       s.batch1 = bn;
     }
-    dim3 grid((unsigned)(gx * gy), 1, (unsigned)(bn * ksplit));
-    gemm_kernel<T, Cfg, TA, TB, TC><<<grid, 256, 0, stream>>>(s, (unsigned)gx, ksplit, kchunk,
-                                                              static_cast<T*>(workspace), only_if);
+    dim3 grid((unsigned)gx, (unsigned)gy, (unsigned)(bn * ksplit));
+    gemm_kernel<T, Cfg, TA, TB, TC><<<grid, 256, 0, stream>>>(s, ksplit, kchunk, static_cast<T*>(workspace), only_if);
     count_launch();
     cudaError_t err = cudaGetLastError();
     if (err != cudaSuccess) return err;
