@@ -436,10 +436,7 @@ void tc_planes_term(cphf_ctx* c, const __half* a_hi, const __half* a_lo, int64_t
   t.out = out;
   t.ld_out = ld_out;
   t.err = err;
-  // as term 1's accumulators, or less where few tiles leave the SMs short ranges anyway
-  const int64_t tiles = std::max<int64_t>(1, div_up(M, 128) * div_up(N, 256));
-  const int64_t ranges = std::max<int64_t>(1, std::min<int64_t>(npc, div_up(2 * (int64_t)c->num_sms, tiles)));
-  t.max_k = std::min<int64_t>(32 * M, 2 * div_up(npc, ranges) * K);
+  t.max_k = 32 * M;
   pair_split2(c, t);
 }
 

@@ -411,8 +411,8 @@ void launch_pair(cphf_ctx* c, const PairTerm& t, int kb_per_cta) {
     // tile's atomics cost about eight K blocks) and short enough to fill the SMs evenly
     // The accumulators drop low bits at every MMA, an error that grows with the products summed, so
     // max_k bounds a range.  Exchange response against FP64, in one accumulator over ranges that the
-    // time alone chooses / hi*hi in one of its own and at most 32 nao products: nao 243 2.4e-5 / 6.3e-6,
-    // nao 400 5.3e-5 / 1.0e-5, nao 600 5.8e-5 / 2.0e-5, for 0.5 % of a solve's time.
+    // time alone chooses / hi*hi in one of its own and at most 32 nao products: nao 243 2.4e-5 / 6.7e-6,
+    // nao 400 5.3e-5 / 1.4e-5, nao 600 5.8e-5 / 2.0e-5, for 0.5 % of a solve's time.
     int64_t best = t.np;
     double best_t = 0.0;
     const int64_t r0 = t.max_k > 0 ? div_up(t.np, std::max<int64_t>(1, t.max_k / t.K)) : 1;
