@@ -256,24 +256,22 @@ __global__ void __launch_bounds__(kMgsThreads) mgs_kernel(MgsArgs a) {
   for (int64_t j = wid; j < m; j += kMgsWarps) {
     // four sums a lane: shorter chains round less (these columns may be the most correlated ones)
     double acc[B] = {0.0, 0.0, 0.0, 0.0}, part[3][B] = {};
-    int64_t r = lane;
-    for (; r + 96 < len; r += 128) {
+    for (int64_t r0 = 0; r0 < len; r0 += 128) {  // (warp-uniform, the last rows predicated)
       double v[4];
 #pragma unroll
-      for (int h = 0; h < 4; ++h) v[h] = Vb[r + 32 * h + n * j];
+      for (int h = 0; h < 4; ++h) {
+        const int64_t r = r0 + 32 * h + lane;
+        v[h] = r < len ? Vb[r + n * j] : 0.0;
+      }
 #pragma unroll
-      for (int q = 0; q < B; ++q)
-        if (q < w) {
-          acc[q] = fma(v[0], panel(cur, 0, q, r), acc[q]);
+      for (int h = 0; h < 4; ++h) {
+        const int64_t r = r0 + 32 * h + lane;
+        if (r0 + 32 * h >= len) break;
+        double* const a4 = h == 0 ? acc : part[h - 1];
 #pragma unroll
-          for (int h = 1; h < 4; ++h) part[h - 1][q] = fma(v[h], panel(cur, 0, q, r + 32 * h), part[h - 1][q]);
-        }
-    }
-    for (; r < len; r += 32) {
-      const double v = Vb[r + n * j];
-#pragma unroll
-      for (int q = 0; q < B; ++q)
-        if (q < w) acc[q] = fma(v, panel(cur, 0, q, r), acc[q]);
+        for (int q = 0; q < B; ++q)
+          if (q < w) a4[q] = fma(v[h], r < len ? panel(cur, 0, q, r) : 0.0, a4[q]);
+      }
     }
 #pragma unroll
     for (int q = 0; q < B; ++q) acc[q] = (acc[q] + part[0][q]) + (part[1][q] + part[2][q]);
